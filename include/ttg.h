@@ -188,11 +188,11 @@ ttg_status ttg_apply_h(ttg_op* op, const ttg_block* X, ttg_block* HX);
  * (eigensolver/MultTm.h:37, eigensolver/MultTm.cu:86-224).  FP64 data and
  * result, computed on the tensor cores: each value becomes six exact BF16
  * digits on a power-of-two scale of its row, the digit products are summed
- * exactly in tensor memory and the 96-deep groups in double-FP32, so an entry
+ * exactly in tensor memory and the 128-deep groups in double-FP32, so an entry
  * lands within about 2^-48 of the product of its two rows' scales times the
- * length (measured: within 2^-44 of the sum of |terms|).  When an operand's
- * alignment rules the tensor cores out, the products and sums run in
- * double-FP32 on the CUDA cores (each value a pair of floats, about 47
+ * length (measured: within 2^-44 of the sum of |terms|).  The digit planes take a
+ * workspace of the operator (at most 1 GiB); without room for it the products
+ * and sums run in double-FP32 on the CUDA cores (each value a pair of floats, about 47
  * significant bits, FP32 exponent range; within ~6e-14 of the sum of |terms|).
  * s_host may be NULL when only the device copy is wanted (kept inside the
  * op). */

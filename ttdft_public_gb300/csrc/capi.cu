@@ -47,8 +47,11 @@ ttg_status check_block(const ttg_op* op, const ttg_block* b) {
 // S = X^T Y (k x k, column-major) from FP64 blocks: on the tensor cores
 // (ozgemm.cu) where the operands allow, else the double-FP32 CUDA-core kernel.
 ttg_status gram_fp64(ttg_op* op, const double* X, const double* Y, int k, double* S, bool sym) {
-  const OzOperand A{X, k, op->n, op->ld, true}, B{Y, k, op->n, op->ld, true};
-  if (ozgemm_supported(A, B)) return ozgemm(op, A, B, S, 1, k, sym);
+  const OzOperand A{X, k, op->n, 1, op->ld}, B{Y, k, op->n, 1, op->ld};
+  if (ozgemm_supported(A, B)) {
+    const ttg_status s = ozgemm(op, A, B, S, OzLayout{1, k}, sym);
+    if (s != TTG_OOM) return s;
+  }
   return gram_tn(op, X, Y, k, S, sym);
 }
 
@@ -58,11 +61,15 @@ ttg_status gram_fp64(ttg_op* op, const double* X, const double* Y, int k, double
 // product then runs on K scales taken from X's columns.
 ttg_status product_fp64(ttg_op* op, const double* X, const double* Q, double* out, int k,
                         int transQ, bool lower, bool kscale = false) {
-  // B(n = q, k = p) = Qop[p, q]: Q[p + q k] (K-major) or, transposed, Q[q + p k] (MN-major)
-  const OzOperand A{X, op->n, k, op->ld, false}, B{Q, k, k, k, transQ != 0};
-  const OzOperand cols{X, k, op->n, op->ld, true};
-  if (ozgemm_supported(A, B))
-    return ozgemm(op, A, B, out, op->ld, 1, false, transQ && lower, kscale ? &cols : nullptr);
+  // B(n = q, k = p) = Qop[p, q]: Q[p + q k] or, transposed, Q[q + p k]
+  const OzOperand A{X, op->n, k, op->ld, 1};
+  const OzOperand B = transQ ? OzOperand{Q, k, k, 1, k} : OzOperand{Q, k, k, k, 1};
+  const OzOperand cols{X, k, op->n, 1, op->ld};
+  if (ozgemm_supported(A, B)) {
+    const ttg_status s = ozgemm(op, A, B, out, OzLayout{op->ld, 1}, false, transQ && lower,
+                                kscale ? &cols : nullptr);
+    if (s != TTG_OOM) return s;
+  }
   return gemm_nn_small(op, X, Q, out, k, transQ, lower);
 }
 

@@ -1,11 +1,10 @@
-// FP64-accurate GEMMs of the orthonormalisation and Rayleigh-Ritz steps on the
-// tcgen05 tensor cores: the Gram matrices X^T X and X^T (H X), the update
-// X L^-T and the rotation X Q (eigensolver/MultTm.cu:86-224, main.cc:1066-1207
-// compute them in FP64).
+// FP64-accurate GEMMs on the tcgen05 tensor cores: the Gram matrices X^T X and
+// X^T (H X), the update X L^-T and the rotation X Q (eigensolver/MultTm.cu:
+// 86-224, main.cc:1066-1207 compute them in FP64), the mode Grams and products
+// of the STHOSVD and the contraction of the Hamiltonian update.
 //
-// C[m][n] (+)= sum_k A(m, k) B(n, k) with FP64 operands A (M x K) and B
-// (N x K), each stored K-major (element (r, k) at p[r ld + k]) or MN-major
-// (p[k ld + r]); C is FP64 at C[m c_rs + n c_cs].
+// C[m][n] = sum_k A(m, k) B(n, k) with FP64 operands A (M x K) and B (N x K)
+// of any strides (OzOperand); C is FP64.
 //
 // Arithmetic (an Ozaki-type error-free split).  Every row r of an operand has
 // a power-of-two scale with max_k |A(r, k)| < 2^e_r (k_rowexp_*, one pass
@@ -17,30 +16,48 @@
 // integer operations: no FP64 arithmetic, which runs at a small fraction of
 // the FP32 rate on this part.  The product of two values is sum_{i,j} d_i d'_j 2^-8(i+j);
 // the 21 digit products with i + j <= 5 are summed per level L = i + j in six
-// FP32 accumulators in tensor memory.  Over a group of 96 values of K a level
-// sum is an integer of magnitude below 96 * 2^17 < 2^24, so the accumulators
+// FP32 accumulators in tensor memory.  Over a group of 128 values of K a level
+// sum is an integer of magnitude at most 128 * 2^17 = 2^24, so the accumulators
 // hold it exactly.  The epilogue folds the six levels of a group with
 // error-free two-sums and adds the groups in double-FP32 (about 2^-48
 // relative).  Left out: the digit products with i + j >= 6 and the rounding
 // of each value to 2^-40 of its row's scale, each below 2^-47 of the product
 // of the two rows' scales.
 //
-// One CTA per output tile of 128 x 32 and K range (split K), warp-specialised:
-//  - warp 0, one thread: TMA tile loads of the FP64 operands (box 16 x 128 of
-//    A, 16 x 32 of B, either layout) into a raw ring of 3 stages;
-//  - warp 3, one thread: waits for the raw copies in order and publishes the
-//    count of landed chunks (one thread polls the barriers, not eight warps);
-//  - warps 4-11, each an eighth of the rows of every chunk: cut the 160 rows x
-//    16 values into six digit planes each, in the canonical K-major MMA
-//    layout, into a ring of 5 stages;
-//  - warp 2, one thread: waits for the digit planes (and, before a group, for
-//    the epilogue to have emptied the accumulator buffer it will use) and
-//    publishes the count of ready chunks;
-//  - warp 1, one thread: 21 MMAs (M128 N32 K16) per chunk into the six level
-//    accumulators of one of two buffers;
-//  - warps 12-15 (one per 32 TMEM lanes): fold the levels of each group into
-//    running double-FP32 sums in registers; at the end scale by
-//    2^(e_m + e_n - 16) and store.
+// Two kernels.  Cutting a value into digits costs about forty integer
+// instructions; inside the GEMM every CTA repeats it for its tile of both
+// operands, and that issue rate bounded the product (tensor pipe 6 %).  So
+//  - k_oz_slice cuts each operand once into digit planes in a workspace
+//    (8 bytes read, 12 written a value: bound by HBM), already in the order
+//    the tensor cores read: per 128 rows and 16 values of K one 24 KB block;
+//  - k_oz_mma multiplies planes only: three copies (TMA) a chunk into a ring,
+//    MMAs, and the fold.
+// Operands larger than the workspace (kPlaneBudget) are taken in slabs of K
+// (Gram matrices: the sums are added in C's partial) or of A's rows.
+//
+// k_oz_mma: one CTA per 128 x 64 output tile and K range (split K), 20 warps.
+//  - The six digit planes of 32 rows of B lie one after the other, and so do
+//    the six level accumulators, so digit i of A times digits 0 .. 5-i of B is
+//    ONE MMA of N = 32 (6 - i) columns, starting at level i: six MMAs a chunk
+//    instead of 21, each reading A's plane once (a 128 x 32 MMA alone is bound
+//    by the shared-memory read of A).
+//  - The tile's two halves of 32 columns (2 x 192 tensor-memory columns) each
+//    have an issuing thread (warps 1 and 3): while one half waits for its eight
+//    epilogue warps to empty its accumulators, the other's MMAs have the tensor
+//    pipe, and the half that is ahead by then stays so.  One thread for both
+//    spent a third of its time in the commits (330 cycles each).  A chunk
+//    costs 36 KB of copies for 2 x 336 MMA cycles.
+//  - warp 0, one thread: the copies (few and large: 18 copies of 1 to 4 KB a
+//    chunk took four times as long, at 85 ns each); warp 2, one thread: waits
+//    for a chunk's copies in order and publishes the count (a thread that
+//    issues MMAs must not wait on an mbarrier with MMAs in flight: the wait
+//    queues behind them); warps 4-11 and 12-19: the folds of the two halves,
+//    running double-FP32 sums in registers, at the end scaled by
+//    2^(e_m + e_n - 16) and stored.
+// Bound: the shared-memory reads of the MMAs (376 cycles a half chunk against
+// 336 of arithmetic) and the folds' tensor-memory reads between them.
+// Measured (GB300): X^T X of 512,000 x 1,200 in FP64: 150 -> 19 ms with the
+// slicing; X L^-T 132 -> 20 ms; X^T Y of 9,261 x 57: 0.17 -> 0.035 ms.
 // Every wait is bounded; a wait that runs out sets the error word and the
 // abort flag, after which no role issues new copies or MMAs and the CTA
 // drains what it issued before releasing tensor memory.
@@ -60,29 +77,30 @@ namespace {
 using namespace tc;
 
 constexpr int OZ_M = 128;                               // rows of an A tile (MMA M)
-constexpr int OZ_N = 32;                                // rows of a B tile (MMA N)
+constexpr int OZ_H = 32;                                // columns of half a tile
+constexpr int OZ_N = 2 * OZ_H;                          // rows of a B tile
 constexpr int OZ_K = 16;                                // K per chunk
 constexpr int kDigits = 6;
 constexpr int kLevels = 6;
-constexpr int kGroupChunks = 6;                         // 96 values of K per exact level sum
-constexpr int kRawA = OZ_M * OZ_K * 8;                  // 16 KB FP64
-constexpr int kRawB = OZ_N * OZ_K * 8;                  // 4 KB
-constexpr int kRawStage = kRawA + kRawB;                // 20 KB
+constexpr int kGroupChunks = 8;                         // 128 values of K per exact level sum
 constexpr int kPlA = OZ_M * OZ_K * 2;                   // 4 KB: one BF16 digit plane of A
-constexpr int kPlB = OZ_N * OZ_K * 2;                   // 1 KB
-constexpr int kSplStage = kDigits * (kPlA + kPlB);      // 30 KB
-constexpr int kRawStages = 3;
-constexpr int kSplStages = 5;
-constexpr int kSmem = kRawStages * kRawStage + kSplStages * kSplStage + 1024;
-constexpr int kConvWarp0 = 4, kConvWarps = 8;           // share every chunk's rows
-constexpr int kEpiWarp0 = 12, kEpiWarps = 4;
-constexpr int kThreads = (kEpiWarp0 + kEpiWarps) * 32;  // 512
-constexpr int kBufCols = kLevels * OZ_N;                // 192
-constexpr uint32_t kTmemCols = 512;                     // two buffers (384)
+constexpr int kPlH = OZ_H * OZ_K * 2;                   // 1 KB: of half a B tile
+constexpr int kStageA = kDigits * kPlA;                 // 24 KB
+constexpr int kStageH = kDigits * kPlH;                 // 6 KB
+constexpr int kStage = kStageA + 2 * kStageH;           // 36 KB
+constexpr int kStages = 6;
+constexpr int kSmem = kStages * kStage + 1024;
+constexpr int kEpiWarp0 = 4, kEpiWarps = 8;             // per half: two per 32 TMEM lanes
+constexpr int OZ_E = OZ_H / 2;                          // columns of an epilogue warp
+constexpr int kThreads = (kEpiWarp0 + 2 * kEpiWarps) * 32;   // 640
+constexpr int kHalfCols = kLevels * OZ_H;               // 192
+constexpr uint32_t kTmemCols = 512;                     // two halves (384)
+constexpr int64_t kPlaneBudget = (int64_t)1 << 30;      // workspace of the digit planes
+constexpr int64_t kRowPad = OZ_M;                       // planes hold whole A tiles of rows
 
-// kind::f16: BF16 x BF16 -> FP32, A and B K-major, M = 128, N = 32
-__device__ __forceinline__ uint32_t idesc_oz() {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_N >> 3) << 17) |
+// kind::f16: BF16 x BF16 -> FP32, A and B K-major, M = 128, N = n
+__device__ __forceinline__ uint32_t idesc_oz(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
          ((uint32_t)(OZ_M >> 4) << 24);
 }
 
@@ -156,47 +174,146 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// byte offset of element (row, k) in a canonical K-major digit plane
-__device__ __forceinline__ int plane_off(int row, int k) {
-  return (row >> 3) * 256 + (k >> 3) * 128 + (row & 7) * 16 + (k & 7) * 2;
+// row scale 2^e from the largest biased exponent of the row (0 for an all-zero
+// row; a NaN or Inf row, 2047, keeps a large scale: its digits are NaN anyway)
+__device__ __forceinline__ int exp_of_bits(int b) { return b == 0 ? 0 : min(b, 2046) - 1022; }
+
+__device__ __forceinline__ int64_t row_at(const OzOperand& o, int64_t r) {
+  return o.rin >= o.rows ? r * o.rs : (r % o.rin) * o.rs + (r / o.rin) * o.rs2;
 }
 
-// Digit planes of one block of 8 operand rows of a chunk (raw FP64 tile of
-// R rows, either layout) by one warp.  Lane (r8, kp) = (lane / 4, lane % 4)
-// takes the pairs (row 8 rb + r8, k = 8 kh + 2 kp, k + 1), kh = 0, 1: the 32
-// lanes of a step store to 32 different banks of each plane (plane_off).
-template <int R, int MN>
-__device__ __forceinline__ void slice_block(const double* __restrict__ raw, const int* es,
-                                            unsigned char* planes, int plane_bytes, int rb,
-                                            int lane, const int* __restrict__ kadj, int ksign) {
-  const int row = 8 * rb + (lane >> 2), kp = lane & 3;
-  const int e = es[row];
-  double v[2][2];
+// One or two operands of the same rows and K (blockIdx.z).
+struct OzSlices {
+  OzOperand o[2];
+  int* ebits[2];              // largest biased exponent of each row
+  unsigned char* planes[2];
+};
+
+// Digit planes of 16 gridDim.x values of K from k0 on and of 128 gridDim.y rows
+// from r0 on: per 128 rows and chunk one 24 KB block, per digit 4 KB of 8-row x
+// 16-byte core matrices.  A thread cuts eight values of one row; rows beyond
+// the operand and values beyond kext are zero.  K scales (kexp, ksign):
+// v 2^(ksign kexp[k]).
+template <bool ROWS_FAST>
+__global__ void __launch_bounds__(256) k_oz_slice(const OzSlices S, int64_t r0, int64_t k0,
+                                                  const int* __restrict__ kexp, int ksign) {
+  const OzOperand& o = S.o[blockIdx.z];
+  const int rt = ROWS_FAST ? threadIdx.x & 127 : threadIdx.x >> 1;
+  const int half = ROWS_FAST ? threadIdx.x >> 7 : threadIdx.x & 1;
+  const int64_t r = r0 + (int64_t)blockIdx.y * 128 + rt;
+  const int64_t k = k0 + (int64_t)blockIdx.x * OZ_K + half * 8;
+  double v[8];
 #pragma unroll
-  for (int kh = 0; kh < 2; ++kh) {
-    const int k = 8 * kh + 2 * kp;
-    if (MN) {                 // raw [k][row]
-      v[kh][0] = raw[k * R + row];
-      v[kh][1] = raw[(k + 1) * R + row];
-    } else {                  // raw [row][16]
-      const double2 vv = *reinterpret_cast<const double2*>(raw + row * OZ_K + k);
-      v[kh][0] = vv.x;
-      v[kh][1] = vv.y;
+  for (int j = 0; j < 8; ++j) v[j] = 0.0;
+  int e = 0;
+  if (r < o.rows) {
+    e = exp_of_bits(__ldg(S.ebits[blockIdx.z] + r));
+    const double* p = o.p + row_at(o, r);
+    int64_t ki = k, kb = 0;
+    if (o.kin < o.kext) {
+      kb = k / o.kin;
+      ki = k - kb * o.kin;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (k + j < o.kext) v[j] = __ldg(p + ki * o.ks + kb * o.ks2);
+      if (++ki == o.kin) {
+        ki = 0;
+        ++kb;
+      }
     }
   }
+  uint32_t w[kDigits][4];
 #pragma unroll
-  for (int kh = 0; kh < 2; ++kh) {
-    const int k = 8 * kh + 2 * kp;
+  for (int j = 0; j < 8; j += 2) {
+    const int a0 = kexp ? ksign * __ldg(kexp + k + j) : 0;
+    const int a1 = kexp ? ksign * __ldg(kexp + k + j + 1) : 0;
     float d0[kDigits], d1[kDigits];
-    const int a0 = kadj ? ksign * __ldg(kadj + k) : 0;
-    const int a1 = kadj ? ksign * __ldg(kadj + k + 1) : 0;
-    digits6(v[kh][0], e, a0, d0);
-    digits6(v[kh][1], e, a1, d1);
-    const int off = plane_off(row, k);
+    digits6(v[j], e, a0, d0);
+    digits6(v[j + 1], e, a1, d1);
 #pragma unroll
-    for (int d = 0; d < kDigits; ++d)
-      *reinterpret_cast<uint32_t*>(planes + d * plane_bytes + off) = pack_bf16(d0[d], d1[d]);
+    for (int d = 0; d < kDigits; ++d) w[d][j / 2] = pack_bf16(d0[d], d1[d]);
   }
+  unsigned char* out = S.planes[blockIdx.z] +
+                       ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * kStageA + (rt >> 3) * 256 +
+                       half * 128 + (rt & 7) * 16;
+#pragma unroll
+  for (int d = 0; d < kDigits; ++d)
+    *reinterpret_cast<uint4*>(out + d * kPlA) = make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
+}
+
+// With K scales (kexp, ksign): the biased exponent of v 2^(ksign kexp[k]).
+__device__ __forceinline__ int scaled_ebits(double v, const int* kexp, int ksign, int64_t k) {
+  int E = (__double2hiint(v) >> 20) & 0x7FF;
+  if (E != 0 && E != 0x7FF && kexp) E = max(0, min(2046, E + ksign * __ldg(kexp + k)));
+  return E;
+}
+
+// Row scales: the largest biased exponent of each row (any v with biased
+// exponent E is below 2^(E - 1022)) into ebits, zeroed before.
+// Rows contiguous: 32 rows x 8 lanes over K, `kb` values of K a block.
+__global__ void __launch_bounds__(256) k_rowexp_rows(const OzSlices S, int64_t kb,
+                                                     const int* __restrict__ kexp, int ksign) {
+  __shared__ int red[8][33];
+  const OzOperand& o = S.o[blockIdx.z];
+  const int64_t r = (int64_t)blockIdx.x * 32 + threadIdx.x;
+  const int64_t k0 = (int64_t)blockIdx.y * kb, k1 = min(o.kext, k0 + kb);
+  int m = 0;
+  if (r < o.rows) {
+    const double* p = o.p + row_at(o, r);
+#pragma unroll 8
+    for (int64_t k = k0 + threadIdx.y; k < k1; k += 8) {
+      const int64_t q = o.kin < o.kext ? (k % o.kin) * o.ks + (k / o.kin) * o.ks2 : k * o.ks;
+      m = max(m, scaled_ebits(p[q], kexp, ksign, k));
+    }
+  }
+  red[threadIdx.y][threadIdx.x] = m;
+  __syncthreads();
+  if (threadIdx.y == 0 && r < o.rows) {
+    for (int y = 1; y < 8; ++y) m = max(m, red[y][threadIdx.x]);
+    if (m) atomicMax(S.ebits[blockIdx.z] + r, m);
+  }
+}
+
+// K contiguous: one warp per row and `kb` values of K
+__global__ void __launch_bounds__(256) k_rowexp_k(const OzSlices S, int64_t kb,
+                                                  const int* __restrict__ kexp, int ksign) {
+  const OzOperand& o = S.o[blockIdx.z];
+  const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (r >= o.rows) return;
+  const int64_t k0 = (int64_t)blockIdx.y * kb, k1 = min(o.kext, k0 + kb);
+  const double* p = o.p + row_at(o, r);
+  int m = 0;
+#pragma unroll 4
+  for (int64_t k = k0 + lane; k < k1; k += 32) {
+    const int64_t q = o.kin < o.kext ? (k % o.kin) * o.ks + (k / o.kin) * o.ks2 : k * o.ks;
+    m = max(m, scaled_ebits(p[q], kexp, ksign, k));
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if (lane == 0 && m) atomicMax(S.ebits[blockIdx.z] + r, m);
+}
+
+__global__ void k_exp_from_bits(int* __restrict__ e, int64_t n) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) e[i] = exp_of_bits(e[i]);
+}
+
+// 2^e times a float, as a double: the exponent is rebased in the bits (the
+// FP64 pipe, two lanes per SM, would take five operations a value)
+__device__ __forceinline__ double scaled_float(float x, int e) {
+  const uint32_t b = __float_as_uint(x), m = b & 0x7fffffffu;
+  if (m == 0) return 0.0;
+  return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + ((896u + (uint32_t)e) << 20))),
+                          (int)(b << 29));
+}
+
+// (hi + lo) 2^e
+__device__ __forceinline__ double scaled_sum(float hi, float lo, int e) {
+  // normal floats (sums of multiples of 2^-40) whose doubles stay normal
+  if (isfinite(hi) && isfinite(lo) && e > -800 && e < 800)
+    return scaled_float(hi, e) + scaled_float(lo, e);
+  return ((double)hi + (double)lo) * ldexp(1.0, e);
 }
 
 struct OzTiles {
@@ -210,7 +327,7 @@ struct OzTiles {
     }
     int m = 0;
     for (;; ++m) {
-      const int row = min(4 * m + 4, tiles_n);
+      const int row = min(2 * m + 2, tiles_n);
       if (t < row) break;
       t -= row;
     }
@@ -219,33 +336,42 @@ struct OzTiles {
   }
 };
 
-template <int A_MN, int B_MN>
-__global__ void __launch_bounds__(kThreads, 1) k_ozgemm(
-    const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-    const int* __restrict__ expA, const int* __restrict__ expB, int M, int N, int K,
-    int k_per_split, int b_lower, OzTiles tiles, double* __restrict__ out, int64_t o_rs,
-    int64_t o_cs, int64_t o_zs, const int* __restrict__ kexp, int* __restrict__ err) {
+struct OzOut {
+  double* p;
+  int64_t rin, rs, rs2, cs, zs;  // (m % rin) rs + (m / rin) rs2 + n cs + split zs
+  int accumulate;                // add to p
+};
+
+struct OzMma {
+  const unsigned char* pa;       // A's digit planes (B's: the tensor map)
+  const int *ea, *eb;            // biased exponents of A's and B's rows
+  int M, N, chunks, split_chunks;
+  int64_t row0;                  // first row of A's slab, for C
+  int b_lower_k0;                // >= 0: B(n, k) = 0 for k > n, planes start at this k
+};
+
+__global__ void __launch_bounds__(kThreads, 1) k_oz_mma(const __grid_constant__ CUtensorMap tmB,
+                                                        const OzMma g, const OzTiles tiles,
+                                                        const OzOut out, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024 - (su32(smem_raw) & 1023)) & 1023);
-  unsigned char* raw = smem;                                  // kRawStages x 20 KB
-  unsigned char* spl = smem + kRawStages * kRawStage;         // kSplStages x 30 KB
-  __shared__ __align__(8) uint64_t raw_full[kRawStages], raw_empty[kRawStages];
-  __shared__ __align__(8) uint64_t spl_full[kSplStages], spl_empty[kSplStages];
+  __shared__ __align__(8) uint64_t full[kStages], empty[kStages];
   __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2];
-  __shared__ __align__(8) uint64_t fin;
+  __shared__ __align__(8) uint64_t fin[2];
   __shared__ uint32_t tmem_slot;
-  __shared__ uint32_t ready, landed;
+  __shared__ uint32_t landed;                                 // chunks whose copies are there
   __shared__ int abort_flag;
   __shared__ int eA[OZ_M], eB[OZ_N];                          // row scales 2^e
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int mt, nt;
   tiles.at(blockIdx.x, mt, nt);
   const int m0 = mt * OZ_M, n0 = nt * OZ_N;
-  const int k0 = blockIdx.y * k_per_split;
-  int k1 = min(K, k0 + k_per_split);
-  if (b_lower) k1 = min(k1, n0 + OZ_N);                       // B(n, k) = 0 for k > n
-  const int nq = k1 > k0 ? (k1 - k0 + OZ_K - 1) / OZ_K : 0;  // chunks
+  const int c0 = blockIdx.y * g.split_chunks;
+  int c1 = min(g.chunks, c0 + g.split_chunks);
+  if (g.b_lower_k0 >= 0) c1 = min(c1, max(0, n0 + OZ_N - g.b_lower_k0 + OZ_K - 1) / OZ_K);
+  const int nq = max(0, c1 - c0);                             // chunks
   const int ng = (nq + kGroupChunks - 1) / kGroupChunks;      // groups
+  const int nh = n0 + OZ_H < g.N ? 2 : 1;                     // halves with columns
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -253,29 +379,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_ozgemm(
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 32) {
-    for (int s = 0; s < kRawStages; ++s) {
-      bar_init(&raw_full[s], 1);
-      bar_init(&raw_empty[s], kConvWarps);
-    }
-    for (int s = 0; s < kSplStages; ++s) {
-      bar_init(&spl_full[s], kConvWarps);
-      bar_init(&spl_empty[s], 1);
+    for (int s = 0; s < kStages; ++s) {
+      bar_init(&full[s], 1);
+      bar_init(&empty[s], nh);
     }
     for (int b = 0; b < 2; ++b) {
       bar_init(&acc_full[b], 1);
       bar_init(&acc_empty[b], kEpiWarps);
+      bar_init(&fin[b], 1);
     }
-    bar_init(&fin, 1);
-    ready = 0;
     landed = 0;
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int i = tid; i < OZ_M; i += blockDim.x) {
-    eA[i] = m0 + i < M ? __ldg(expA + m0 + i) : 0;
-  }
-  for (int i = tid; i < OZ_N; i += blockDim.x) {
-    eB[i] = n0 + i < N ? __ldg(expB + n0 + i) : 0;
+  for (int i = tid; i < OZ_M + OZ_N; i += kThreads) {
+    if (i < OZ_M) eA[i] = m0 + i < g.M ? exp_of_bits(__ldg(g.ea + m0 + i)) : 0;
+    else eB[i - OZ_M] = n0 + i - OZ_M < g.N ? exp_of_bits(__ldg(g.eb + n0 + i - OZ_M)) : 0;
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -285,42 +404,47 @@ __global__ void __launch_bounds__(kThreads, 1) k_ozgemm(
   bool ok = true;
 
   if (warp == 0) {
-    // ---- TMA producer
+    // ---- copies of chunk q into stage q % kStages once chunk q - kStages has
+    // been multiplied by both halves: A's six planes are one piece, the six
+    // 1 KB pieces of a half of B one tensor copy
     if (lane == 0) {
+      const unsigned char* src = g.pa + ((int64_t)mt * g.chunks + c0) * kStageA;
+      const int bz = (n0 >> 7) * g.chunks + c0, bx = (n0 & 127) * 4;
       int q = 0;
       for (; q < nq; ++q) {
-        const int s = q % kRawStages;
-        if (q >= kRawStages &&
-            !bar_wait(&raw_empty[s], (uint32_t)((q / kRawStages - 1) & 1), abrt, 32)) {
-          ok = false;
-          break;
+        const int s = q % kStages;
+        if (q >= kStages) {
+          const uint32_t par = (uint32_t)((q / kStages - 1) & 1);
+          if (!bar_wait(&empty[s], par, abrt, 0)) {
+            ok = false;
+            break;
+          }
+          // the stage's previous copies must have landed before it is armed again
+          if (!bar_test(&full[s], par)) {
+            atomicExch(err, 3);
+            ok = false;
+            *abrt = 1;
+            break;
+          }
         }
-        // the stage's previous copy must have landed before it is armed again
-        if (q >= kRawStages && !bar_test(&raw_full[s], (uint32_t)((q / kRawStages - 1) & 1))) {
-          atomicExch(err, 3);
-          ok = false;
-          *abrt = 1;
-          break;
-        }
-        const uint32_t fb = su32(&raw_full[s]);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb),
-                     "r"(kRawStage) : "memory");
-        const uint32_t dst = su32(raw + s * kRawStage);
-        const int kc = k0 + q * OZ_K;
-        if (A_MN) tma_load(dst, &tmA, m0, kc, 0, false, fb);
-        else tma_load(dst, &tmA, kc, m0, 0, false, fb);
-        if (B_MN) tma_load(dst + kRawA, &tmB, n0, kc, 0, false, fb);
-        else tma_load(dst + kRawA, &tmB, kc, n0, 0, false, fb);
+        const uint32_t fb = su32(&full[s]), dst = su32(smem) + s * kStage;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                     ::"r"(fb), "r"(kStageA + nh * kStageH) : "memory");
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+            ::"r"(dst), "l"(src + (int64_t)q * kStageA), "r"(kStageA), "r"(fb) : "memory");
+        for (int h = 0; h < nh; ++h)
+          tma_load(dst + kStageA + h * kStageH, &tmB, bx + h * OZ_H * 4, 0, bz + q, true, fb);
       }
       if (!ok)
-        for (int r = (q > kRawStages ? q - kRawStages : 0); r < q; ++r)
-          bar_drain(&raw_full[r % kRawStages], (uint32_t)((r / kRawStages) & 1));
+        for (int r = (q > kStages ? q - kStages : 0); r < q; ++r)
+          bar_drain(&full[r % kStages], (uint32_t)((r / kStages) & 1));
     }
-  } else if (warp == 3) {
-    // ---- raw copies landed, in order
+  } else if (warp == 2) {
+    // ---- chunks landed, in order
     if (lane == 0) {
       for (int q = 0; q < nq; ++q) {
-        if (!bar_wait(&raw_full[q % kRawStages], (uint32_t)((q / kRawStages) & 1), abrt, 32)) {
+        if (!bar_wait(&full[q % kStages], (uint32_t)((q / kStages) & 1), abrt, 0)) {
           ok = false;
           break;
         }
@@ -328,161 +452,121 @@ __global__ void __launch_bounds__(kThreads, 1) k_ozgemm(
                      "r"((uint32_t)(q + 1)) : "memory");
       }
     }
-  } else if (warp >= kConvWarp0 && warp < kConvWarp0 + kConvWarps) {
-    // ---- digit planes: every converter warp takes its share of the rows of
-    // every chunk (row blocks of 8: cw, cw + 8, ...), so a chunk's raw stage
-    // is released after an eighth of the work; each warp waits on every phase
-    // of the barriers it uses, in order
-    const int cw = warp - kConvWarp0;
-    for (int q = 0; q < nq; ++q) {
-      const int s = q % kRawStages, s2 = q % kSplStages;
-      bool w = true;
-      if (lane == 0) {
-        w = false;
-        for (int i = 0; i < kTcMaxWait; ++i) {
-          uint32_t l;
-          asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(l) : "r"(su32(&landed))
-                       : "memory");
-          if (l > (uint32_t)q) { w = true; break; }
-          if (*abrt) break;
-          __nanosleep(32);
-        }
-        if (!w) *abrt = 1;
-        if (w && q >= kSplStages)
-          w = bar_wait(&spl_empty[s2], (uint32_t)((q / kSplStages - 1) & 1), abrt, 32);
-      }
-      w = __shfl_sync(0xffffffffu, w, 0);
-      if (!w) { ok = false; break; }
-      const double* ra = reinterpret_cast<const double*>(raw + s * kRawStage);
-      const double* rb = reinterpret_cast<const double*>(raw + s * kRawStage + kRawA);
-      unsigned char* dst = spl + s2 * kSplStage;
-      for (int blk = cw; blk < (OZ_M + OZ_N) / 8; blk += kConvWarps) {
-        // K scales of this chunk (K values beyond the operands are zero)
-        const int* kq = kexp ? kexp + (k0 + q * OZ_K) : nullptr;
-        if (blk < OZ_M / 8) slice_block<OZ_M, A_MN>(ra, eA, dst, kPlA, blk, lane, kq, -1);
-        else slice_block<OZ_N, B_MN>(rb, eB, dst + kDigits * kPlA, kPlB, blk - OZ_M / 8, lane, kq,
-                                     1);
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) {
-        bar_arrive(&raw_empty[s]);
-        bar_arrive(&spl_full[s2]);
-      }
-    }
-  } else if (warp == 2) {
-    // ---- digit planes ready (and accumulator buffers emptied), in order
-    if (lane == 0) {
-      for (int q = 0; q < nq && ok; ++q) {
-        const int g = q / kGroupChunks;
-        if (q % kGroupChunks == 0 && g >= 2 &&
-            !bar_wait(&acc_empty[g & 1], (uint32_t)(((g >> 1) - 1) & 1), abrt, 32)) {
-          ok = false;
-          break;
-        }
-        if (!bar_wait(&spl_full[q % kSplStages], (uint32_t)((q / kSplStages) & 1), abrt, 16)) {
-          ok = false;
-          break;
-        }
-        asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(su32(&ready)),
-                     "r"((uint32_t)(q + 1)) : "memory");
-      }
-    }
-  } else if (warp == 1) {
-    // ---- MMA issue: 21 digit products per chunk into six level accumulators
-    if (lane == 0) {
-      const uint32_t idesc = idesc_oz();
-      const uint32_t spl0 = su32(spl);
+  } else if (warp == 1 || warp == 3) {
+    // ---- MMAs of one half: digit i of A times digits 0 .. 5 - i of B in one
+    const int h = warp >> 1;
+    if (lane == 0 && h < nh) {
+      const uint32_t base0 = su32(smem), dcol = tmem + (uint32_t)(h * kHalfCols);
       uint32_t avail = 0;
       for (int q = 0; q < nq; ++q) {
-        const int g = q / kGroupChunks, c = q % kGroupChunks;
-        const uint32_t dbuf = tmem + (uint32_t)((g & 1) * kBufCols);
+        const int gr = q / kGroupChunks, c = q % kGroupChunks, s = q % kStages;
+        // the group's accumulators emptied (its own MMAs are long done by then)
+        if (c == 0 && gr > 0 && !bar_wait(&acc_empty[h], (uint32_t)((gr - 1) & 1), abrt, 0)) {
+          ok = false;
+          break;
+        }
         for (int i = 0; i < kTcMaxWait && avail <= (uint32_t)q; ++i) {
           asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(avail)
-                       : "r"(su32(&ready)) : "memory");
+                       : "r"(su32(&landed)) : "memory");
           if (avail > (uint32_t)q || *abrt) break;
-          __nanosleep(16);
         }
         if (avail <= (uint32_t)q) { ok = false; *abrt = 1; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t base = spl0 + (uint32_t)((q % kSplStages) * kSplStage);
-        int p = 0;
+        const uint32_t base = base0 + (uint32_t)(s * kStage);
+        const uint64_t db = kmajor_desc(base + kStageA + h * kStageH);
 #pragma unroll
-        for (int L = kLevels - 1; L >= 0; --L) {
-#pragma unroll
-          for (int i = 0; i <= L; ++i, ++p) {
-            const int j = L - i;
-            const uint64_t da = kmajor_desc(base + i * kPlA);
-            const uint64_t db = kmajor_desc(base + kDigits * kPlA + j * kPlB);
-            const uint32_t acc = (c > 0 || i > 0) ? 1u : 0u;
-            asm volatile(
-                "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                ::"r"(dbuf + (uint32_t)(L * OZ_N)), "l"(da), "l"(db), "r"(idesc), "r"(acc));
-          }
+        for (int i = 0; i < kDigits; ++i) {
+          const uint64_t da = kmajor_desc(base + i * kPlA);
+          const uint32_t acc = (c > 0 || i > 0) ? 1u : 0u;
+          asm volatile(
+              "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+              ::"r"(dcol + (uint32_t)(i * OZ_H)), "l"(da), "l"(db),
+                "r"(idesc_oz(OZ_H * (kDigits - i))), "r"(acc));
         }
         asm volatile(
             "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-            ::"r"(su32(&spl_empty[q % kSplStages])) : "memory");
+            ::"r"(su32(&empty[s])) : "memory");
         if (c == kGroupChunks - 1 || q == nq - 1)
           asm volatile(
               "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-              ::"r"(su32(&acc_full[g & 1])) : "memory");
+              ::"r"(su32(&acc_full[h])) : "memory");
       }
       asm volatile(
           "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-          ::"r"(su32(&fin)) : "memory");
-      bar_drain(&fin, 0);
+          ::"r"(su32(&fin[h])) : "memory");
+      bar_drain(&fin[h], 0);
     }
-  } else if (warp >= kEpiWarp0) {
-    // ---- epilogue: TMEM lanes 32 (warp & 3) .., all 32 columns
-    const int qd = warp & 3;
+  } else if (warp >= kEpiWarp0 && (warp - kEpiWarp0) / kEpiWarps < nh) {
+    // ---- fold of half a tile: TMEM lanes 32 (warp & 3) .., 16 columns a warp
+    // (two warps per lane quarter: each waits on its tensor-memory loads)
+    const int h = (warp - kEpiWarp0) / kEpiWarps, qd = warp & 3;
+    const int cb = (((warp - kEpiWarp0) >> 2) & 1) * OZ_E;
     const int row = qd * 32 + lane;
-    const uint32_t lanes = (uint32_t)(qd * 32) << 16;
-    float hi[OZ_N], lo[OZ_N];
+    const uint32_t acol = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(h * kHalfCols + cb);
+    float hi[OZ_E], lo[OZ_E];
 #pragma unroll
-    for (int c = 0; c < OZ_N; ++c) { hi[c] = 0.f; lo[c] = 0.f; }
-    for (int g = 0; g < ng; ++g) {
-      if (!bar_wait(&acc_full[g & 1], (uint32_t)((g >> 1) & 1), abrt, 64)) { ok = false; break; }
+    for (int c = 0; c < OZ_E; ++c) { hi[c] = 0.f; lo[c] = 0.f; }
+    for (int gr = 0; gr < ng; ++gr) {
+      // one lane polls: 512 threads on two barriers would slow every wait
+      bool w = true;
+      if (lane == 0) w = bar_wait(&acc_full[h], (uint32_t)(gr & 1), abrt, 32);
+      ok = __shfl_sync(0xffffffffu, w, 0);
+      if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t acol = tmem + lanes + (uint32_t)((g & 1) * kBufCols);
 #pragma unroll
-      for (int c0 = 0; c0 < OZ_N; c0 += 8) {
+      for (int cc = 0; cc < OZ_E; cc += 8) {
         float S[kLevels][8];
-        tmem_ld8x3(acol + c0, acol + OZ_N + c0, acol + 2 * OZ_N + c0, S[0], S[1], S[2]);
-        tmem_ld8x3(acol + 3 * OZ_N + c0, acol + 4 * OZ_N + c0, acol + 5 * OZ_N + c0, S[3], S[4],
+        tmem_ld8x3(acol + cc, acol + OZ_H + cc, acol + 2 * OZ_H + cc, S[0], S[1], S[2]);
+        tmem_ld8x3(acol + 3 * OZ_H + cc, acol + 4 * OZ_H + cc, acol + 5 * OZ_H + cc, S[3], S[4],
                    S[5]);
+        if (cc + 8 == OZ_E) {              // the last loads are in registers: release the buffer
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) bar_arrive(&acc_empty[h]);
+        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          // S0 + S1 2^-8 + ... + S5 2^-40 as (h, l), then into (hi, lo)
-          float h = S[0][i], l = 0.f;
+          // S0 + S1 2^-8 + ... + S5 2^-40 as (f, l), then into (hi, lo)
+          float f = S[0][i], l = 0.f;
           float sc = 1.f / 256.f;
 #pragma unroll
           for (int L = 1; L < kLevels; ++L, sc *= (1.f / 256.f)) {
             const float t = S[L][i] * sc;
-            const float h2 = h + t;
-            const float bv = h2 - h;
-            l += (h - (h2 - bv)) + (t - bv);
-            h = h2;
+            const float h2 = f + t;
+            const float bv = h2 - f;
+            l += (f - (h2 - bv)) + (t - bv);
+            f = h2;
           }
-          const float sum = hi[c0 + i] + h;
-          const float bv = sum - hi[c0 + i];
-          lo[c0 + i] += (hi[c0 + i] - (sum - bv)) + (h - bv) + l;
-          hi[c0 + i] = sum;
+          const float sum = hi[cc + i] + f;
+          const float bv = sum - hi[cc + i];
+          lo[cc + i] += (hi[cc + i] - (sum - bv)) + (f - bv) + l;
+          hi[cc + i] = sum;
         }
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) bar_arrive(&acc_empty[g & 1]);
     }
-    if (ok && m0 + row < M) {
-      const int em = eA[row];
+    if (ok && m0 + row < g.M) {
+      const int em = eA[row] - 16;
+      const int64_t m = g.row0 + m0 + row;
+      const int nb = n0 + h * OZ_H + cb;
+      double* o = out.p + blockIdx.y * out.zs + nb * out.cs +
+                  (m < out.rin ? m * out.rs : (m % out.rin) * out.rs + (m / out.rin) * out.rs2);
+      const bool pairs = out.cs == 1 && !out.accumulate && (reinterpret_cast<uintptr_t>(o) & 15) == 0;
 #pragma unroll
-      for (int c = 0; c < OZ_N; ++c) {
-        const int n = n0 + c;
-        if (n < N) {
-          const double v = ((double)hi[c] + (double)lo[c]) * ldexp(1.0, em + eB[c] - 16);
-          out[(int64_t)blockIdx.y * o_zs + (int64_t)(m0 + row) * o_rs + (int64_t)n * o_cs] = v;
+      for (int c = 0; c < OZ_E; c += 2) {
+        double v[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          v[u] = scaled_sum(hi[c + u], lo[c + u], em + eB[h * OZ_H + cb + c + u]);
+        if (pairs && nb + c + 1 < g.N) {
+          *reinterpret_cast<double2*>(o + c) = make_double2(v[0], v[1]);
+        } else {
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+            if (nb + c + u < g.N) {
+              double* t = o + (c + u) * out.cs;
+              *t = out.accumulate ? *t + v[u] : v[u];
+            }
         }
       }
     }
@@ -497,65 +581,34 @@ __global__ void __launch_bounds__(kThreads, 1) k_ozgemm(
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
-// Row scales: e[r] with max_k |A(r, k)| < 2^e[r] (0 for an all-zero row), from
-// the largest biased exponent of the row: any v with biased exponent E is
-// below 2^(E - 1022).  ebits[r] (zeroed by the caller) collects the maxima.
-// With K scales (kexp, ksign): the biased exponent of v 2^(ksign kexp[k]).
-__device__ __forceinline__ int scaled_ebits(double v, const int* kexp, int ksign, int64_t k) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-  int E = (int)((b >> 52) & 0x7FF);
-  if (E != 0 && E != 0x7FF && kexp) E = max(0, min(2046, E + ksign * __ldg(kexp + k)));
-  return E;
-}
-
-__global__ void k_rowexp_mn(const double* __restrict__ p, int64_t rows, int64_t kext, int64_t ld,
-                            int64_t k_per_block, const int* __restrict__ kexp, int ksign,
-                            int* __restrict__ ebits) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= rows) return;
-  const int64_t k0 = (int64_t)blockIdx.y * k_per_block;
-  const int64_t k1 = min(kext, k0 + k_per_block);
-  int m = 0;
-  for (int64_t k = k0; k < k1; ++k) m = max(m, scaled_ebits(p[k * ld + r], kexp, ksign, k));
-  if (m) atomicMax(ebits + r, m);
-}
-
-// K-major rows: one warp per row
-__global__ void k_rowexp_k(const double* __restrict__ p, int64_t rows, int64_t kext, int64_t ld,
-                           const int* __restrict__ kexp, int ksign, int* __restrict__ ebits) {
-  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (r >= rows) return;
-  int m = 0;
-  for (int64_t k = lane; k < kext; k += 32) m = max(m, scaled_ebits(p[r * ld + k], kexp, ksign, k));
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (lane == 0) ebits[r] = m;
-}
-
-__global__ void k_exp_from_bits(int* __restrict__ e, int64_t n) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    const int b = e[i];
-    // a NaN or Inf row (b = 2047) keeps a large scale: its digits are NaN anyway
-    e[i] = b == 0 ? 0 : min(b, 2046) - 1022;
-  }
-}
-
 // S = sum of the split partials (column-major M x N); sym: tiles above the
-// diagonal were not computed, S[m, n] is read from [n, m] there.
-__global__ void k_oz_reduce(const double* __restrict__ part, int nsplit, int M, int N, int sym,
-                            double* __restrict__ C, int64_t c_rs, int64_t c_cs) {
+// diagonal were not computed, S[m, n] is read from [n, m] there.  Eight
+// threads share an element's splits (fixed order), 32 elements a block.
+__global__ void __launch_bounds__(256) k_oz_reduce(const double* __restrict__ part, int nsplit,
+                                                   int M, int N, int sym, double* __restrict__ C,
+                                                   int64_t c_rs, int64_t c_cs) {
+  __shared__ double red[8][33];
   const int64_t mn = (int64_t)M * N;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < mn;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int m = (int)(i % M), n = (int)(i / M);
-    int64_t src = i;
-    if (sym && (n / OZ_N) * OZ_N > (m / OZ_M) * OZ_M + OZ_M - 1) src = n + (int64_t)m * M;
+  for (int64_t b = blockIdx.x; b * 32 < mn; b += gridDim.x) {
+    const int64_t i = b * 32 + threadIdx.x;
     double s = 0.0;
-    for (int z = 0; z < nsplit; ++z) s += part[(int64_t)z * mn + src];
-    C[m * c_rs + n * c_cs] = s;
+    const int m = (int)(i % M), n = (int)(i / M);
+    if (i < mn) {
+      int64_t src = i;
+      if (sym && (n / OZ_N) * OZ_N > (m / OZ_M) * OZ_M + OZ_M - 1) src = n + (int64_t)m * M;
+      for (int z = threadIdx.y; z < nsplit; z += 8) s += part[(int64_t)z * mn + src];
+    }
+    red[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.y == 0 && i < mn) {
+      for (int y = 1; y < 8; ++y) s += red[y][threadIdx.x];
+      C[m * c_rs + n * c_cs] = s;
+    }
+    __syncthreads();
   }
 }
+
+int64_t rup(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static std::once_flag once;
@@ -573,74 +626,57 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-bool map_ok(const OzOperand& o) {
-  return o.p && o.rows > 0 && o.kext > 0 && (o.ld * 8) % 16 == 0 &&
-         (reinterpret_cast<uintptr_t>(o.p) & 15) == 0 &&
-         (o.mn_major ? o.ld >= o.rows : o.ld >= o.kext);
-}
-
-ttg_status make_map(CUtensorMap* map, const OzOperand& o, int box_rows) {
+// B's planes as (8-byte words of a 4 KB plane, digit, 128-row block and chunk);
+// a box is 32 rows (1 KB) of all six digits
+ttg_status plane_map(CUtensorMap* map, const unsigned char* planes, int64_t blocks) {
   auto fn = encode_fn();
   if (!fn) return TTG_CUDA_ERR;
-  cuuint64_t dims[2], strides[1] = {(cuuint64_t)o.ld * 8};
-  cuuint32_t box[2], es[2] = {1, 1};
-  if (o.mn_major) {
-    dims[0] = (cuuint64_t)o.rows;
-    dims[1] = (cuuint64_t)o.kext;
-    box[0] = (cuuint32_t)box_rows;
-    box[1] = (cuuint32_t)OZ_K;
-  } else {
-    dims[0] = (cuuint64_t)o.kext;
-    dims[1] = (cuuint64_t)o.rows;
-    box[0] = (cuuint32_t)OZ_K;
-    box[1] = (cuuint32_t)box_rows;
-  }
-  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<double*>(o.p), dims,
-                        strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  cuuint64_t dims[3] = {kPlA / 8, kDigits, (cuuint64_t)blocks};
+  cuuint64_t strides[2] = {kPlA, kStageA};
+  cuuint32_t box[3] = {kPlH / 8, kDigits, 1}, es[3] = {1, 1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<unsigned char*>(planes),
+                        dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? TTG_OK : TTG_BAD_ARG;
 }
 
-ttg_status row_exps(cudaStream_t st, const OzOperand& o, int* e, const int* kexp = nullptr,
-                    int ksign = 0) {
-  TTG_CUDA_TRY(cudaMemsetAsync(e, 0, (size_t)o.rows * sizeof(int), st));
-  if (o.mn_major) {
-    const int64_t kb = 256;                 // enough CTAs for a narrow block of many rows
-    dim3 grid((unsigned)((o.rows + 255) / 256), (unsigned)((o.kext + kb - 1) / kb));
-    k_rowexp_mn<<<grid, 256, 0, st>>>(o.p, o.rows, o.kext, o.ld, kb, kexp, ksign, e); TTG_COUNT();
+bool rows_fast(const OzOperand& o) { return o.rs == 1 && o.ks != 1; }
+
+bool same_operand(const OzOperand& a, const OzOperand& b) {
+  return a.p == b.p && a.rows == b.rows && a.kext == b.kext && a.rin == b.rin && a.rs == b.rs &&
+         a.rs2 == b.rs2 && a.kin == b.kin && a.ks == b.ks && a.ks2 == b.ks2;
+}
+
+ttg_status row_exps(cudaStream_t st, const OzSlices& S, int nz, const int* kexp, int ksign) {
+  const OzOperand& o = S.o[0];
+  for (int z = 0; z < nz; ++z)
+    TTG_CUDA_TRY(cudaMemsetAsync(S.ebits[z], 0, (size_t)o.rows * sizeof(int), st));
+  if (rows_fast(o)) {
+    int64_t kb = 128;            // values of K a block: many blocks for a narrow operand
+    while ((o.kext + kb - 1) / kb > 8192) kb *= 2;
+    k_rowexp_rows<<<dim3((unsigned)((o.rows + 31) / 32), (unsigned)((o.kext + kb - 1) / kb), nz),
+                    dim3(32, 8), 0, st>>>(S, kb, kexp, ksign); TTG_COUNT();
   } else {
-    k_rowexp_k<<<(unsigned)((o.rows * 32 + 255) / 256), 256, 0, st>>>(o.p, o.rows, o.kext, o.ld,
-                                                                     kexp, ksign, e); TTG_COUNT();
+    int64_t kb = 4096;
+    while ((o.kext + kb - 1) / kb > 8192) kb *= 2;
+    k_rowexp_k<<<dim3((unsigned)((o.rows + 7) / 8), (unsigned)((o.kext + kb - 1) / kb), nz), 256,
+                 0, st>>>(S, kb, kexp, ksign); TTG_COUNT();
   }
-  TTG_CUDA_TRY(cudaGetLastError());
-  k_exp_from_bits<<<(unsigned)((o.rows + 255) / 256), 256, 0, st>>>(e, o.rows); TTG_COUNT();
   TTG_CUDA_TRY(cudaGetLastError());
   return TTG_OK;
 }
 
-template <int A_MN, int B_MN>
-ttg_status launch(dim3 grid, cudaStream_t st, const CUtensorMap& ma, const CUtensorMap& mb,
-                  const int* ea, const int* eb, int M, int N, int K, int kps, int b_lower,
-                  OzTiles tiles, double* out, int64_t o_rs, int64_t o_cs, int64_t o_zs,
-                  const int* kexp, int* err) {
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(k_ozgemm<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kSmem);
-  });
-  if (attr != cudaSuccess) return TTG_CUDA_ERR;
-  k_ozgemm<A_MN, B_MN><<<grid, kThreads, kSmem, st>>>(ma, mb, ea, eb, M, N, K, kps, b_lower,
-                                                     tiles, out, o_rs, o_cs, o_zs, kexp, err);
+ttg_status slice(cudaStream_t st, const OzSlices& S, int nz, int64_t r0, int64_t rpad, int64_t k0,
+                 int64_t chunks, const int* kexp, int ksign) {
+  if (chunks <= 0) return TTG_OK;
+  const dim3 grid((unsigned)chunks, (unsigned)(rpad / 128), nz);
+  if (rows_fast(S.o[0]))
+    k_oz_slice<true><<<grid, 256, 0, st>>>(S, r0, k0, kexp, ksign);
+  else
+    k_oz_slice<false><<<grid, 256, 0, st>>>(S, r0, k0, kexp, ksign);
   TTG_COUNT();
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess && sync_launches()) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) {
-    fprintf(stderr, "ttg: k_ozgemm<%d, %d> (M %d, N %d, K %d) failed: %s\n", A_MN, B_MN, M, N, K,
-            cudaGetErrorString(e));
-    return TTG_CUDA_ERR;
-  }
+  TTG_CUDA_TRY(cudaGetLastError());
   return TTG_OK;
 }
 
@@ -648,16 +684,44 @@ ttg_status launch(dim3 grid, cudaStream_t st, const CUtensorMap& ma, const CUten
 
 bool ozgemm_supported(const OzOperand& A, const OzOperand& B) {
   if (getenv("TTG_DISABLE_OZGEMM")) return false;
-  return map_ok(A) && map_ok(B) && A.kext == B.kext && A.rows <= INT32_MAX &&
-         B.rows <= INT32_MAX && A.kext <= INT32_MAX;
+  return A.p && B.p && A.rows > 0 && B.rows > 0 && A.kext > 0 && A.kext == B.kext &&
+         A.rows <= INT32_MAX - 256 && B.rows <= INT32_MAX - 256 && A.kext <= INT32_MAX - 256;
 }
 
-ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C, int64_t c_rs,
-                  int64_t c_cs, bool sym, bool b_lower, const OzOperand* kscale_of) {
+ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C, OzLayout c,
+                  bool sym, bool b_lower, const OzOperand* kscale_of) {
   if (!ozgemm_supported(A, B) || !C) return TTG_BAD_ARG;
-  if (sym && A.rows != B.rows) return TTG_BAD_ARG;
+  if (sym && (A.rows != B.rows || c.rin < A.rows)) return TTG_BAD_ARG;
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  std::call_once(once, [] {
+    attr = cudaFuncSetAttribute(k_oz_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  });
+  if (attr != cudaSuccess) return TTG_CUDA_ERR;
   cudaStream_t st = op->stream;
-  const int M = (int)A.rows, N = (int)B.rows, K = (int)A.kext;
+  const int64_t M = A.rows, N = B.rows, K = A.kext;
+  const int64_t mpad = rup(M, kRowPad), npad = rup(N, kRowPad), chunks = (K + OZ_K - 1) / OZ_K;
+  const bool same = !kscale_of && same_operand(A, B);
+  // Slabs that keep the digit planes within the workspace: of A's rows when
+  // B's planes take a quarter of it at most (N x k products), else of K
+  // (Gram matrices), whole groups at a time.
+  const int64_t per_chunk = kDigits * 32;                       // bytes of a row's chunk
+  const int64_t bytes_a = mpad * chunks * per_chunk, bytes_b = same ? 0 : npad * chunks * per_chunk;
+  int64_t mslab = mpad, kslab = chunks;                          // rows, chunks
+  if (bytes_a + bytes_b > kPlaneBudget) {
+    if (!sym && !same && bytes_b <= kPlaneBudget / 4) {
+      mslab = std::max<int64_t>(1, (kPlaneBudget - bytes_b) / (chunks * per_chunk) / kRowPad) * kRowPad;
+    } else {
+      const int64_t rows = same ? mpad : mpad + npad;
+      kslab = std::max<int64_t>(1, kPlaneBudget / (rows * per_chunk) / kGroupChunks) * kGroupChunks;
+    }
+    mslab = std::min(mslab, mpad);
+    kslab = std::min(kslab, chunks);
+  }
+  const int64_t need_a = mslab * kslab * per_chunk, need_b = same ? 0 : npad * kslab * per_chunk;
+  if (op->oz_planes.bytes < (size_t)(need_a + need_b)) TTG_TRY(op->oz_planes.alloc(need_a + need_b));
+  unsigned char* pa = op->oz_planes.as<unsigned char>();
+  unsigned char* pb = same ? pa : pa + need_a;
   if (op->oz_exp.bytes < (size_t)(M + N) * sizeof(int))
     TTG_TRY(op->oz_exp.alloc((size_t)(M + N) * sizeof(int)));
   if (!op->oz_err.p) {
@@ -665,67 +729,104 @@ ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C,
     TTG_CUDA_TRY(cudaMemsetAsync(op->oz_err.p, 0, sizeof(int), st));
   }
   int* ea = op->oz_exp.as<int>();
-  int* eb = ea + M;
-  // K scales: the row scales of kscale_of (an MN-major view whose rows are
-  // the K index), A scaled by 2^-f_k and B by 2^f_k; the buffer is padded
-  // with zeros to whole chunks
+  int* eb = same ? ea : ea + M;
+  int* err = op->oz_err.as<int>();
+  // K scales: the row scales of kscale_of (a view whose rows are the K
+  // index), A scaled by 2^-f_k and B by 2^f_k; the buffer is padded with zeros
+  // to whole chunks
   const int* kexp = nullptr;
   if (kscale_of) {
     if (kscale_of->rows != K) return TTG_BAD_ARG;
-    const size_t kb = (size_t)((K + OZ_K - 1) / OZ_K * OZ_K) * sizeof(int);
+    const size_t kb = (size_t)(chunks * OZ_K) * sizeof(int);
     if (op->oz_kexp.bytes < kb) TTG_TRY(op->oz_kexp.alloc(kb));
     TTG_CUDA_TRY(cudaMemsetAsync(op->oz_kexp.p, 0, kb, st));
-    TTG_TRY(row_exps(st, *kscale_of, op->oz_kexp.as<int>()));
+    OzSlices S{};
+    S.o[0] = *kscale_of;
+    S.ebits[0] = op->oz_kexp.as<int>();
+    TTG_TRY(row_exps(st, S, 1, nullptr, 0));
+    k_exp_from_bits<<<(unsigned)((K + 255) / 256), 256, 0, st>>>(op->oz_kexp.as<int>(), K); TTG_COUNT();
+    TTG_CUDA_TRY(cudaGetLastError());
     kexp = op->oz_kexp.as<int>();
   }
-  TTG_TRY(row_exps(st, A, ea, kexp, -1));
-  if (!kexp && B.p == A.p && B.rows == A.rows && B.kext == A.kext && B.ld == A.ld &&
-      B.mn_major == A.mn_major)
-    TTG_CUDA_TRY(cudaMemcpyAsync(eb, ea, (size_t)M * sizeof(int), cudaMemcpyDeviceToDevice, st));
-  else
-    TTG_TRY(row_exps(st, B, eb, kexp, 1));
-  CUtensorMap ma, mb;
-  TTG_TRY(make_map(&ma, A, OZ_M));
-  TTG_TRY(make_map(&mb, B, OZ_N));
-  OzTiles tiles{(M + OZ_M - 1) / OZ_M, (N + OZ_N - 1) / OZ_N, sym ? 1 : 0};
-  int64_t ntiles = (int64_t)tiles.tiles_m * tiles.tiles_n;
+  // both operands in one launch where they have one shape and orientation
+  const bool pair = !same && !kexp && M == N && rows_fast(A) == rows_fast(B);
+  OzSlices SA{}, SB{};
+  SA.o[0] = A;
+  SA.ebits[0] = ea;
+  SA.planes[0] = pa;
+  SB.o[0] = B;
+  SB.ebits[0] = eb;
+  SB.planes[0] = pb;
+  if (pair) {
+    SA.o[1] = B;
+    SA.ebits[1] = eb;
+    SA.planes[1] = pb;
+  }
+  TTG_TRY(row_exps(st, SA, pair ? 2 : 1, kexp, -1));
+  if (!same && !pair) TTG_TRY(row_exps(st, SB, 1, kexp, 1));
+  const int tiles_n = (int)((N + OZ_N - 1) / OZ_N);
+  OzTiles tiles{(int)((std::min(mslab, M) + OZ_M - 1) / OZ_M), tiles_n, sym ? 1 : 0};
+  int64_t ntiles = (int64_t)tiles.tiles_m * tiles_n;
   if (sym) {
     ntiles = 0;
-    for (int m = 0; m < tiles.tiles_m; ++m) ntiles += std::min(4 * m + 4, tiles.tiles_n);
+    for (int m = 0; m < tiles.tiles_m; ++m) ntiles += std::min(2 * m + 2, tiles_n);
   }
-  // split K so that the CTAs (one per SM) fill the GPU a few times over
-  const int groupk = kGroupChunks * OZ_K;
-  const int64_t kgroups = (K + groupk - 1) / groupk;
-  int nsplit = (int)std::max<int64_t>(1, std::min<int64_t>(kgroups, (4 * 152 + ntiles - 1) / ntiles));
-  if (b_lower) nsplit = 1;
-  const int kps = (int)(((kgroups + nsplit - 1) / nsplit) * groupk);
-  nsplit = (int)((K + kps - 1) / kps);
-  double* out = C;
-  int64_t o_rs = c_rs, o_cs = c_cs;
-  if (nsplit > 1 || sym) {
+  // Split K for the least time: waves of CTAs (one per SM) times their groups
+  // (about 1.2 us each, three more to start and to store), plus the partials
+  // written and summed.
+  const int64_t kgroups = (kslab + kGroupChunks - 1) / kGroupChunks;
+  int64_t nsplit = 1;
+  if (!b_lower && c.rin >= M) {
+    double best = 1e300;
+    for (int64_t t = 1; t <= std::min<int64_t>(kgroups, 8 * 152 / ntiles + 1); ++t) {
+      const double cost = (double)((ntiles * t + 151) / 152) * ((kgroups + t - 1) / t + 3) +
+                          (t > 1 || sym ? t * (double)M * N * 16 / 7e6 : 0.0);
+      if (cost < best) {
+        best = cost;
+        nsplit = t;
+      }
+    }
+  }
+  const int64_t sgroups = (kgroups + nsplit - 1) / nsplit;
+  nsplit = (kgroups + sgroups - 1) / sgroups;
+  if (ntiles > INT32_MAX || nsplit > 65535 || mslab / 128 > 65535 || npad / 128 > 65535)
+    return TTG_BAD_ARG;
+  OzOut out{C, c.rin, c.rs, c.rs2, c.cs, 0, 0};
+  const bool partial = nsplit > 1 || sym;
+  if (partial) {
     const size_t need = (size_t)nsplit * M * N * sizeof(double);
     if (op->partial.bytes < need) TTG_TRY(op->partial.alloc(need));
-    out = op->partial.as<double>();
-    o_rs = 1;
-    o_cs = M;
+    out = OzOut{op->partial.as<double>(), M, 1, 0, M, M * N, 0};
   }
-  if (ntiles > INT32_MAX || nsplit > 65535) return TTG_BAD_ARG;
-  const dim3 grid((unsigned)ntiles, (unsigned)nsplit);
-  const int64_t zs = (out == C) ? 0 : (int64_t)M * N;
-  int* err = op->oz_err.as<int>();
-  const int bl = b_lower ? 1 : 0;
-  if (A.mn_major && B.mn_major)
-    TTG_TRY((launch<1, 1>(grid, st, ma, mb, ea, eb, M, N, K, kps, bl, tiles, out, o_rs, o_cs, zs, kexp, err)));
-  else if (A.mn_major)
-    TTG_TRY((launch<1, 0>(grid, st, ma, mb, ea, eb, M, N, K, kps, bl, tiles, out, o_rs, o_cs, zs, kexp, err)));
-  else if (B.mn_major)
-    TTG_TRY((launch<0, 1>(grid, st, ma, mb, ea, eb, M, N, K, kps, bl, tiles, out, o_rs, o_cs, zs, kexp, err)));
-  else
-    TTG_TRY((launch<0, 0>(grid, st, ma, mb, ea, eb, M, N, K, kps, bl, tiles, out, o_rs, o_cs, zs, kexp, err)));
-  if (out != C) {
-    const int64_t mn = (int64_t)M * N;
-    k_oz_reduce<<<(unsigned)std::min<int64_t>((mn + 255) / 256, 4096), 256, 0, st>>>(
-        out, nsplit, M, N, sym ? 1 : 0, C, c_rs, c_cs); TTG_COUNT();
+  for (int64_t q0 = 0; q0 < chunks; q0 += kslab) {
+    const int64_t nq = std::min(kslab, chunks - q0);
+    if (!same && !pair) TTG_TRY(slice(st, SB, 1, 0, npad, q0 * OZ_K, nq, kexp, 1));
+    for (int64_t r0 = 0; r0 < M; r0 += mslab) {
+      const int64_t rows = std::min(mslab, M - r0), rpad = rup(rows, kRowPad);
+      TTG_TRY(slice(st, SA, pair ? 2 : 1, r0, rpad, q0 * OZ_K, nq, kexp, -1));
+      OzTiles tl = tiles;
+      tl.tiles_m = (int)((rows + OZ_M - 1) / OZ_M);
+      const int64_t nt = sym ? ntiles : (int64_t)tl.tiles_m * tiles_n;
+      CUtensorMap mb;
+      TTG_TRY(plane_map(&mb, pb, npad / 128 * nq));
+      OzMma g{pa, ea + r0, eb, (int)rows, (int)N, (int)nq,
+              (int)(sgroups * kGroupChunks), r0, b_lower ? (int)(q0 * OZ_K) : -1};
+      OzOut o = out;
+      o.accumulate = q0 > 0 ? 1 : 0;
+      k_oz_mma<<<dim3((unsigned)nt, (unsigned)nsplit), kThreads, kSmem, st>>>(mb, g, tl, o, err); TTG_COUNT();
+      cudaError_t e = cudaGetLastError();
+      if (e == cudaSuccess && sync_launches()) e = cudaStreamSynchronize(st);
+      if (e != cudaSuccess) {
+        fprintf(stderr, "ttg: k_oz_mma (M %lld, N %lld, K %lld) failed: %s\n", (long long)M,
+                (long long)N, (long long)K, cudaGetErrorString(e));
+        return TTG_CUDA_ERR;
+      }
+    }
+  }
+  if (partial) {
+    const int64_t mn = M * N;
+    k_oz_reduce<<<(unsigned)std::min<int64_t>((mn + 31) / 32, 152 * 16), dim3(32, 8), 0, st>>>(
+        out.p, (int)nsplit, (int)M, (int)N, sym ? 1 : 0, C, c.rs, c.cs); TTG_COUNT();
     TTG_CUDA_TRY(cudaGetLastError());
   }
   return TTG_OK;

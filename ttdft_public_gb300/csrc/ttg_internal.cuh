@@ -228,6 +228,7 @@ struct ttg_op {
   ttg::DevBuf oz_exp;         // FP64 tensor-core GEMM: row scales of its operands
   ttg::DevBuf oz_kexp;        // FP64 tensor-core GEMM: K scales (padded to whole chunks)
   ttg::DevBuf oz_err;         // FP64 tensor-core GEMM: error word
+  ttg::DevBuf oz_planes;      // FP64 tensor-core GEMM: digit planes of its operands
   ttg::DevBuf eigbuf;         // eigensolver refinement (5 k*k doubles)
   ttg::DevBuf eigf;           // FP32 tridiagonalisation scratch
   ttg::DevBuf partial;        // split-K partials for the Gram
@@ -341,26 +342,33 @@ ttg_status dgemm(cudaStream_t st, int M, int N, int K, int batch, DOp A, DOp B, 
                  int64_t c_rs, int64_t c_cs, int64_t c_bs, DevBuf& scratch, bool sym = false);
 
 // ozgemm.cu: FP64-accurate C = A B^T on the tensor cores (see the file).
-// A FP64 operand: `rows` rows of `kext` values, K-major (element (r, k) at
-// p[r ld + k]) or MN-major (p[k ld + r]); ld * 8 a multiple of 16.
+// An FP64 operand: `rows` rows of `kext` values; element (r, k) at
+//   p[(r % rin) rs + (r / rin) rs2 + (k % kin) ks + (k / kin) ks2].
 struct OzOperand {
   const double* p;
-  int64_t rows, kext, ld;
-  bool mn_major;
+  int64_t rows, kext;
+  int64_t rs, ks;
+  int64_t rin = INT64_MAX, rs2 = 0;   // rows in two levels
+  int64_t kin = INT64_MAX, ks2 = 0;   // K in two levels
 };
-// Whether ozgemm takes these operands (TMA alignment, sizes; off with
-// TTG_DISABLE_OZGEMM); callers fall back to the double-FP32 CUDA-core GEMMs.
+// Where C(m, n) goes: (m % rin) rs + (m / rin) rs2 + n cs.
+struct OzLayout {
+  int64_t rs, cs;
+  int64_t rin = INT64_MAX, rs2 = 0;
+};
+// Whether ozgemm takes these operands (sizes; off with TTG_DISABLE_OZGEMM);
+// callers fall back to the double-FP32 CUDA-core GEMMs.
 bool ozgemm_supported(const OzOperand& A, const OzOperand& B);
-// C[m c_rs + n c_cs] = sum_k A(m, k) B(n, k).  sym: A B^T is symmetric (A = B,
-// or B = H A): only tiles on and below the diagonal are computed and the
-// others mirrored.  b_lower: B(n, k) = 0 for k > n (the sum stops at n).
-// kscale_of: an MN-major operand whose rows are the K index (K of them);
-// with power-of-two scales f_k = its row scales, A is sliced as
-// A(m, k) 2^-f_k and B as B(n, k) 2^f_k, which leaves A B^T unchanged and
-// keeps small K columns of A (that B amplifies) at full precision.
-ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C, int64_t c_rs,
-                  int64_t c_cs, bool sym, bool b_lower = false,
-                  const OzOperand* kscale_of = nullptr);
+// C(m, n) = sum_k A(m, k) B(n, k).  sym: A B^T is symmetric (A = B, or
+// B = H A): only tiles on and below the diagonal are computed and the others
+// mirrored.  b_lower: B(n, k) = 0 for k > n (the sum stops at n).
+// kscale_of: an operand whose rows are the K index (K of them); with
+// power-of-two scales f_k = its row scales, A is sliced as A(m, k) 2^-f_k and
+// B as B(n, k) 2^f_k, which leaves A B^T unchanged and keeps small K columns
+// of A (that B amplifies) at full precision.  TTG_OOM: no room for the digit
+// planes (at most kPlaneBudget, 1 GiB, for sizes beyond it).
+ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C, OzLayout c,
+                  bool sym, bool b_lower = false, const OzOperand* kscale_of = nullptr);
 // Reads and clears the tensor-core GEMM's error word (synchronises).
 ttg_status ozgemm_error(ttg_op* op);
 
