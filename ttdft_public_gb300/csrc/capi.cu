@@ -312,6 +312,7 @@ ttg_status ttg_op_sync(ttg_op* op) {
   if (!op) return TTG_BAD_ARG;
   TTG_CUDA_TRY(cudaStreamSynchronize(op->stream));
   TTG_TRY(umma_check_error(op));
+  TTG_TRY(ozgemm_error(op));
   return hartree_error(op);
 }
 

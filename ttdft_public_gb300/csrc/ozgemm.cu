@@ -35,7 +35,8 @@
 // Operands larger than the workspace (kPlaneBudget) are taken in slabs of K
 // (Gram matrices: the sums are added in C's partial) or of A's rows.
 //
-// k_oz_mma: one CTA per 128 x 64 output tile and K range (split K), 20 warps.
+// k_oz_mma: persistent CTAs over items of a 128 x 64 output tile and a range of
+// K (split K), 20 warps.
 //  - The six digit planes of 32 rows of B lie one after the other, and so do
 //    the six level accumulators, so digit i of A times digits 0 .. 5-i of B is
 //    ONE MMA of N = 32 (6 - i) columns, starting at level i: six MMAs a chunk
@@ -96,6 +97,7 @@ constexpr int kThreads = (kEpiWarp0 + 2 * kEpiWarps) * 32;   // 640
 constexpr int kHalfCols = kLevels * OZ_H;               // 192
 constexpr uint32_t kTmemCols = 512;                     // two halves (384)
 constexpr int64_t kPlaneBudget = (int64_t)1 << 30;      // workspace of the digit planes
+constexpr int kSMs = 152;                               // one persistent CTA each
 constexpr int64_t kRowPad = OZ_M;                       // planes hold whole A tiles of rows
 
 // kind::f16: BF16 x BF16 -> FP32, A and B K-major, M = 128, N = n
@@ -189,57 +191,69 @@ struct OzSlices {
   unsigned char* planes[2];
 };
 
-// Digit planes of 16 gridDim.x values of K from k0 on and of 128 gridDim.y rows
+// Digit planes of `chunks` x 16 values of K from k0 on and of 128 gridDim.y rows
 // from r0 on: per 128 rows and chunk one 24 KB block, per digit 4 KB of 8-row x
-// 16-byte core matrices.  A thread cuts eight values of one row; rows beyond
-// the operand and values beyond kext are zero.  K scales (kexp, ksign):
-// v 2^(ksign kexp[k]).
+// 16-byte core matrices.  A block cuts kSliceChunks chunks of 128 rows, a thread
+// eight values of one row at a time; rows beyond the operand and values beyond
+// kext are zero.  K scales (kexp, ksign): v 2^(ksign kexp[k]).
+// diag: collects sum_k d3^2 of each row, see k_oz_reduce.
+constexpr int kSliceChunks = 4;
+
 template <bool ROWS_FAST>
 __global__ void __launch_bounds__(256) k_oz_slice(const OzSlices S, int64_t r0, int64_t k0,
-                                                  const int* __restrict__ kexp, int ksign) {
+                                                  int chunks, const int* __restrict__ kexp,
+                                                  int ksign, unsigned long long* diag) {
   const OzOperand& o = S.o[blockIdx.z];
   const int rt = ROWS_FAST ? threadIdx.x & 127 : threadIdx.x >> 1;
   const int half = ROWS_FAST ? threadIdx.x >> 7 : threadIdx.x & 1;
   const int64_t r = r0 + (int64_t)blockIdx.y * 128 + rt;
-  const int64_t k = k0 + (int64_t)blockIdx.x * OZ_K + half * 8;
-  double v[8];
+  const bool row_ok = r < o.rows;
+  const int e = row_ok ? exp_of_bits(__ldg(S.ebits[blockIdx.z] + r)) : 0;
+  const double* p = o.p + (row_ok ? row_at(o, r) : 0);
+  const int cb = blockIdx.x * kSliceChunks, ce = min(chunks, cb + kSliceChunks);
+  unsigned int d3sum = 0;                               // at most 4 x 8 x 2^14
+  for (int ch = cb; ch < ce; ++ch) {
+    const int64_t k = k0 + (int64_t)ch * OZ_K + half * 8;
+    double v[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) v[j] = 0.0;
-  int e = 0;
-  if (r < o.rows) {
-    e = exp_of_bits(__ldg(S.ebits[blockIdx.z] + r));
-    const double* p = o.p + row_at(o, r);
-    int64_t ki = k, kb = 0;
-    if (o.kin < o.kext) {
-      kb = k / o.kin;
-      ki = k - kb * o.kin;
-    }
+    for (int j = 0; j < 8; ++j) v[j] = 0.0;
+    if (row_ok) {
+      int64_t ki = k, kb = 0;
+      if (o.kin < o.kext) {
+        kb = k / o.kin;
+        ki = k - kb * o.kin;
+      }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (k + j < o.kext) v[j] = __ldg(p + ki * o.ks + kb * o.ks2);
-      if (++ki == o.kin) {
-        ki = 0;
-        ++kb;
+      for (int j = 0; j < 8; ++j) {
+        if (k + j < o.kext) v[j] = __ldg(p + ki * o.ks + kb * o.ks2);
+        if (++ki == o.kin) {
+          ki = 0;
+          ++kb;
+        }
       }
     }
+    uint32_t w[kDigits][4];
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      const int a0 = kexp ? ksign * __ldg(kexp + k + j) : 0;
+      const int a1 = kexp ? ksign * __ldg(kexp + k + j + 1) : 0;
+      float d0[kDigits], d1[kDigits];
+      digits6(v[j], e, a0, d0);
+      digits6(v[j + 1], e, a1, d1);
+      if (diag) d3sum += (unsigned int)(d0[3] * d0[3] + d1[3] * d1[3]);
+#pragma unroll
+      for (int d = 0; d < kDigits; ++d) w[d][j / 2] = pack_bf16(d0[d], d1[d]);
+    }
+    unsigned char* out = S.planes[blockIdx.z] + ((int64_t)blockIdx.y * chunks + ch) * kStageA +
+                         (rt >> 3) * 256 + half * 128 + (rt & 7) * 16;
+#pragma unroll
+    for (int d = 0; d < kDigits; ++d)
+      *reinterpret_cast<uint4*>(out + d * kPlA) = make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
   }
-  uint32_t w[kDigits][4];
-#pragma unroll
-  for (int j = 0; j < 8; j += 2) {
-    const int a0 = kexp ? ksign * __ldg(kexp + k + j) : 0;
-    const int a1 = kexp ? ksign * __ldg(kexp + k + j + 1) : 0;
-    float d0[kDigits], d1[kDigits];
-    digits6(v[j], e, a0, d0);
-    digits6(v[j + 1], e, a1, d1);
-#pragma unroll
-    for (int d = 0; d < kDigits; ++d) w[d][j / 2] = pack_bf16(d0[d], d1[d]);
+  if (diag) {
+    if (!ROWS_FAST) d3sum += __shfl_down_sync(0xffffffffu, d3sum, 1);
+    if (row_ok && (ROWS_FAST || half == 0) && d3sum) atomicAdd(diag + r, (unsigned long long)d3sum);
   }
-  unsigned char* out = S.planes[blockIdx.z] +
-                       ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * kStageA + (rt >> 3) * 256 +
-                       half * 128 + (rt & 7) * 16;
-#pragma unroll
-  for (int d = 0; d < kDigits; ++d)
-    *reinterpret_cast<uint4*>(out + d * kPlA) = make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
 }
 
 // With K scales (kexp, ksign): the biased exponent of v 2^(ksign kexp[k]).
@@ -321,8 +335,10 @@ struct OzTiles {
   int sym;          // only tiles with n0 <= m0 + 127 (on and below the diagonal)
   __device__ void at(int t, int& mt, int& nt) const {
     if (!sym) {
+      // rotated: a persistent CTA's items (a fixed step apart) then run through
+      // all columns, whose K ranges differ for a triangular B
       mt = t / tiles_n;
-      nt = t - mt * tiles_n;
+      nt = (t + mt) % tiles_n;
       return;
     }
     int m = 0;
@@ -350,8 +366,29 @@ struct OzMma {
   int b_lower_k0;                // >= 0: B(n, k) = 0 for k > n, planes start at this k
 };
 
+// What one CTA does of a work item: a tile and a range of K.
+struct OzItem {
+  int mt, m0, n0, c0, nq, nh, split;     // nq chunks from c0 on, nh halves with columns
+  __device__ OzItem(const OzMma& g, const OzTiles& tiles, int w, int ntiles) {
+    split = w / ntiles;
+    int nt;
+    tiles.at(w - split * ntiles, mt, nt);
+    m0 = mt * OZ_M;
+    n0 = nt * OZ_N;
+    c0 = split * g.split_chunks;
+    int c1 = min(g.chunks, c0 + g.split_chunks);
+    if (g.b_lower_k0 >= 0) c1 = min(c1, max(0, n0 + OZ_N - g.b_lower_k0 + OZ_K - 1) / OZ_K);
+    nq = max(0, c1 - c0);
+    nh = n0 + OZ_H < g.N ? 2 : 1;
+  }
+};
+
+// Persistent: CTA b takes items b, b + gridDim.x, ...; the copies and MMAs of
+// an item run under the fold and the stores of the one before.  Counters
+// (chunks, groups) run on over the items, and so do the barriers' phases.
 __global__ void __launch_bounds__(kThreads, 1) k_oz_mma(const __grid_constant__ CUtensorMap tmB,
                                                         const OzMma g, const OzTiles tiles,
+                                                        const int ntiles, const int items,
                                                         const OzOut out, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024 - (su32(smem_raw) & 1023)) & 1023);
@@ -361,17 +398,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_mma(const __grid_constant__ 
   __shared__ uint32_t tmem_slot;
   __shared__ uint32_t landed;                                 // chunks whose copies are there
   __shared__ int abort_flag;
-  __shared__ int eA[OZ_M], eB[OZ_N];                          // row scales 2^e
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  int mt, nt;
-  tiles.at(blockIdx.x, mt, nt);
-  const int m0 = mt * OZ_M, n0 = nt * OZ_N;
-  const int c0 = blockIdx.y * g.split_chunks;
-  int c1 = min(g.chunks, c0 + g.split_chunks);
-  if (g.b_lower_k0 >= 0) c1 = min(c1, max(0, n0 + OZ_N - g.b_lower_k0 + OZ_K - 1) / OZ_K);
-  const int nq = max(0, c1 - c0);                             // chunks
-  const int ng = (nq + kGroupChunks - 1) / kGroupChunks;      // groups
-  const int nh = n0 + OZ_H < g.N ? 2 : 1;                     // halves with columns
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -381,7 +408,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_mma(const __grid_constant__ 
   if (tid == 32) {
     for (int s = 0; s < kStages; ++s) {
       bar_init(&full[s], 1);
-      bar_init(&empty[s], nh);
+      bar_init(&empty[s], 2);
     }
     for (int b = 0; b < 2; ++b) {
       bar_init(&acc_full[b], 1);
@@ -391,10 +418,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_mma(const __grid_constant__ 
     landed = 0;
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  for (int i = tid; i < OZ_M + OZ_N; i += kThreads) {
-    if (i < OZ_M) eA[i] = m0 + i < g.M ? exp_of_bits(__ldg(g.ea + m0 + i)) : 0;
-    else eB[i - OZ_M] = n0 + i - OZ_M < g.N ? exp_of_bits(__ldg(g.eb + n0 + i - OZ_M)) : 0;
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -408,156 +431,180 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_mma(const __grid_constant__ 
     // been multiplied by both halves: A's six planes are one piece, the six
     // 1 KB pieces of a half of B one tensor copy
     if (lane == 0) {
-      const unsigned char* src = g.pa + ((int64_t)mt * g.chunks + c0) * kStageA;
-      const int bz = (n0 >> 7) * g.chunks + c0, bx = (n0 & 127) * 4;
-      int q = 0;
-      for (; q < nq; ++q) {
-        const int s = q % kStages;
-        if (q >= kStages) {
-          const uint32_t par = (uint32_t)((q / kStages - 1) & 1);
-          if (!bar_wait(&empty[s], par, abrt, 0)) {
-            ok = false;
-            break;
+      uint32_t q = 0;
+      for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+        const OzItem it(g, tiles, w, ntiles);
+        const unsigned char* src = g.pa + ((int64_t)it.mt * g.chunks + it.c0) * kStageA;
+        const int bz = (it.n0 >> 7) * g.chunks + it.c0, bx = (it.n0 & 127) * 4;
+        for (int c = 0; c < it.nq; ++c, ++q) {
+          const int s = q % kStages;
+          if (q >= kStages) {
+            const uint32_t par = (q / kStages - 1) & 1;
+            if (!bar_wait(&empty[s], par, abrt, 0)) {
+              ok = false;
+              break;
+            }
+            // the stage's previous copies must have landed before it is armed again
+            if (!bar_test(&full[s], par)) {
+              atomicExch(err, 3);
+              ok = false;
+              *abrt = 1;
+              break;
+            }
           }
-          // the stage's previous copies must have landed before it is armed again
-          if (!bar_test(&full[s], par)) {
-            atomicExch(err, 3);
-            ok = false;
-            *abrt = 1;
-            break;
-          }
+          const uint32_t fb = su32(&full[s]), dst = su32(smem) + s * kStage;
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                       ::"r"(fb), "r"(kStageA + it.nh * kStageH) : "memory");
+          asm volatile(
+              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+              ::"r"(dst), "l"(src + (int64_t)c * kStageA), "r"(kStageA), "r"(fb) : "memory");
+          for (int h = 0; h < it.nh; ++h)
+            tma_load(dst + kStageA + h * kStageH, &tmB, bx + h * OZ_H * 4, 0, bz + c, true, fb);
         }
-        const uint32_t fb = su32(&full[s]), dst = su32(smem) + s * kStage;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                     ::"r"(fb), "r"(kStageA + nh * kStageH) : "memory");
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-            ::"r"(dst), "l"(src + (int64_t)q * kStageA), "r"(kStageA), "r"(fb) : "memory");
-        for (int h = 0; h < nh; ++h)
-          tma_load(dst + kStageA + h * kStageH, &tmB, bx + h * OZ_H * 4, 0, bz + q, true, fb);
       }
       if (!ok)
-        for (int r = (q > kStages ? q - kStages : 0); r < q; ++r)
-          bar_drain(&full[r % kStages], (uint32_t)((r / kStages) & 1));
+        for (uint32_t r = (q > kStages ? q - kStages : 0); r < q; ++r)
+          bar_drain(&full[r % kStages], (r / kStages) & 1);
     }
   } else if (warp == 2) {
     // ---- chunks landed, in order
     if (lane == 0) {
-      for (int q = 0; q < nq; ++q) {
-        if (!bar_wait(&full[q % kStages], (uint32_t)((q / kStages) & 1), abrt, 0)) {
-          ok = false;
-          break;
+      uint32_t q = 0;
+      for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+        const OzItem it(g, tiles, w, ntiles);
+        for (int c = 0; c < it.nq; ++c, ++q) {
+          if (!bar_wait(&full[q % kStages], (q / kStages) & 1, abrt, 0)) {
+            ok = false;
+            break;
+          }
+          asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(su32(&landed)),
+                       "r"(q + 1) : "memory");
         }
-        asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(su32(&landed)),
-                     "r"((uint32_t)(q + 1)) : "memory");
       }
     }
   } else if (warp == 1 || warp == 3) {
     // ---- MMAs of one half: digit i of A times digits 0 .. 5 - i of B in one
     const int h = warp >> 1;
-    if (lane == 0 && h < nh) {
+    if (lane == 0) {
       const uint32_t base0 = su32(smem), dcol = tmem + (uint32_t)(h * kHalfCols);
-      uint32_t avail = 0;
-      for (int q = 0; q < nq; ++q) {
-        const int gr = q / kGroupChunks, c = q % kGroupChunks, s = q % kStages;
-        // the group's accumulators emptied (its own MMAs are long done by then)
-        if (c == 0 && gr > 0 && !bar_wait(&acc_empty[h], (uint32_t)((gr - 1) & 1), abrt, 0)) {
-          ok = false;
-          break;
-        }
-        for (int i = 0; i < kTcMaxWait && avail <= (uint32_t)q; ++i) {
-          asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(avail)
-                       : "r"(su32(&landed)) : "memory");
-          if (avail > (uint32_t)q || *abrt) break;
-        }
-        if (avail <= (uint32_t)q) { ok = false; *abrt = 1; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t base = base0 + (uint32_t)(s * kStage);
-        const uint64_t db = kmajor_desc(base + kStageA + h * kStageH);
+      uint32_t avail = 0, q = 0, gr = 0;                  // chunks, groups of this half
+      for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+        const OzItem it(g, tiles, w, ntiles);
+        const bool on = h < it.nh;
+        for (int j = 0; j < it.nq; ++j, ++q) {
+          const int c = j % kGroupChunks, s = q % kStages;
+          // the group's accumulators emptied (its own MMAs are long done by then)
+          if (on && c == 0 && gr > 0 && !bar_wait(&acc_empty[h], (gr - 1) & 1, abrt, 0)) {
+            ok = false;
+            break;
+          }
+          for (int i = 0; i < kTcMaxWait && avail <= q; ++i) {
+            asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(avail)
+                         : "r"(su32(&landed)) : "memory");
+            if (avail > q || *abrt) break;
+          }
+          if (avail <= q) { ok = false; *abrt = 1; break; }
+          if (!on) {                        // no columns in this half: it only frees the stage
+            bar_arrive(&empty[s]);
+            continue;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t base = base0 + (uint32_t)(s * kStage);
+          const uint64_t db = kmajor_desc(base + kStageA + h * kStageH);
 #pragma unroll
-        for (int i = 0; i < kDigits; ++i) {
-          const uint64_t da = kmajor_desc(base + i * kPlA);
-          const uint32_t acc = (c > 0 || i > 0) ? 1u : 0u;
-          asm volatile(
-              "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-              ::"r"(dcol + (uint32_t)(i * OZ_H)), "l"(da), "l"(db),
-                "r"(idesc_oz(OZ_H * (kDigits - i))), "r"(acc));
-        }
-        asm volatile(
-            "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-            ::"r"(su32(&empty[s])) : "memory");
-        if (c == kGroupChunks - 1 || q == nq - 1)
+          for (int i = 0; i < kDigits; ++i) {
+            const uint64_t da = kmajor_desc(base + i * kPlA);
+            const uint32_t acc = (c > 0 || i > 0) ? 1u : 0u;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                ::"r"(dcol + (uint32_t)(i * OZ_H)), "l"(da), "l"(db),
+                  "r"(idesc_oz(OZ_H * (kDigits - i))), "r"(acc));
+          }
           asm volatile(
               "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-              ::"r"(su32(&acc_full[h])) : "memory");
+              ::"r"(su32(&empty[s])) : "memory");
+          if (c == kGroupChunks - 1 || j == it.nq - 1) {
+            asm volatile(
+                "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                ::"r"(su32(&acc_full[h])) : "memory");
+            ++gr;
+          }
+        }
       }
       asm volatile(
           "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
           ::"r"(su32(&fin[h])) : "memory");
       bar_drain(&fin[h], 0);
     }
-  } else if (warp >= kEpiWarp0 && (warp - kEpiWarp0) / kEpiWarps < nh) {
+  } else if (warp >= kEpiWarp0) {
     // ---- fold of half a tile: TMEM lanes 32 (warp & 3) .., 16 columns a warp
     // (two warps per lane quarter: each waits on its tensor-memory loads)
     const int h = (warp - kEpiWarp0) / kEpiWarps, qd = warp & 3;
     const int cb = (((warp - kEpiWarp0) >> 2) & 1) * OZ_E;
     const int row = qd * 32 + lane;
     const uint32_t acol = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(h * kHalfCols + cb);
-    float hi[OZ_E], lo[OZ_E];
+    uint32_t gr = 0;
+    for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+      const OzItem it(g, tiles, w, ntiles);
+      if (h >= it.nh) continue;
+      const int ng = (it.nq + kGroupChunks - 1) / kGroupChunks;
+      float hi[OZ_E], lo[OZ_E];
 #pragma unroll
-    for (int c = 0; c < OZ_E; ++c) { hi[c] = 0.f; lo[c] = 0.f; }
-    for (int gr = 0; gr < ng; ++gr) {
-      // one lane polls: 512 threads on two barriers would slow every wait
-      bool w = true;
-      if (lane == 0) w = bar_wait(&acc_full[h], (uint32_t)(gr & 1), abrt, 32);
-      ok = __shfl_sync(0xffffffffu, w, 0);
-      if (!ok) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      for (int c = 0; c < OZ_E; ++c) { hi[c] = 0.f; lo[c] = 0.f; }
+      for (int t = 0; t < ng; ++t, ++gr) {
+        // one lane polls: 512 threads on two barriers would slow every wait
+        bool wt = true;
+        if (lane == 0) wt = bar_wait(&acc_full[h], gr & 1, abrt, 32);
+        ok = __shfl_sync(0xffffffffu, wt, 0);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-      for (int cc = 0; cc < OZ_E; cc += 8) {
-        float S[kLevels][8];
-        tmem_ld8x3(acol + cc, acol + OZ_H + cc, acol + 2 * OZ_H + cc, S[0], S[1], S[2]);
-        tmem_ld8x3(acol + 3 * OZ_H + cc, acol + 4 * OZ_H + cc, acol + 5 * OZ_H + cc, S[3], S[4],
-                   S[5]);
-        if (cc + 8 == OZ_E) {              // the last loads are in registers: release the buffer
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) bar_arrive(&acc_empty[h]);
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          // S0 + S1 2^-8 + ... + S5 2^-40 as (f, l), then into (hi, lo)
-          float f = S[0][i], l = 0.f;
-          float sc = 1.f / 256.f;
-#pragma unroll
-          for (int L = 1; L < kLevels; ++L, sc *= (1.f / 256.f)) {
-            const float t = S[L][i] * sc;
-            const float h2 = f + t;
-            const float bv = h2 - f;
-            l += (f - (h2 - bv)) + (t - bv);
-            f = h2;
+        for (int cc = 0; cc < OZ_E; cc += 8) {
+          float S[kLevels][8];
+          tmem_ld8x3(acol + cc, acol + OZ_H + cc, acol + 2 * OZ_H + cc, S[0], S[1], S[2]);
+          tmem_ld8x3(acol + 3 * OZ_H + cc, acol + 4 * OZ_H + cc, acol + 5 * OZ_H + cc, S[3], S[4],
+                     S[5]);
+          if (cc + 8 == OZ_E) {              // the last loads are in registers: release the buffer
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) bar_arrive(&acc_empty[h]);
           }
-          const float sum = hi[cc + i] + f;
-          const float bv = sum - hi[cc + i];
-          lo[cc + i] += (hi[cc + i] - (sum - bv)) + (f - bv) + l;
-          hi[cc + i] = sum;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            // S0 + S1 2^-8 + ... + S5 2^-40 as (f, l), then into (hi, lo)
+            float f = S[0][i], l = 0.f;
+            float sc = 1.f / 256.f;
+#pragma unroll
+            for (int L = 1; L < kLevels; ++L, sc *= (1.f / 256.f)) {
+              const float u = S[L][i] * sc;
+              const float h2 = f + u;
+              const float bv = h2 - f;
+              l += (f - (h2 - bv)) + (u - bv);
+              f = h2;
+            }
+            const float sum = hi[cc + i] + f;
+            const float bv = sum - hi[cc + i];
+            lo[cc + i] += (hi[cc + i] - (sum - bv)) + (f - bv) + l;
+            hi[cc + i] = sum;
+          }
         }
       }
-    }
-    if (ok && m0 + row < g.M) {
-      const int em = eA[row] - 16;
-      const int64_t m = g.row0 + m0 + row;
-      const int nb = n0 + h * OZ_H + cb;
-      double* o = out.p + blockIdx.y * out.zs + nb * out.cs +
+      if (!ok || it.m0 + row >= g.M) continue;
+      const int em = exp_of_bits(__ldg(g.ea + it.m0 + row)) - 16;
+      const int64_t m = g.row0 + it.m0 + row;
+      const int nb = it.n0 + h * OZ_H + cb;
+      double* o = out.p + it.split * out.zs + nb * out.cs +
                   (m < out.rin ? m * out.rs : (m % out.rin) * out.rs + (m / out.rin) * out.rs2);
       const bool pairs = out.cs == 1 && !out.accumulate && (reinterpret_cast<uintptr_t>(o) & 15) == 0;
 #pragma unroll
       for (int c = 0; c < OZ_E; c += 2) {
         double v[2];
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
-          v[u] = scaled_sum(hi[c + u], lo[c + u], em + eB[h * OZ_H + cb + c + u]);
+        for (int u = 0; u < 2; ++u) {
+          const int n = min(nb + c + u, g.N - 1);
+          v[u] = scaled_sum(hi[c + u], lo[c + u], em + exp_of_bits(__ldg(g.eb + n)));
+        }
         if (pairs && nb + c + 1 < g.N) {
           *reinterpret_cast<double2*>(o + c) = make_double2(v[0], v[1]);
         } else {
@@ -584,9 +631,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_mma(const __grid_constant__ 
 // S = sum of the split partials (column-major M x N); sym: tiles above the
 // diagonal were not computed, S[m, n] is read from [n, m] there.  Eight
 // threads share an element's splits (fixed order), 32 elements a block.
+// diag (X^T X): the products left out, of digits i + j >= 6, sum to about zero
+// except the squares on the diagonal; sum_k d3^2 of each row, exact, is added
+// there (weight 2^-48 of the row's scale squared).  Without it the diagonal of
+// a peaked field's Gram matrix is low by 1e-13, which turns the trailing
+// eigenvectors of an STHOSVD more than double-FP32 sums did.
 __global__ void __launch_bounds__(256) k_oz_reduce(const double* __restrict__ part, int nsplit,
-                                                   int M, int N, int sym, double* __restrict__ C,
-                                                   int64_t c_rs, int64_t c_cs) {
+                                                   int M, int N, int sym,
+                                                   const unsigned long long* __restrict__ diag,
+                                                   const int* __restrict__ ebits,
+                                                   double* __restrict__ C, int64_t c_rs,
+                                                   int64_t c_cs) {
   __shared__ double red[8][33];
   const int64_t mn = (int64_t)M * N;
   for (int64_t b = blockIdx.x; b * 32 < mn; b += gridDim.x) {
@@ -602,6 +657,7 @@ __global__ void __launch_bounds__(256) k_oz_reduce(const double* __restrict__ pa
     __syncthreads();
     if (threadIdx.y == 0 && i < mn) {
       for (int y = 1; y < 8; ++y) s += red[y][threadIdx.x];
+      if (diag && m == n) s += ldexp((double)diag[m], 2 * exp_of_bits(ebits[m]) - 16 - 48);
       C[m * c_rs + n * c_cs] = s;
     }
     __syncthreads();
@@ -668,13 +724,13 @@ ttg_status row_exps(cudaStream_t st, const OzSlices& S, int nz, const int* kexp,
 }
 
 ttg_status slice(cudaStream_t st, const OzSlices& S, int nz, int64_t r0, int64_t rpad, int64_t k0,
-                 int64_t chunks, const int* kexp, int ksign) {
+                 int64_t chunks, const int* kexp, int ksign, unsigned long long* diag = nullptr) {
   if (chunks <= 0) return TTG_OK;
-  const dim3 grid((unsigned)chunks, (unsigned)(rpad / 128), nz);
+  const dim3 grid((unsigned)((chunks + kSliceChunks - 1) / kSliceChunks), (unsigned)(rpad / 128), nz);
   if (rows_fast(S.o[0]))
-    k_oz_slice<true><<<grid, 256, 0, st>>>(S, r0, k0, kexp, ksign);
+    k_oz_slice<true><<<grid, 256, 0, st>>>(S, r0, k0, (int)chunks, kexp, ksign, diag);
   else
-    k_oz_slice<false><<<grid, 256, 0, st>>>(S, r0, k0, kexp, ksign);
+    k_oz_slice<false><<<grid, 256, 0, st>>>(S, r0, k0, (int)chunks, kexp, ksign, diag);
   TTG_COUNT();
   TTG_CUDA_TRY(cudaGetLastError());
   return TTG_OK;
@@ -724,6 +780,12 @@ ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C,
   unsigned char* pb = same ? pa : pa + need_a;
   if (op->oz_exp.bytes < (size_t)(M + N) * sizeof(int))
     TTG_TRY(op->oz_exp.alloc((size_t)(M + N) * sizeof(int)));
+  unsigned long long* diag = nullptr;            // X^T X: the diagonal's share of d3 d3
+  if (same && sym) {
+    if (op->oz_diag.bytes < (size_t)M * 8) TTG_TRY(op->oz_diag.alloc((size_t)M * 8));
+    diag = op->oz_diag.as<unsigned long long>();
+    TTG_CUDA_TRY(cudaMemsetAsync(diag, 0, (size_t)M * 8, st));
+  }
   if (!op->oz_err.p) {
     TTG_TRY(op->oz_err.alloc(sizeof(int)));
     TTG_CUDA_TRY(cudaMemsetAsync(op->oz_err.p, 0, sizeof(int), st));
@@ -771,15 +833,15 @@ ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C,
     ntiles = 0;
     for (int m = 0; m < tiles.tiles_m; ++m) ntiles += std::min(2 * m + 2, tiles_n);
   }
-  // Split K for the least time: waves of CTAs (one per SM) times their groups
-  // (about 1.2 us each, three more to start and to store), plus the partials
-  // written and summed.
+  // Split K for the least time: items per CTA (one per SM) times their groups
+  // (about 1.2 us each, two more to fill the ring and to store), plus the
+  // partials written and summed.
   const int64_t kgroups = (kslab + kGroupChunks - 1) / kGroupChunks;
   int64_t nsplit = 1;
   if (!b_lower && c.rin >= M) {
     double best = 1e300;
-    for (int64_t t = 1; t <= std::min<int64_t>(kgroups, 8 * 152 / ntiles + 1); ++t) {
-      const double cost = (double)((ntiles * t + 151) / 152) * ((kgroups + t - 1) / t + 3) +
+    for (int64_t t = 1; t <= std::min<int64_t>(kgroups, 8 * kSMs / ntiles + 1); ++t) {
+      const double cost = (double)((ntiles * t + kSMs - 1) / kSMs) * ((kgroups + t - 1) / t + 2) +
                           (t > 1 || sym ? t * (double)M * N * 16 / 7e6 : 0.0);
       if (cost < best) {
         best = cost;
@@ -803,7 +865,7 @@ ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C,
     if (!same && !pair) TTG_TRY(slice(st, SB, 1, 0, npad, q0 * OZ_K, nq, kexp, 1));
     for (int64_t r0 = 0; r0 < M; r0 += mslab) {
       const int64_t rows = std::min(mslab, M - r0), rpad = rup(rows, kRowPad);
-      TTG_TRY(slice(st, SA, pair ? 2 : 1, r0, rpad, q0 * OZ_K, nq, kexp, -1));
+      TTG_TRY(slice(st, SA, pair ? 2 : 1, r0, rpad, q0 * OZ_K, nq, kexp, -1, diag));
       OzTiles tl = tiles;
       tl.tiles_m = (int)((rows + OZ_M - 1) / OZ_M);
       const int64_t nt = sym ? ntiles : (int64_t)tl.tiles_m * tiles_n;
@@ -813,7 +875,10 @@ ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C,
               (int)(sgroups * kGroupChunks), r0, b_lower ? (int)(q0 * OZ_K) : -1};
       OzOut o = out;
       o.accumulate = q0 > 0 ? 1 : 0;
-      k_oz_mma<<<dim3((unsigned)nt, (unsigned)nsplit), kThreads, kSmem, st>>>(mb, g, tl, o, err); TTG_COUNT();
+      const int64_t items = nt * nsplit;
+      if (items > INT32_MAX) return TTG_BAD_ARG;
+      k_oz_mma<<<(unsigned)std::min<int64_t>(items, kSMs), kThreads, kSmem, st>>>(
+          mb, g, tl, (int)nt, (int)items, o, err); TTG_COUNT();
       cudaError_t e = cudaGetLastError();
       if (e == cudaSuccess && sync_launches()) e = cudaStreamSynchronize(st);
       if (e != cudaSuccess) {
@@ -826,7 +891,7 @@ ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C,
   if (partial) {
     const int64_t mn = M * N;
     k_oz_reduce<<<(unsigned)std::min<int64_t>((mn + 31) / 32, 152 * 16), dim3(32, 8), 0, st>>>(
-        out.p, (int)nsplit, (int)M, (int)N, sym ? 1 : 0, C, c.rs, c.cs); TTG_COUNT();
+        out.p, (int)nsplit, (int)M, (int)N, sym ? 1 : 0, diag, ea, C, c.rs, c.cs); TTG_COUNT();
     TTG_CUDA_TRY(cudaGetLastError());
   }
   return TTG_OK;

@@ -200,11 +200,36 @@ ttg_status dgemm(cudaStream_t st, int M, int N, int K, int batch, DOp A, DOp B, 
 
 namespace {
 
+// Below this many flops the CUDA-core GEMM's one or two launches win over the
+// tensor-core GEMM's seven.  Measured, all Gram matrices and mode products of
+// an n^3 grid cut to rank n/4, device time: n = 64: 387 against 441 us on the
+// CUDA cores, but sixteen launches (50 us) more; 96 (1.7e8 flops in the first
+// Gram): 449 against 579; 200: 910 against 2,824; 360: 2.1 against 17 ms.
+constexpr double kOzMinFlops = 1e8;
+
+bool use_oz(const OzOperand& A, const OzOperand& B) {
+  return 2.0 * (double)A.rows * (double)B.rows * (double)A.kext >= kOzMinFlops &&
+         ozgemm_supported(A, B);
+}
+
 // Mode-d product of an x-fastest tensor (n0, n1, n2) with Mmat (p x n_d,
 // row-major): mode d of the result has size p.
-ttg_status mode_product(cudaStream_t st, const double* T, const int* n, int d, const double* Mmat,
+ttg_status mode_product(ttg_op* op, const double* T, const int* n, int d, const double* Mmat,
                         int p, double* out, DevBuf& scratch) {
   const int64_t n0 = n[0], n1 = n[1], n2 = n[2];
+  cudaStream_t st = op->stream;
+  // the long dimension as the GEMM's rows: (y, z), (x, z) or (x, y)
+  const OzOperand A = d == 0   ? OzOperand{T, n1 * n2, n0, n0, 1}
+                      : d == 1 ? OzOperand{T, n0 * n2, n1, 1, n0, n0, n0 * n1}
+                               : OzOperand{T, n0 * n1, n2, 1, n0 * n1};
+  const OzOperand B{Mmat, p, n[d], n[d], 1};
+  if (use_oz(A, B)) {
+    const OzLayout c = d == 0   ? OzLayout{p, 1}
+                       : d == 1 ? OzLayout{1, n0, n0, n0 * p}
+                                : OzLayout{1, n0 * n1};
+    const ttg_status s = ozgemm(op, A, B, out, c, false);
+    if (s != TTG_OOM) return s;
+  }
   if (d == 0) {
     // out (p x n1 n2) = M (p x n0) T_(0) (n0 x n1 n2)
     return dgemm(st, p, (int)(n1 * n2), (int)n0, 1, DOp{Mmat, (int64_t)n0, 1, 0},
@@ -221,9 +246,21 @@ ttg_status mode_product(cudaStream_t st, const double* T, const int* n, int d, c
 }
 
 // Gram matrix of mode d, G (n_d x n_d) column-major.
-ttg_status mode_gram(cudaStream_t st, const double* T, const int* n, int d, double* G,
+ttg_status mode_gram(ttg_op* op, const double* T, const int* n, int d, double* G,
                      DevBuf& scratch, DevBuf& scratch2) {
   const int64_t n0 = n[0], n1 = n[1], n2 = n[2];
+  cudaStream_t st = op->stream;
+  OzOperand A = d == 0   ? OzOperand{T, n0, n1 * n2, 1, n0}
+                : d == 1 ? OzOperand{T, n1, n0 * n2, n0, 1}
+                         : OzOperand{T, n2, n0 * n1, n0 * n1, 1};
+  if (d == 1) {          // K = (x, z): slabs of n0 n1 values apart
+    A.kin = n0;
+    A.ks2 = n0 * n1;
+  }
+  if (use_oz(A, A)) {
+    const ttg_status s = ozgemm(op, A, A, G, OzLayout{1, n[d]}, true);
+    if (s != TTG_OOM) return s;
+  }
   if (d == 0)
     return dgemm(st, (int)n0, (int)n0, (int)(n1 * n2), 1, DOp{T, 1, n0, 0}, DOp{T, n0, 1, 0}, G,
                  1, n0, 0, scratch, true);
@@ -611,7 +648,7 @@ ttg_status ttg_tucker_sthosvd(ttg_op* op, const double* t_dev, const int32_t* di
     const int rcap = std::min(nd, (max_ranks && max_ranks[d] > 0) ? (int)max_ranks[d] : nd);
     const size_t kk = (size_t)nd * nd * 8;
     if (op->kk0.bytes < kk) TTG_TRY(op->kk0.alloc(kk));
-    TTG_TRY(mode_gram(st, A.as<double>(), cur, d, op->kk0.as<double>(), part, part2));
+    TTG_TRY(mode_gram(op, A.as<double>(), cur, d, op->kk0.as<double>(), part, part2));
     // trace of the Gram = sum of all eigenvalues
     k_diag_sum<<<1, 256, 0, st>>>(op->kk0.as<double>(), nd, norm.as<double>() + 2049); TTG_COUNT();
     TTG_LAUNCHED(op);
@@ -639,7 +676,7 @@ ttg_status ttg_tucker_sthosvd(ttg_op* op, const double* t_dev, const int32_t* di
     }
     ranks_out[d] = r;
     // project: A <- A x_d U_d^T
-    TTG_TRY(mode_product(st, A.as<double>(), cur, d, U[d], r, B.as<double>(), part));
+    TTG_TRY(mode_product(op, A.as<double>(), cur, d, U[d], r, B.as<double>(), part));
     std::swap(A.p, B.p);
     std::swap(A.bytes, B.bytes);
     cur[d] = r;
@@ -647,7 +684,7 @@ ttg_status ttg_tucker_sthosvd(ttg_op* op, const double* t_dev, const int32_t* di
   TTG_CUDA_TRY(cudaMemcpyAsync(core_dev, A.p, (size_t)cur[0] * cur[1] * cur[2] * 8,
                                cudaMemcpyDeviceToDevice, st));
   TTG_CUDA_TRY(cudaStreamSynchronize(st));
-  return TTG_OK;
+  return ozgemm_error(op);
 }
 
 ttg_status ttg_tucker_reconstruct(const double* core_dev, const int32_t* ranks,

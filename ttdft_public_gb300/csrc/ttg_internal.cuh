@@ -229,6 +229,7 @@ struct ttg_op {
   ttg::DevBuf oz_kexp;        // FP64 tensor-core GEMM: K scales (padded to whole chunks)
   ttg::DevBuf oz_err;         // FP64 tensor-core GEMM: error word
   ttg::DevBuf oz_planes;      // FP64 tensor-core GEMM: digit planes of its operands
+  ttg::DevBuf oz_diag;        // FP64 tensor-core GEMM: sums of d3^2 of the rows of X^T X
   ttg::DevBuf eigbuf;         // eigensolver refinement (5 k*k doubles)
   ttg::DevBuf eigf;           // FP32 tridiagonalisation scratch
   ttg::DevBuf partial;        // split-K partials for the Gram
