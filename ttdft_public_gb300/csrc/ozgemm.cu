@@ -181,6 +181,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 __device__ __forceinline__ int exp_of_bits(int b) { return b == 0 ? 0 : min(b, 2046) - 1022; }
 
 __device__ __forceinline__ int64_t row_at(const OzOperand& o, int64_t r) {
+  if (o.idx) r = __ldg(o.idx + r);
   return o.rin >= o.rows ? r * o.rs : (r % o.rin) * o.rs + (r / o.rin) * o.rs2;
 }
 
@@ -333,7 +334,19 @@ __device__ __forceinline__ double scaled_sum(float hi, float lo, int e) {
 struct OzTiles {
   int tiles_m, tiles_n;
   int sym;          // only tiles with n0 <= m0 + 127 (on and below the diagonal)
+  const int* first; // ragged: prefix sums of the column tiles (null: all tiles_n)
   __device__ void at(int t, int& mt, int& nt) const {
+    if (first) {
+      int lo = 0, hi = tiles_m;              // first[lo] <= t < first[hi]
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(first + mid) <= t) lo = mid;
+        else hi = mid;
+      }
+      mt = lo;
+      nt = t - __ldg(first + lo);
+      return;
+    }
     if (!sym) {
       // rotated: a persistent CTA's items (a fixed step apart) then run through
       // all columns, whose K ranges differ for a triangular B
@@ -356,6 +369,8 @@ struct OzOut {
   double* p;
   int64_t rin, rs, rs2, cs, zs;  // (m % rin) rs + (m / rin) rs2 + n cs + split zs
   int accumulate;                // add to p
+  const int64_t* base;           // ragged: base[mt] + row ld[mt] + n
+  const int* ld;
 };
 
 struct OzMma {
@@ -369,7 +384,8 @@ struct OzMma {
 // What one CTA does of a work item: a tile and a range of K.
 struct OzItem {
   int mt, m0, n0, c0, nq, nh, split;     // nq chunks from c0 on, nh halves with columns
-  __device__ OzItem(const OzMma& g, const OzTiles& tiles, int w, int ntiles) {
+  int N;                                 // columns of C here
+  __device__ OzItem(const OzMma& g, const OzTiles& tiles, const OzOut& out, int w, int ntiles) {
     split = w / ntiles;
     int nt;
     tiles.at(w - split * ntiles, mt, nt);
@@ -379,7 +395,8 @@ struct OzItem {
     int c1 = min(g.chunks, c0 + g.split_chunks);
     if (g.b_lower_k0 >= 0) c1 = min(c1, max(0, n0 + OZ_N - g.b_lower_k0 + OZ_K - 1) / OZ_K);
     nq = max(0, c1 - c0);
-    nh = n0 + OZ_H < g.N ? 2 : 1;
+    N = out.ld ? __ldg(out.ld + mt) : g.N;
+    nh = n0 + OZ_H < N ? 2 : 1;
   }
 };
 
@@ -433,7 +450,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_mma(const __grid_constant__ 
     if (lane == 0) {
       uint32_t q = 0;
       for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
-        const OzItem it(g, tiles, w, ntiles);
+        const OzItem it(g, tiles, out, w, ntiles);
         const unsigned char* src = g.pa + ((int64_t)it.mt * g.chunks + it.c0) * kStageA;
         const int bz = (it.n0 >> 7) * g.chunks + it.c0, bx = (it.n0 & 127) * 4;
         for (int c = 0; c < it.nq; ++c, ++q) {
@@ -471,7 +488,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_mma(const __grid_constant__ 
     if (lane == 0) {
       uint32_t q = 0;
       for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
-        const OzItem it(g, tiles, w, ntiles);
+        const OzItem it(g, tiles, out, w, ntiles);
         for (int c = 0; c < it.nq; ++c, ++q) {
           if (!bar_wait(&full[q % kStages], (q / kStages) & 1, abrt, 0)) {
             ok = false;
@@ -489,7 +506,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_mma(const __grid_constant__ 
       const uint32_t base0 = su32(smem), dcol = tmem + (uint32_t)(h * kHalfCols);
       uint32_t avail = 0, q = 0, gr = 0;                  // chunks, groups of this half
       for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
-        const OzItem it(g, tiles, w, ntiles);
+        const OzItem it(g, tiles, out, w, ntiles);
         const bool on = h < it.nh;
         for (int j = 0; j < it.nq; ++j, ++q) {
           const int c = j % kGroupChunks, s = q % kStages;
@@ -546,7 +563,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_mma(const __grid_constant__ 
     const uint32_t acol = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(h * kHalfCols + cb);
     uint32_t gr = 0;
     for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
-      const OzItem it(g, tiles, w, ntiles);
+      const OzItem it(g, tiles, out, w, ntiles);
       if (h >= it.nh) continue;
       const int ng = (it.nq + kGroupChunks - 1) / kGroupChunks;
       float hi[OZ_E], lo[OZ_E];
@@ -594,8 +611,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_mma(const __grid_constant__ 
       const int em = exp_of_bits(__ldg(g.ea + it.m0 + row)) - 16;
       const int64_t m = g.row0 + it.m0 + row;
       const int nb = it.n0 + h * OZ_H + cb;
-      double* o = out.p + it.split * out.zs + nb * out.cs +
-                  (m < out.rin ? m * out.rs : (m % out.rin) * out.rs + (m / out.rin) * out.rs2);
+      double* o = out.p;
+      if (out.ld)
+        o += __ldg(out.base + it.mt) + (int64_t)row * it.N + nb;
+      else
+        o += it.split * out.zs + nb * out.cs +
+             (m < out.rin ? m * out.rs : (m % out.rin) * out.rs + (m / out.rin) * out.rs2);
       const bool pairs = out.cs == 1 && !out.accumulate && (reinterpret_cast<uintptr_t>(o) & 15) == 0;
 #pragma unroll
       for (int c = 0; c < OZ_E; c += 2) {
@@ -605,12 +626,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_mma(const __grid_constant__ 
           const int n = min(nb + c + u, g.N - 1);
           v[u] = scaled_sum(hi[c + u], lo[c + u], em + exp_of_bits(__ldg(g.eb + n)));
         }
-        if (pairs && nb + c + 1 < g.N) {
+        if (pairs && nb + c + 1 < it.N) {
           *reinterpret_cast<double2*>(o + c) = make_double2(v[0], v[1]);
         } else {
 #pragma unroll
           for (int u = 0; u < 2; ++u)
-            if (nb + c + u < g.N) {
+            if (nb + c + u < it.N) {
               double* t = o + (c + u) * out.cs;
               *t = out.accumulate ? *t + v[u] : v[u];
             }
@@ -701,7 +722,7 @@ bool rows_fast(const OzOperand& o) { return o.rs == 1 && o.ks != 1; }
 
 bool same_operand(const OzOperand& a, const OzOperand& b) {
   return a.p == b.p && a.rows == b.rows && a.kext == b.kext && a.rin == b.rin && a.rs == b.rs &&
-         a.rs2 == b.rs2 && a.kin == b.kin && a.ks == b.ks && a.ks2 == b.ks2;
+         a.rs2 == b.rs2 && a.kin == b.kin && a.ks == b.ks && a.ks2 == b.ks2 && a.idx == b.idx;
 }
 
 ttg_status row_exps(cudaStream_t st, const OzSlices& S, int nz, const int* kexp, int ksign) {
@@ -738,23 +759,30 @@ ttg_status slice(cudaStream_t st, const OzSlices& S, int nz, int64_t r0, int64_t
 
 }  // namespace
 
+int64_t ozgemm_ragged_rows(int64_t K, int64_t N) {
+  const int64_t row = (K + OZ_K - 1) / OZ_K * kDigits * 32;        // bytes of a row's planes
+  return std::max<int64_t>(0, (kPlaneBudget - rup(N, kRowPad) * row) / row / kRowPad * kRowPad);
+}
+
 bool ozgemm_supported(const OzOperand& A, const OzOperand& B) {
   if (getenv("TTG_DISABLE_OZGEMM")) return false;
   return A.p && B.p && A.rows > 0 && B.rows > 0 && A.kext > 0 && A.kext == B.kext &&
          A.rows <= INT32_MAX - 256 && B.rows <= INT32_MAX - 256 && A.kext <= INT32_MAX - 256;
 }
 
-ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C, OzLayout c,
-                  bool sym, bool b_lower, const OzOperand* kscale_of) {
+ttg_status ozgemm(cudaStream_t st, OzWork& ws, DevBuf& partial_buf, const OzOperand& A,
+                  const OzOperand& B, double* C, OzLayout c, bool sym, bool b_lower,
+                  const OzOperand* kscale_of, const OzRagged* ragged) {
   if (!ozgemm_supported(A, B) || !C) return TTG_BAD_ARG;
   if (sym && (A.rows != B.rows || c.rin < A.rows)) return TTG_BAD_ARG;
+  if (ragged && (sym || b_lower || kscale_of || A.rows > ozgemm_ragged_rows(A.kext, B.rows)))
+    return TTG_BAD_ARG;
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
   std::call_once(once, [] {
     attr = cudaFuncSetAttribute(k_oz_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   });
   if (attr != cudaSuccess) return TTG_CUDA_ERR;
-  cudaStream_t st = op->stream;
   const int64_t M = A.rows, N = B.rows, K = A.kext;
   const int64_t mpad = rup(M, kRowPad), npad = rup(N, kRowPad), chunks = (K + OZ_K - 1) / OZ_K;
   const bool same = !kscale_of && same_operand(A, B);
@@ -775,24 +803,24 @@ ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C,
     kslab = std::min(kslab, chunks);
   }
   const int64_t need_a = mslab * kslab * per_chunk, need_b = same ? 0 : npad * kslab * per_chunk;
-  if (op->oz_planes.bytes < (size_t)(need_a + need_b)) TTG_TRY(op->oz_planes.alloc(need_a + need_b));
-  unsigned char* pa = op->oz_planes.as<unsigned char>();
+  if (ws.planes.bytes < (size_t)(need_a + need_b)) TTG_TRY(ws.planes.alloc(need_a + need_b));
+  unsigned char* pa = ws.planes.as<unsigned char>();
   unsigned char* pb = same ? pa : pa + need_a;
-  if (op->oz_exp.bytes < (size_t)(M + N) * sizeof(int))
-    TTG_TRY(op->oz_exp.alloc((size_t)(M + N) * sizeof(int)));
+  if (ws.exp.bytes < (size_t)(M + N) * sizeof(int))
+    TTG_TRY(ws.exp.alloc((size_t)(M + N) * sizeof(int)));
   unsigned long long* diag = nullptr;            // X^T X: the diagonal's share of d3 d3
   if (same && sym) {
-    if (op->oz_diag.bytes < (size_t)M * 8) TTG_TRY(op->oz_diag.alloc((size_t)M * 8));
-    diag = op->oz_diag.as<unsigned long long>();
+    if (ws.diag.bytes < (size_t)M * 8) TTG_TRY(ws.diag.alloc((size_t)M * 8));
+    diag = ws.diag.as<unsigned long long>();
     TTG_CUDA_TRY(cudaMemsetAsync(diag, 0, (size_t)M * 8, st));
   }
-  if (!op->oz_err.p) {
-    TTG_TRY(op->oz_err.alloc(sizeof(int)));
-    TTG_CUDA_TRY(cudaMemsetAsync(op->oz_err.p, 0, sizeof(int), st));
+  if (!ws.err.p) {
+    TTG_TRY(ws.err.alloc(sizeof(int)));
+    TTG_CUDA_TRY(cudaMemsetAsync(ws.err.p, 0, sizeof(int), st));
   }
-  int* ea = op->oz_exp.as<int>();
+  int* ea = ws.exp.as<int>();
   int* eb = same ? ea : ea + M;
-  int* err = op->oz_err.as<int>();
+  int* err = ws.err.as<int>();
   // K scales: the row scales of kscale_of (a view whose rows are the K
   // index), A scaled by 2^-f_k and B by 2^f_k; the buffer is padded with zeros
   // to whole chunks
@@ -800,15 +828,15 @@ ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C,
   if (kscale_of) {
     if (kscale_of->rows != K) return TTG_BAD_ARG;
     const size_t kb = (size_t)(chunks * OZ_K) * sizeof(int);
-    if (op->oz_kexp.bytes < kb) TTG_TRY(op->oz_kexp.alloc(kb));
-    TTG_CUDA_TRY(cudaMemsetAsync(op->oz_kexp.p, 0, kb, st));
+    if (ws.kexp.bytes < kb) TTG_TRY(ws.kexp.alloc(kb));
+    TTG_CUDA_TRY(cudaMemsetAsync(ws.kexp.p, 0, kb, st));
     OzSlices S{};
     S.o[0] = *kscale_of;
-    S.ebits[0] = op->oz_kexp.as<int>();
+    S.ebits[0] = ws.kexp.as<int>();
     TTG_TRY(row_exps(st, S, 1, nullptr, 0));
-    k_exp_from_bits<<<(unsigned)((K + 255) / 256), 256, 0, st>>>(op->oz_kexp.as<int>(), K); TTG_COUNT();
+    k_exp_from_bits<<<(unsigned)((K + 255) / 256), 256, 0, st>>>(ws.kexp.as<int>(), K); TTG_COUNT();
     TTG_CUDA_TRY(cudaGetLastError());
-    kexp = op->oz_kexp.as<int>();
+    kexp = ws.kexp.as<int>();
   }
   // both operands in one launch where they have one shape and orientation
   const bool pair = !same && !kexp && M == N && rows_fast(A) == rows_fast(B);
@@ -827,8 +855,9 @@ ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C,
   TTG_TRY(row_exps(st, SA, pair ? 2 : 1, kexp, -1));
   if (!same && !pair) TTG_TRY(row_exps(st, SB, 1, kexp, 1));
   const int tiles_n = (int)((N + OZ_N - 1) / OZ_N);
-  OzTiles tiles{(int)((std::min(mslab, M) + OZ_M - 1) / OZ_M), tiles_n, sym ? 1 : 0};
-  int64_t ntiles = (int64_t)tiles.tiles_m * tiles_n;
+  OzTiles tiles{(int)((std::min(mslab, M) + OZ_M - 1) / OZ_M), tiles_n, sym ? 1 : 0,
+                ragged ? ragged->first : nullptr};
+  int64_t ntiles = ragged ? ragged->items : (int64_t)tiles.tiles_m * tiles_n;
   if (sym) {
     ntiles = 0;
     for (int m = 0; m < tiles.tiles_m; ++m) ntiles += std::min(2 * m + 2, tiles_n);
@@ -838,7 +867,7 @@ ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C,
   // partials written and summed.
   const int64_t kgroups = (kslab + kGroupChunks - 1) / kGroupChunks;
   int64_t nsplit = 1;
-  if (!b_lower && c.rin >= M) {
+  if (!b_lower && !ragged && c.rin >= M) {
     double best = 1e300;
     for (int64_t t = 1; t <= std::min<int64_t>(kgroups, 8 * kSMs / ntiles + 1); ++t) {
       const double cost = (double)((ntiles * t + kSMs - 1) / kSMs) * ((kgroups + t - 1) / t + 2) +
@@ -853,12 +882,17 @@ ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C,
   nsplit = (kgroups + sgroups - 1) / sgroups;
   if (ntiles > INT32_MAX || nsplit > 65535 || mslab / 128 > 65535 || npad / 128 > 65535)
     return TTG_BAD_ARG;
-  OzOut out{C, c.rin, c.rs, c.rs2, c.cs, 0, 0};
+  OzOut out{C, c.rin, c.rs, c.rs2, c.cs, 0, 0, nullptr, nullptr};
+  if (ragged) {
+    out.cs = 1;
+    out.base = ragged->base;
+    out.ld = ragged->ld;
+  }
   const bool partial = nsplit > 1 || sym;
   if (partial) {
     const size_t need = (size_t)nsplit * M * N * sizeof(double);
-    if (op->partial.bytes < need) TTG_TRY(op->partial.alloc(need));
-    out = OzOut{op->partial.as<double>(), M, 1, 0, M, M * N, 0};
+    if (partial_buf.bytes < need) TTG_TRY(partial_buf.alloc(need));
+    out = OzOut{partial_buf.as<double>(), M, 1, 0, M, M * N, 0, nullptr, nullptr};
   }
   for (int64_t q0 = 0; q0 < chunks; q0 += kslab) {
     const int64_t nq = std::min(kslab, chunks - q0);
@@ -868,7 +902,7 @@ ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C,
       TTG_TRY(slice(st, SA, pair ? 2 : 1, r0, rpad, q0 * OZ_K, nq, kexp, -1, diag));
       OzTiles tl = tiles;
       tl.tiles_m = (int)((rows + OZ_M - 1) / OZ_M);
-      const int64_t nt = sym ? ntiles : (int64_t)tl.tiles_m * tiles_n;
+      const int64_t nt = sym || ragged ? ntiles : (int64_t)tl.tiles_m * tiles_n;
       CUtensorMap mb;
       TTG_TRY(plane_map(&mb, pb, npad / 128 * nq));
       OzMma g{pa, ea + r0, eb, (int)rows, (int)N, (int)nq,
@@ -897,18 +931,25 @@ ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C,
   return TTG_OK;
 }
 
-ttg_status ozgemm_error(ttg_op* op) {
-  if (!op->oz_err.p) return TTG_OK;
+ttg_status ozgemm_error(cudaStream_t st, OzWork& ws) {
+  if (!ws.err.p) return TTG_OK;
   int e = 0;
-  TTG_CUDA_TRY(cudaMemcpyAsync(&e, op->oz_err.p, sizeof(int), cudaMemcpyDeviceToHost, op->stream));
-  TTG_CUDA_TRY(cudaStreamSynchronize(op->stream));
+  TTG_CUDA_TRY(cudaMemcpyAsync(&e, ws.err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+  TTG_CUDA_TRY(cudaStreamSynchronize(st));
   if (e) {
-    TTG_CUDA_TRY(cudaMemsetAsync(op->oz_err.p, 0, sizeof(int), op->stream));
+    TTG_CUDA_TRY(cudaMemsetAsync(ws.err.p, 0, sizeof(int), st));
     fprintf(stderr, "ttg: FP64 tensor-core GEMM: %s\n",
             e == 3 ? "a copy barrier out of phase" : "a bounded wait ran out");
     return e == 3 ? TTG_CUDA_ERR : TTG_TIMEOUT;
   }
   return TTG_OK;
 }
+
+ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C, OzLayout c,
+                  bool sym, bool b_lower, const OzOperand* kscale_of, const OzRagged* ragged) {
+  return ozgemm(op->stream, op->oz, op->partial, A, B, C, c, sym, b_lower, kscale_of, ragged);
+}
+
+ttg_status ozgemm_error(ttg_op* op) { return ozgemm_error(op->stream, op->oz); }
 
 }  // namespace ttg

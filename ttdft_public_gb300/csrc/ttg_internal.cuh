@@ -136,6 +136,28 @@ struct UmmaOp {
   DevBuf err;      // int: a bounded wait of the kernel ran out
 };
 
+// How the value update (hupdate.cu) splits the pattern: slabs of the row's y
+// coordinate, and within a slab its (y, x) index pairs by falling half-width in
+// z, in tiles of 128.
+struct UpdatePlan {
+  bool made = false;
+  int nq = 0;                 // z pairs |dz| <= bw in the order of |dz|
+  struct Slab {
+    int y0, y1;
+    int pair0, pairs;         // its part of `pairs`
+    int tile0, items;         // its part of the tile arrays, its GEMM items
+  };
+  std::vector<Slab> slabs;
+  int64_t out_max = 0;        // values of the largest slab
+  DevBuf pairs;      // int32 per slab pair: yp nxp + xp
+  DevBuf where;      // int32 [nyp nxp]: position of the pair in its slab, -1 if unused
+  DevBuf first;      // int32 per slab, tiles + 1: prefix sums of column tiles
+  DevBuf base;       // int64 per tile: offset of its values
+  DevBuf ld;         // int32 per tile: its columns
+  DevBuf zq;         // int32 [rz (2 bw + 1)]: position of the z pair, -1 outside
+  DevBuf zlist;      // int32 [nq]: z pair index i (2 bw + 1) + dz + bw of each position
+};
+
 // The fixed sparsity pattern of H_loc and where each entry lives in the device
 // formats, kept when the operator is created with Tucker ranks so that its
 // values can be recomputed on the device for a new potential (hupdate.cu).
@@ -153,6 +175,8 @@ struct Pattern {
   bool kinetic_set = false;
   DevBuf work;       // pair tables and the Tucker intermediates
   DevBuf work2;
+  UpdatePlan plan;   // ragged products of the value update, made on first use
+  DevBuf values;     // their results, of one slab
 };
 
 // Device time of the fused filter-degree kernels, by kind (TTG_KT_*): with
@@ -190,6 +214,15 @@ struct DensityWork {
   DevBuf amax;     // FP32 group maxima of the operands (the tensor-core slicing grid)
 };
 
+// Work buffers of the FP64 tensor-core GEMM (ozgemm.cu), grow-only.
+struct OzWork {
+  DevBuf planes;   // digit planes of the operands
+  DevBuf exp;      // row scales of the operands
+  DevBuf kexp;     // K scales (padded to whole chunks)
+  DevBuf diag;     // sums of d3^2 of the rows of X^T X
+  DevBuf err;      // error word
+};
+
 struct Csr {
   int64_t rows = 0, cols = 0, nnz = 0, max_row_nnz = 0;
   DevBuf ptr;      // int64
@@ -225,15 +258,11 @@ struct ttg_op {
   ttg::DevBuf kk0, kk1, kk2;  // k x k FP64 matrices
   ttg::DevBuf kk3;            // eigensolver scratch (k*k + 6k doubles)
   ttg::DevBuf chol;           // blocked Cholesky: the diagonal before factorisation
-  ttg::DevBuf oz_exp;         // FP64 tensor-core GEMM: row scales of its operands
-  ttg::DevBuf oz_kexp;        // FP64 tensor-core GEMM: K scales (padded to whole chunks)
-  ttg::DevBuf oz_err;         // FP64 tensor-core GEMM: error word
-  ttg::DevBuf oz_planes;      // FP64 tensor-core GEMM: digit planes of its operands
-  ttg::DevBuf oz_diag;        // FP64 tensor-core GEMM: sums of d3^2 of the rows of X^T X
+  ttg::OzWork oz;             // FP64 tensor-core GEMM
   ttg::DevBuf eigbuf;         // eigensolver refinement (5 k*k doubles)
   ttg::DevBuf eigf;           // FP32 tridiagonalisation scratch
   ttg::DevBuf partial;        // split-K partials for the Gram
-  ttg::DevBuf sth_a, sth_b, sth_part, sth_part2;  // STHOSVD work (grow-only)
+  ttg::DevBuf sth_a, sth_b, sth_part, sth_part2, sth_w;  // STHOSVD work (grow-only)
   ttg::DevBuf scal;           // small FP64 scratch (reductions, status)
   ttg::DevBuf status;         // int32 device status words
   cudaEvent_t ev[ttg::kMaxSlots] = {};
@@ -351,12 +380,24 @@ struct OzOperand {
   int64_t rs, ks;
   int64_t rin = INT64_MAX, rs2 = 0;   // rows in two levels
   int64_t kin = INT64_MAX, ks2 = 0;   // K in two levels
+  const int* idx = nullptr;           // r is idx[r] in the address
 };
 // Where C(m, n) goes: (m % rin) rs + (m / rin) rs2 + n cs.
 struct OzLayout {
   int64_t rs, cs;
   int64_t rin = INT64_MAX, rs2 = 0;
 };
+// A ragged product: of every 128 rows (tile mt) of C only the first ld[mt]
+// columns (even) are computed, stored row-major at base[mt] (even) + row ld[mt].
+// Device arrays: first = exclusive prefix sums of ceil(ld / 64), tiles + 1.
+struct OzRagged {
+  const int* first;
+  const int64_t* base;
+  const int* ld;
+  int items;                          // first[tiles]
+};
+// The most rows of A, of K values, that a ragged product takes with N rows of B.
+int64_t ozgemm_ragged_rows(int64_t K, int64_t N);
 // Whether ozgemm takes these operands (sizes; off with TTG_DISABLE_OZGEMM);
 // callers fall back to the double-FP32 CUDA-core GEMMs.
 bool ozgemm_supported(const OzOperand& A, const OzOperand& B);
@@ -368,9 +409,16 @@ bool ozgemm_supported(const OzOperand& A, const OzOperand& B);
 // B as B(n, k) 2^f_k, which leaves A B^T unchanged and keeps small K columns
 // of A (that B amplifies) at full precision.  TTG_OOM: no room for the digit
 // planes (at most kPlaneBudget, 1 GiB, for sizes beyond it).
+// `partial`: scratch of the split sums.
+ttg_status ozgemm(cudaStream_t st, OzWork& w, DevBuf& partial, const OzOperand& A,
+                  const OzOperand& B, double* C, OzLayout c, bool sym, bool b_lower = false,
+                  const OzOperand* kscale_of = nullptr, const OzRagged* ragged = nullptr);
+// The same on an operator's stream and buffers.
 ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C, OzLayout c,
-                  bool sym, bool b_lower = false, const OzOperand* kscale_of = nullptr);
+                  bool sym, bool b_lower = false, const OzOperand* kscale_of = nullptr,
+                  const OzRagged* ragged = nullptr);
 // Reads and clears the tensor-core GEMM's error word (synchronises).
+ttg_status ozgemm_error(cudaStream_t st, OzWork& w);
 ttg_status ozgemm_error(ttg_op* op);
 
 // dense.cu
