@@ -451,23 +451,44 @@ __global__ void __launch_bounds__(1024) k_tridiag_ql(T* A, T* Q, T* w, int n, in
 }
 
 // Sort eigenpairs ascending (stable rank sort), normalise each eigenvector's
-// sign so that its largest-magnitude component is positive.
-__global__ void k_sort_eig(const double* w, const double* V, double* w_out, double* V_out,
-                           int k) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < k; j += gridDim.x * blockDim.x) {
-    int rank = 0;
-    const double wj = w[j];
-    for (int i = 0; i < k; ++i) rank += (w[i] < wj) || (w[i] == wj && i < j);
-    w_out[rank] = wj;
-    double big = 0.0;
-    int ib = 0;
-    for (int i = 0; i < k; ++i) {
-      const double a = fabs(V[i + (int64_t)j * k]);
-      if (a > big) { big = a; ib = i; }
-    }
-    const double sg = V[ib + (int64_t)j * k] < 0 ? -1.0 : 1.0;
-    for (int i = 0; i < k; ++i) V_out[i + (int64_t)rank * k] = sg * V[i + (int64_t)j * k];
+// sign so that its largest-magnitude component (the first of equal ones) is
+// positive.  One CTA per pair (one thread per pair took 66 us at k = 160).
+__global__ void __launch_bounds__(128) k_sort_eig(const double* w, const double* V, double* w_out,
+                                                  double* V_out, int k) {
+  __shared__ double s_big[4];
+  __shared__ int s_at[4], s_rank[4];
+  const int j = blockIdx.x, tid = threadIdx.x;
+  const double wj = w[j];
+  const double* v = V + (int64_t)j * k;
+  int rank = 0, at = 0;
+  double big = 0.0;
+  for (int i = tid; i < k; i += 128) {
+    rank += (w[i] < wj) || (w[i] == wj && i < j);
+    const double a = fabs(v[i]);
+    if (a > big) { big = a; at = i; }
   }
+  for (int o = 16; o > 0; o >>= 1) {
+    rank += __shfl_xor_sync(0xffffffffu, rank, o);
+    const double b2 = __shfl_xor_sync(0xffffffffu, big, o);
+    const int a2 = __shfl_xor_sync(0xffffffffu, at, o);
+    if (b2 > big || (b2 == big && a2 < at)) { big = b2; at = a2; }
+  }
+  if ((tid & 31) == 0) {
+    s_big[tid >> 5] = big;
+    s_at[tid >> 5] = at;
+    s_rank[tid >> 5] = rank;
+  }
+  __syncthreads();
+  rank = 0;
+  big = s_big[0];
+  at = s_at[0];
+  for (int i = 0; i < 4; ++i) {
+    rank += s_rank[i];
+    if (s_big[i] > big || (s_big[i] == big && s_at[i] < at)) { big = s_big[i]; at = s_at[i]; }
+  }
+  const double sg = v[at] < 0 ? -1.0 : 1.0;
+  if (tid == 0) w_out[rank] = wj;
+  for (int i = tid; i < k; i += 128) V_out[i + (int64_t)rank * k] = sg * v[i];
 }
 
 // One step of the Ogita-Aishima iterative refinement of a symmetric
@@ -1007,7 +1028,7 @@ ttg_status syev_device(ttg_op* op, double* A, double* V, double* w, int k, int* 
     double* wtmp = op->scal.as<double>() + kScalJacobi;
     double* Vd = op->kk2.as<double>();
     TTG_TRY(sym_topk(op, A, k, k, wtmp, Vd, d_status));
-    k_sort_eig<<<(k + 127) / 128, 128, 0, op->stream>>>(wtmp, Vd, w, V, k); TTG_COUNT();
+    k_sort_eig<<<k, 128, 0, op->stream>>>(wtmp, Vd, w, V, k); TTG_COUNT();
     TTG_LAUNCHED(op);
     return TTG_OK;
   }
@@ -1068,7 +1089,7 @@ ttg_status syev_device(ttg_op* op, double* A, double* V, double* w, int k, int* 
     k_add<<<64, 256, 0, st>>>(Vd, VE, kk); TTG_COUNT();
     TTG_LAUNCHED(op);
   }
-  k_sort_eig<<<(k + 127) / 128, 128, 0, st>>>(wtmp, Vd, w, V, k); TTG_COUNT();
+  k_sort_eig<<<k, 128, 0, st>>>(wtmp, Vd, w, V, k); TTG_COUNT();
   TTG_LAUNCHED(op);
   return TTG_OK;
 }

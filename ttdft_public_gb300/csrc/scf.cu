@@ -541,11 +541,18 @@ __global__ void __launch_bounds__(256) k_dot_part(const double* __restrict__ G,
   }
 }
 
-__global__ void k_diag_sum(const double* __restrict__ A, int n, double* out) {
+__global__ void __launch_bounds__(256) k_diag_sum(const double* __restrict__ A, int n,
+                                                  double* out) {
+  __shared__ double red[8];
+  double s = 0.0;
+  for (int i = threadIdx.x; i < n; i += 256) s += A[i + (int64_t)i * n];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
   if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < n; ++i) s += A[i + (int64_t)i * n];
-    *out = s;
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) t += red[w];
+    *out = t;
   }
 }
 
@@ -618,29 +625,18 @@ ttg_status ttg_tucker_sthosvd(ttg_op* op, const double* t_dev, const int32_t* di
     if (n[d] <= 0 || n[d] > 2048) return TTG_BAD_ARG;
   cudaStream_t st = op->stream;
   const int64_t total = (int64_t)n[0] * n[1] * n[2];
-  DevBuf norm;
   DevBuf& A = op->sth_a;
   DevBuf& B = op->sth_b;
   DevBuf& part = op->sth_part;
   DevBuf& part2 = op->sth_part2;
   if (A.bytes < (size_t)total * 8) TTG_TRY(A.alloc(total * 8));
   if (B.bytes < (size_t)total * 8) TTG_TRY(B.alloc(total * 8));
-  TTG_TRY(norm.alloc(4096 * 8));
-  TTG_CUDA_TRY(cudaMemcpyAsync(A.p, t_dev, total * 8, cudaMemcpyDeviceToDevice, st));
-  // ||T||^2 for the truncation threshold eps^2 ||T||^2 / 3 per mode
-  {
-    std::vector<double> ones(4096, 1.0);
-    DevBuf w1;
-    TTG_TRY(w1.alloc(4096 * 8));
-    TTG_CUDA_TRY(cudaMemcpyAsync(w1.p, ones.data(), 4096 * 8, cudaMemcpyHostToDevice, st));
-    launch_wsum(st, A.as<double>(), A.as<double>(), w1.as<double>(), w1.as<double>(),
-                w1.as<double>(), n, norm.as<double>(), norm.as<double>() + 2048);
-    TTG_LAUNCHED(op);
-    TTG_CUDA_TRY(cudaStreamSynchronize(st));
-  }
-  double norm2 = 0.0;
-  TTG_CUDA_TRY(cudaMemcpy(&norm2, norm.as<double>() + 2048, 8, cudaMemcpyDeviceToHost));
-  const double thr = eps * eps * norm2 / 3.0;
+  // eigenvalues (up to 2048) and the trace of a mode's Gram matrix
+  if (!op->sth_w.p) TTG_TRY(op->sth_w.alloc((2048 + 8) * 8));
+  double* wdev = op->sth_w.as<double>();
+  double* tdev = wdev + 2048;
+  const double* cur_t = t_dev;                 // the tensor before mode d
+  double thr = 0.0;
   double* U[3] = {u0_dev, u1_dev, u2_dev};
   int cur[3] = {n[0], n[1], n[2]};
   for (int d = 0; d < 3; ++d) {
@@ -648,22 +644,23 @@ ttg_status ttg_tucker_sthosvd(ttg_op* op, const double* t_dev, const int32_t* di
     const int rcap = std::min(nd, (max_ranks && max_ranks[d] > 0) ? (int)max_ranks[d] : nd);
     const size_t kk = (size_t)nd * nd * 8;
     if (op->kk0.bytes < kk) TTG_TRY(op->kk0.alloc(kk));
-    TTG_TRY(mode_gram(op, A.as<double>(), cur, d, op->kk0.as<double>(), part, part2));
+    TTG_TRY(mode_gram(op, cur_t, cur, d, op->kk0.as<double>(), part, part2));
     // trace of the Gram = sum of all eigenvalues
-    k_diag_sum<<<1, 256, 0, st>>>(op->kk0.as<double>(), nd, norm.as<double>() + 2049); TTG_COUNT();
+    k_diag_sum<<<1, 256, 0, st>>>(op->kk0.as<double>(), nd, tdev); TTG_COUNT();
     TTG_LAUNCHED(op);
     // the rcap largest eigenpairs in FP64 (the truncation needs eigenvectors whose
     // eigenvalues are many orders below the largest one)
-    double* wdev = norm.as<double>() + 1024;
     TTG_TRY(sym_topk(op, op->kk0.as<double>(), nd, rcap, wdev, U[d], op->status.as<int>()));
     std::vector<double> w(rcap + 1);
     int stat = 0;
     TTG_CUDA_TRY(cudaMemcpyAsync(w.data(), wdev, rcap * 8, cudaMemcpyDeviceToHost, st));
-    TTG_CUDA_TRY(cudaMemcpyAsync(&w[rcap], norm.as<double>() + 2049, 8, cudaMemcpyDeviceToHost, st));
+    TTG_CUDA_TRY(cudaMemcpyAsync(&w[rcap], tdev, 8, cudaMemcpyDeviceToHost, st));
     TTG_CUDA_TRY(cudaMemcpyAsync(&stat, op->status.p, 4, cudaMemcpyDeviceToHost, st));
     TTG_CUDA_TRY(cudaStreamSynchronize(st));
     if (stat) return TTG_NOT_CONVERGED;
     const double trace = w[rcap];
+    // the first trace is ||T||^2: threshold eps^2 ||T||^2 / 3 per mode
+    if (d == 0) thr = eps * eps * trace / 3.0;
     // smallest r whose discarded eigenvalues sum to <= thr
     int r = rcap;   // eps 0: fixed rank
     double kept = 0.0;
@@ -676,13 +673,11 @@ ttg_status ttg_tucker_sthosvd(ttg_op* op, const double* t_dev, const int32_t* di
     }
     ranks_out[d] = r;
     // project: A <- A x_d U_d^T
-    TTG_TRY(mode_product(op, A.as<double>(), cur, d, U[d], r, B.as<double>(), part));
-    std::swap(A.p, B.p);
-    std::swap(A.bytes, B.bytes);
+    double* to = d == 2 ? core_dev : d == 1 ? B.as<double>() : A.as<double>();
+    TTG_TRY(mode_product(op, cur_t, cur, d, U[d], r, to, part));
+    cur_t = to;
     cur[d] = r;
   }
-  TTG_CUDA_TRY(cudaMemcpyAsync(core_dev, A.p, (size_t)cur[0] * cur[1] * cur[2] * 8,
-                               cudaMemcpyDeviceToDevice, st));
   TTG_CUDA_TRY(cudaStreamSynchronize(st));
   return ozgemm_error(op);
 }
@@ -695,39 +690,39 @@ ttg_status ttg_tucker_reconstruct(const double* core_dev, const int32_t* ranks,
     return TTG_BAD_ARG;
   Stream S(stream);
   const double* U[3] = {u0_dev, u1_dev, u2_dev};
-  int cur[3] = {ranks[0], ranks[1], ranks[2]};
+  const int64_t r0 = ranks[0], r1 = ranks[1], r2 = ranks[2], n0 = dims[0], n1 = dims[1], n2 = dims[2];
   DevBuf a, b, part;
-  const int64_t big = (int64_t)std::max(dims[0], ranks[0]) * std::max(dims[1], ranks[1]) *
-                      std::max(dims[2], ranks[2]);
-  TTG_TRY(a.alloc(big * 8));
-  TTG_TRY(b.alloc(big * 8));
-  TTG_CUDA_TRY(cudaMemcpyAsync(a.p, core_dev, (size_t)cur[0] * cur[1] * cur[2] * 8,
-                               cudaMemcpyDeviceToDevice, S.s));
-  // U_d is n_d x r_d column-major = (r_d x n_d)^T; as the row-major p x n matrix
-  // M of mode_product we need M[i, a] = U[i + n*a]: rows i, stride 1 between a
-  // -> pass through dgemm directly here
+  OzWork w;
+  TTG_TRY(a.alloc(n0 * r1 * r2 * 8));
+  TTG_TRY(b.alloc(n0 * n1 * r2 * 8));
+  // core (r0, r1, r2) -> a (n0, r1, r2) -> b (n0, n1, r2) -> out; U_d is n_d x r_d
+  // column-major.  On the tensor cores with the long dimension as the rows, or
+  // on the CUDA cores (360^3 from rank 72: 3.3 -> 0.6 ms).
+  const OzOperand A[3] = {{core_dev, r1 * r2, r0, r0, 1},
+                          {a.as<double>(), n0 * r2, r1, 1, n0, n0, n0 * r1},
+                          {b.as<double>(), n0 * n1, r2, 1, n0 * n1}};
+  const OzLayout L[3] = {{n0, 1}, {1, n0, n0, n0 * n1}, {1, n0 * n1}};
+  double* to[3] = {a.as<double>(), b.as<double>(), out_dev};
   for (int d = 0; d < 3; ++d) {
-    const int nd = dims[d], rd = cur[d];
-    const int64_t n0 = cur[0], n1 = cur[1], n2 = cur[2];
-    ttg_status s;
-    if (d == 0)
-      s = dgemm(S.s, nd, (int)(n1 * n2), rd, 1, DOp{U[0], 1, nd, 0}, DOp{a.as<double>(), 1, n0, 0},
-                b.as<double>(), 1, nd, 0, part);
-    else if (d == 1)
-      s = dgemm(S.s, (int)n0, nd, rd, (int)n2, DOp{a.as<double>(), 1, n0, n0 * n1},
-                DOp{U[1], nd, 1, 0}, b.as<double>(), 1, n0, n0 * nd, part);
-    else
-      s = dgemm(S.s, (int)(n0 * n1), nd, rd, 1, DOp{a.as<double>(), 1, n0 * n1, 0},
-                DOp{U[2], nd, 1, 0}, b.as<double>(), 1, n0 * n1, 0, part);
+    const int nd = dims[d], rd = ranks[d];
+    const OzOperand B{U[d], nd, rd, 1, nd};
+    ttg_status s = TTG_OOM;
+    if (use_oz(A[d], B)) s = ozgemm(S.s, w, part, A[d], B, to[d], L[d], false);
+    if (s == TTG_OOM) {
+      if (d == 0)
+        s = dgemm(S.s, nd, (int)(r1 * r2), rd, 1, DOp{U[0], 1, nd, 0}, DOp{core_dev, 1, r0, 0}, to[0],
+                  1, nd, 0, part);
+      else if (d == 1)
+        s = dgemm(S.s, (int)n0, nd, rd, (int)r2, DOp{a.as<double>(), 1, n0, n0 * r1},
+                  DOp{U[1], nd, 1, 0}, to[1], 1, n0, n0 * nd, part);
+      else
+        s = dgemm(S.s, (int)(n0 * n1), nd, rd, 1, DOp{b.as<double>(), 1, n0 * n1, 0},
+                  DOp{U[2], nd, 1, 0}, out_dev, 1, n0 * n1, 0, part);
+    }
     if (s != TTG_OK) return s;
-    std::swap(a.p, b.p);
-    std::swap(a.bytes, b.bytes);
-    cur[d] = nd;
   }
-  TTG_CUDA_TRY(cudaMemcpyAsync(out_dev, a.p, (size_t)dims[0] * dims[1] * dims[2] * 8,
-                               cudaMemcpyDeviceToDevice, S.s));
   TTG_CUDA_TRY(cudaStreamSynchronize(S.s));
-  return TTG_OK;
+  return ozgemm_error(S.s, w);
 }
 
 ttg_status ttg_hartree_energy(int32_t K, const double* alpha, const double* omega,
