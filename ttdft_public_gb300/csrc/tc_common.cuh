@@ -1,6 +1,6 @@
 // Building blocks of the tcgen05 kernels (tgemm.cu, ozgemm.cu): shared-memory
 // addresses and matrix descriptors, bounded mbarrier waits, TMA tile loads and
-// tensor-memory loads and stores.  Every wait is bounded (kTcMaxWait polls).
+// tensor-memory loads.  Every wait is bounded (kTcMaxWait polls).
 #pragma once
 
 #include <cuda.h>
@@ -96,25 +96,31 @@ __device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap* map, i
         : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld8(uint32_t addr, float* v) {
-  uint32_t r[8];
+// four 8-column loads and one wait, in one statement (the registers are
+// defined only after the wait)
+__device__ __forceinline__ void tmem_ld8x4(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                           float* v0, float* v1, float* v2, float* v3) {
+  uint32_t r[32];
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%33];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16,%17,%18,%19,%20,%21,%22,%23}, [%34];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%24,%25,%26,%27,%28,%29,%30,%31}, [%35];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7])
-      : "r"(addr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
-}
-
-__device__ __forceinline__ void tmem_st8(uint32_t addr, const float* v) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-      ::"r"(addr), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])),
-        "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])),
-        "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
+        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
+        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3)
       : "memory");
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    v0[j] = __uint_as_float(r[j]);
+    v1[j] = __uint_as_float(r[8 + j]);
+    v2[j] = __uint_as_float(r[16 + j]);
+    v3[j] = __uint_as_float(r[24 + j]);
+  }
 }
 
 }  // namespace tc

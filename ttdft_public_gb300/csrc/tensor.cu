@@ -66,10 +66,44 @@ __device__ __forceinline__ void warp_max_abs(float* amax, float v) {
   if ((threadIdx.x & 31) == 0 && m) atomicMax(reinterpret_cast<unsigned int*>(amax), m);
 }
 
-// F_t[i, a] = scale_t sum_q wq[q] exp(-alpha_t (x_i - xq_q)^2) U[q, a] in
-// FP64 on the CUDA cores (KSDFTPotential.cc:509-523), stored FP32 at
-// out[t ost + i osi + a] for a < r and zero for r <= a < rpad; amax[t] gets
-// the term's largest |F|.
+// The expansion factors F_t[i, a] = scale_t sum_q wq[q] exp(-alpha_t (x_i - xq_q)^2)
+// U[q, a] in FP64 (KSDFTPotential.cc:509-523): the weighted Gaussians E as a
+// matrix of (t, i) by q, its product with U as an FP64 tensor-core GEMM, and the
+// result rounded to FP32.  Summing on the FP64 pipe took 2.0 ms for the three
+// directions of the 64-atom case, the product takes 0.9 with the exponentials.
+__global__ void __launch_bounds__(256) k_gauss_rows(const double* __restrict__ alpha, int K,
+                                                    const double* __restrict__ x, int nx,
+                                                    const double* __restrict__ xq,
+                                                    const double* __restrict__ wq, int nq,
+                                                    double* __restrict__ E) {
+  const int row = blockIdx.x;                     // t nx + i
+  const double at = alpha[row / nx], xi = x[row % nx];
+  for (int q = threadIdx.x; q < nq; q += 256) {
+    const double d = xi - xq[q];
+    E[(int64_t)row * nq + q] = wq[q] * exp(-at * d * d);
+  }
+}
+
+// out[t ost + i osi + a] = scale_t F[(t, i)][a] for a < r, zero for r <= a < rpad;
+// amax[t] gets the term's largest |value|.
+__global__ void __launch_bounds__(256) k_factor_store(const double* __restrict__ F, int nx, int r,
+                                                      int rpad, float* __restrict__ out,
+                                                      int64_t ost, int64_t osi,
+                                                      const double* __restrict__ scale,
+                                                      float* __restrict__ amax) {
+  const int t = blockIdx.y;
+  const double sc = scale ? scale[t] : 1.0;
+  float vmax = 0.f;
+  for (int e = blockIdx.x * 256 + threadIdx.x; e < nx * rpad; e += gridDim.x * 256) {
+    const int i = e / rpad, a = e - i * rpad;
+    const float v = a < r ? (float)(sc * F[((int64_t)t * nx + i) * r + a]) : 0.f;
+    out[(int64_t)t * ost + (int64_t)i * osi + a] = v;
+    vmax = fmaxf(vmax, fabsf(v));
+  }
+  warp_max_abs(amax + t, vmax);
+}
+
+// The same sum on the FP64 pipe, where the tensor-core GEMM is off.
 __global__ void k_hfactor(const double* __restrict__ alpha, const double* __restrict__ x, int nx,
                           const double* __restrict__ xq, const double* __restrict__ wq, int nq,
                           const double* __restrict__ U, int r, int rpad, float* __restrict__ out,
@@ -114,9 +148,19 @@ __global__ void k_core_rows(const double* __restrict__ G, int rx, int64_t rows, 
   warp_max_abs(amax, vmax);
 }
 
-// FP64 column-major basis values (n x r) -> FP32 [i][a], row stride rp
-__global__ void k_basis_rows(const double* __restrict__ U, int n, int r, int rp,
-                             float* __restrict__ out, float* __restrict__ amax) {
+// FP64 column-major basis values (n x r) of direction blockIdx.y -> FP32 [i][a],
+// row stride rp
+struct BasisRows {
+  const double* U[3];
+  int n[3], r[3], rp[3];
+  float* out[3];
+};
+
+__global__ void k_basis_rows(const BasisRows S, float* __restrict__ amax_all) {
+  const int d = blockIdx.y, n = S.n[d], r = S.r[d], rp = S.rp[d];
+  const double* __restrict__ U = S.U[d];
+  float* __restrict__ out = S.out[d];
+  float* amax = amax_all + d;
   const int64_t total = (int64_t)n * r;
   float vmax = 0.f;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
@@ -146,6 +190,9 @@ __global__ void k_block_chunk(const double* __restrict__ X, int64_t n, int64_t l
   }
   warp_max_abs(amax + s, vmax);
 }
+
+// From this many flops a direction the factors' sums run on the tensor cores.
+constexpr double kFactorOzFlops = 5e7;
 
 // Device inputs of one Hartree evaluation (all FP64, device pointers).
 struct HartreeIn {
@@ -206,9 +253,36 @@ ttg_status hartree_tc(cudaStream_t st, HartreeWork& w, const HartreeIn& in, doub
   const int64_t osi[3] = {rxp, ryp, kt};
   const int rpad[3] = {(int)rxp, (int)ryp, (int)ktt};
   for (int d = 0; d < 3; ++d) {
-    k_hfactor<<<dim3(1, in.n[d], K), 128, in.nq[d] * 8, st>>>(
-        in.alpha, in.x[d], in.n[d], in.xq[d], in.wq[d], in.nq[d], in.U[d], in.r[d], rpad[d],
-        w.F[d].as<float>(), ost[d], osi[d], d == 2 ? in.omega : nullptr, am_f[d]); TTG_COUNT();
+    const double* scale = d == 2 ? in.omega : nullptr;
+    const int nx_d = in.n[d], nq_d = in.nq[d], r_d = in.r[d];
+    const int64_t rows = (int64_t)K * nx_d;
+    ttg_status s = TTG_OOM;
+    // few or short sums: the two launches less are worth more
+    if (2.0 * rows * nq_d * r_d >= kFactorOzFlops) {
+      const OzOperand U{in.U[d], r_d, nq_d, nq_d, 1};
+      if ((w.gauss.bytes >= (size_t)(rows * nq_d * 8) || w.gauss.alloc(rows * nq_d * 8) == TTG_OK) &&
+          (w.fd.bytes >= (size_t)(rows * r_d * 8) || w.fd.alloc(rows * r_d * 8) == TTG_OK)) {
+        const OzOperand E{w.gauss.as<double>(), rows, nq_d, nq_d, 1};
+        if (ozgemm_supported(E, U)) {
+          k_gauss_rows<<<(unsigned)rows, 256, 0, st>>>(in.alpha, K, in.x[d], nx_d, in.xq[d],
+                                                       in.wq[d], nq_d, w.gauss.as<double>()); TTG_COUNT();
+          TTG_CUDA_TRY(cudaGetLastError());
+          s = ozgemm(st, w.oz, w.ozpart, E, U, w.fd.as<double>(), OzLayout{r_d, 1}, false);
+          if (s == TTG_OK) {
+            k_factor_store<<<dim3(16, (unsigned)K), 256, 0, st>>>(
+                w.fd.as<double>(), nx_d, r_d, rpad[d], w.F[d].as<float>(), ost[d], osi[d], scale,
+                am_f[d]); TTG_COUNT();
+          } else if (s != TTG_OOM) {
+            return s;
+          }
+        }
+      }
+    }
+    if (s == TTG_OOM) {
+      k_hfactor<<<dim3(1, nx_d, K), 128, nq_d * 8, st>>>(
+          in.alpha, in.x[d], nx_d, in.xq[d], in.wq[d], nq_d, in.U[d], r_d, rpad[d],
+          w.F[d].as<float>(), ost[d], osi[d], scale, am_f[d]); TTG_COUNT();
+    }
     TTG_CUDA_TRY(cudaGetLastError());
   }
   k_core_rows<<<blocks_for((int64_t)rx * ry * rz), 256, 0, st>>>(
@@ -216,31 +290,36 @@ ttg_status hartree_tc(cudaStream_t st, HartreeWork& w, const HartreeIn& in, doub
   TTG_CUDA_TRY(cudaGetLastError());
   if (e0) TTG_CUDA_TRY(cudaEventRecord(e0, st));
   int* err = w.err.as<int>();
+  const TOperand A1{w.gf.as<float>(), (int64_t)ry * rz, rx, rxp, 0, 0, am_g};
+  const TOperand B1{w.F[0].as<float>(), nx, rx, rxp, K, (int64_t)nx * rxp, am_f[0]};
+  const TOperand A2{w.p2.as<float>(), (int64_t)nx * rz, ry, ryp, K, (int64_t)nx * rz * ryp, am_p};
+  const TOperand B2{w.F[1].as<float>(), ny, ry, ryp, K, (int64_t)ny * ryp, am_f[1]};
+  const TOperand A3{w.q.as<float>(), qrows, kt, kt, 0, 0, am_q};
+  const TOperand B3{w.F[2].as<float>(), nz, kt, kt, 0, 0, am_f[2]};
+  const int kg1 = (rx + 15) / 16, kg2 = (ry + 15) / 16, kg3 = (int)(ktt / 16);
+  TTG_TRY(grow(w.planes, std::max({tgemm_plane_bytes(TG_STORE_F32, A1, B1, K, 1, kg1),
+                                   tgemm_plane_bytes(TG_STORE_F32, A2, B2, K, 1, kg2),
+                                   tgemm_plane_bytes(TG_SUM_F64, A3, B3, 1, K, kg3)})));
   // 1) P_t[(i, c)][b] = sum_a G[(b, c)][a] Fx_t[i][a]      rows (b, c) x cols i, batch t
-  TOperand A1{w.gf.as<float>(), (int64_t)ry * rz, rx, rxp, 0, 0, am_g};
-  TOperand B1{w.F[0].as<float>(), nx, rx, rxp, K, (int64_t)nx * rxp, am_f[0]};
   TOut o1{w.p2.p, ry, 1, ryp, (int64_t)rz * ryp, (int64_t)nx * rz * ryp};
   o1.omax = am_p;
   o1.limit = (int64_t)K * nx * rz * ryp;
-  TTG_TRY(tgemm(st, TG_STORE_F32, A1, B1, K, 1, (int)((rx + 15) / 16), o1, err));
+  TTG_TRY(tgemm(st, TG_STORE_F32, A1, B1, K, 1, kg1, o1, err, w.planes));
   // 2) Q[(i + nx j)][(t, c)] = sum_b P_t[(i, c)][b] Fy_t[j][b]   rows (i, c) x cols j, batch t
-  TOperand A2{w.p2.as<float>(), (int64_t)nx * rz, ry, ryp, K, (int64_t)nx * rz * ryp, am_p};
-  TOperand B2{w.F[1].as<float>(), ny, ry, ryp, K, (int64_t)ny * ryp, am_f[1]};
   TOut o2{w.q.p, rz, 1, kt, (int64_t)nx * kt, ktt};
   o2.omax = am_q;
   o2.limit = qrows * kt;
-  TTG_TRY(tgemm(st, TG_STORE_F32, A2, B2, K, 1, (int)((ry + 15) / 16), o2, err));
+  TTG_TRY(tgemm(st, TG_STORE_F32, A2, B2, K, 1, kg2, o2, err, w.planes));
   // 3) V[(i, j), l] = sum_t sum_c Q[(i, j)][(t, c)] w_t Fz_t[l][c], one group per term
-  TOperand A3{w.q.as<float>(), qrows, kt, kt, 0, 0, am_q};
-  TOperand B3{w.F[2].as<float>(), nz, kt, kt, 0, 0, am_f[2]};
   TOut o3{V, qrows + 1, 1, 0, qrows, 0};
   o3.limit = qrows * nz;
-  TTG_TRY(tgemm(st, TG_SUM_F64, A3, B3, 1, K, (int)(ktt / 16), o3, err));
+  TTG_TRY(tgemm(st, TG_SUM_F64, A3, B3, 1, K, kg3, o3, err, w.planes));
   if (e1) TTG_CUDA_TRY(cudaEventRecord(e1, st));
   return TTG_OK;
 }
 
 ttg_status hartree_check(HartreeWork& w, cudaStream_t st) {
+  TTG_TRY(ozgemm_error(st, w.oz));
   if (!w.err.p) return TTG_OK;
   int e = 0;
   TTG_CUDA_TRY(cudaMemcpyAsync(&e, w.err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -275,23 +354,30 @@ ttg_status density_tc(ttg_op* op, const ttg_block* X, const double* occ, int rx,
   const int rr[3] = {rx, ry, rz}, nn[3] = {nx, ny, nz};
   const int64_t rp[3] = {rxp, ryp, rzp};
   const double* U[3] = {ux, uy, uz};
-  // group maxima: [Ux][Uy][Uz][X_s: S][P1_s: S][P2_s: S]
-  TTG_TRY(grow(D.amax, (size_t)(3 + 3 * (int64_t)k) * 4));
-  float* dm = D.amax.as<float>();
-  TTG_CUDA_TRY(cudaMemsetAsync(dm, 0, 3 * 4, st));
-  for (int d = 0; d < 3; ++d) {
-    TTG_TRY(grow(D.uf[d], (size_t)nn[d] * rp[d] * 4));
-    k_basis_rows<<<blocks_for((int64_t)nn[d] * rr[d]), 256, 0, st>>>(
-        U[d], nn[d], rr[d], (int)rp[d], D.uf[d].as<float>(), dm + d); TTG_COUNT();
-    TTG_LAUNCHED(op);
-  }
-  TTG_TRY(ensure_err(op->hw, st));
   // states per chunk: the three intermediates within a fixed budget
   const int64_t per_state = ((int64_t)ry * rz * rxp + (int64_t)rz * nx * ryp +
                              (int64_t)ny * nx * rzp) * 4;
   const char* env = getenv("TTG_DENSITY_CHUNK_BYTES");
   const int64_t budget = env ? std::max<int64_t>(atoll(env), 1) : ((int64_t)3 << 30);
   const int S = (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)k, budget / per_state, 65535}));
+  // group maxima: [Ux][Uy][Uz][X_s: S][P1_s: S][P2_s: S]
+  TTG_TRY(grow(D.amax, (size_t)(3 + 3 * (int64_t)k) * 4));
+  float* dm = D.amax.as<float>();
+  TTG_CUDA_TRY(cudaMemsetAsync(dm, 0, (size_t)(3 + 3 * S) * 4, st));
+  BasisRows br;
+  int64_t widest = 0;
+  for (int d = 0; d < 3; ++d) {
+    TTG_TRY(grow(D.uf[d], (size_t)nn[d] * rp[d] * 4));
+    br.U[d] = U[d];
+    br.n[d] = nn[d];
+    br.r[d] = rr[d];
+    br.rp[d] = (int)rp[d];
+    br.out[d] = D.uf[d].as<float>();
+    widest = std::max(widest, (int64_t)nn[d] * rr[d]);
+  }
+  k_basis_rows<<<dim3(blocks_for(widest), 3), 256, 0, st>>>(br, dm); TTG_COUNT();
+  TTG_LAUNCHED(op);
+  TTG_TRY(ensure_err(op->hw, st));
   TTG_TRY(grow(D.xt, (size_t)S * ry * rz * rxp * 4));
   TTG_TRY(grow(D.p1, (size_t)S * rz * nx * ryp * 4));
   TTG_TRY(grow(D.p2, (size_t)S * ny * nx * rzp * 4));
@@ -305,32 +391,38 @@ ttg_status density_tc(ttg_op* op, const ttg_block* X, const double* occ, int rx,
     float* am_x = dm + 3;
     float* am_1 = am_x + S;
     float* am_2 = am_1 + S;
-    TTG_CUDA_TRY(cudaMemsetAsync(am_x, 0, (size_t)3 * S * 4, st));
+    if (s0 > 0) TTG_CUDA_TRY(cudaMemsetAsync(am_x, 0, (size_t)3 * S * 4, st));
     const int gx = (int)std::min<int64_t>((op->n + 255) / 256, 64);
     k_block_chunk<<<dim3(gx, sc), 256, 0, st>>>(X->x.as<double>(), op->n, op->ld, s0, rx,
                                                 (int)rxp, D.xt.as<float>(), am_x); TTG_COUNT();
     TTG_LAUNCHED(op);
-    // 1) P1[s][c][i][b] = sum_a X_s[(b, c)][a] Ux[i][a]       rows (b, c), cols i, batch s
-    TOperand A1{D.xt.as<float>(), (int64_t)ry * rz, rx, rxp, sc, (int64_t)ry * rz * rxp, am_x};
-    TOperand B1{D.uf[0].as<float>(), nx, rx, rxp, 0, 0, dm};
-    TOut o1{D.p1.p, ry, 1, (int64_t)nx * ryp, ryp, (int64_t)rz * nx * ryp};
+    const TOperand A1{D.xt.as<float>(), (int64_t)ry * rz, rx, rxp, sc, (int64_t)ry * rz * rxp, am_x};
+    const TOperand B1{D.uf[0].as<float>(), nx, rx, rxp, 0, 0, dm};
+    const TOperand A2{D.p1.as<float>(), (int64_t)rz * nx, ry, ryp, sc, (int64_t)rz * nx * ryp, am_1};
+    const TOperand B2{D.uf[1].as<float>(), ny, ry, ryp, 0, 0, dm + 1};
+    const TOperand A3{D.p2.as<float>(), (int64_t)nx * ny, rz, rzp, sc, (int64_t)ny * nx * rzp, am_2};
+    const TOperand B3{D.uf[2].as<float>(), nz, rz, rzp, 0, 0, dm + 2};
+    const int kg1 = (rx + 15) / 16, kg2 = (ry + 15) / 16, kg3 = (rz + 15) / 16;
+    TTG_TRY(grow(D.planes, std::max({tgemm_plane_bytes(TG_STORE_F32, A1, B1, sc, 1, kg1),
+                                     tgemm_plane_bytes(TG_STORE_F32, A2, B2, sc, 1, kg2),
+                                     tgemm_plane_bytes(TG_SQSUM_F64, A3, B3, 1, sc, kg3)})));
+    // 1) P1[s][i][c][b] = sum_a X_s[(b, c)][a] Ux[i][a]       rows (b, c), cols i, batch s
+    TOut o1{D.p1.p, ry, 1, ryp, (int64_t)rz * ryp, (int64_t)rz * nx * ryp};
     o1.omax = am_1;
     o1.limit = (int64_t)sc * rz * nx * ryp;
-    TTG_TRY(tgemm(st, TG_STORE_F32, A1, B1, sc, 1, (rx + 15) / 16, o1, err));
+    TTG_TRY(tgemm(st, TG_STORE_F32, A1, B1, sc, 1, kg1, o1, err, D.planes));
     // 2) P2[s][j][i][c] = sum_b P1[s][(c, i)][b] Uy[j][b]       rows (c, i), cols j, batch s
-    TOperand A2{D.p1.as<float>(), (int64_t)rz * nx, ry, ryp, sc, (int64_t)rz * nx * ryp, am_1};
-    TOperand B2{D.uf[1].as<float>(), ny, ry, ryp, 0, 0, dm + 1};
-    TOut o2{D.p2.p, nx, rzp, 1, (int64_t)nx * rzp, (int64_t)ny * nx * rzp};
+    // (rows run through c first, so that a warp's rows store consecutive values:
+    // with i first this product took 4.8 ms instead of 0.86)
+    TOut o2{D.p2.p, rz, 1, rzp, (int64_t)nx * rzp, (int64_t)ny * nx * rzp};
     o2.omax = am_2;
     o2.limit = (int64_t)sc * ny * nx * rzp;
-    TTG_TRY(tgemm(st, TG_STORE_F32, A2, B2, sc, 1, (ry + 15) / 16, o2, err));
+    TTG_TRY(tgemm(st, TG_STORE_F32, A2, B2, sc, 1, kg2, o2, err, D.planes));
     // 3) rho[(i, j), l] (+)= sum_s w_s (sum_c P2[s][(j, i)][c] Uz[l][c])^2
-    TOperand A3{D.p2.as<float>(), (int64_t)nx * ny, rz, rzp, sc, (int64_t)ny * nx * rzp, am_2};
-    TOperand B3{D.uf[2].as<float>(), nz, rz, rzp, 0, 0, dm + 2};
     TOut o3{rho, (int64_t)nx * ny + 1, 1, 0, (int64_t)nx * ny, 0, D.w.as<float>() + s0,
             (accumulate || s0 > 0) ? 1 : 0};
     o3.limit = (int64_t)nx * ny * nz;
-    TTG_TRY(tgemm(st, TG_SQSUM_F64, A3, B3, 1, sc, (rz + 15) / 16, o3, err));
+    TTG_TRY(tgemm(st, TG_SQSUM_F64, A3, B3, 1, sc, kg3, o3, err, D.planes));
     op->launches += 3;
   }
   return TTG_OK;

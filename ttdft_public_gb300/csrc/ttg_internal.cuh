@@ -192,6 +192,15 @@ struct KernelTimer {
   long long count[TTG_KT_KINDS] = {};
 };
 
+// Work buffers of the FP64 tensor-core GEMM (ozgemm.cu), grow-only.
+struct OzWork {
+  DevBuf planes;   // digit planes of the operands
+  DevBuf exp;      // row scales of the operands
+  DevBuf kexp;     // K scales (padded to whole chunks)
+  DevBuf diag;     // sums of d3^2 of the rows of X^T X
+  DevBuf err;      // error word
+};
+
 // Work buffers of the Hartree kernel expansion (tensor.cu), grow-only and
 // owned by the operator, so the SCF's calls allocate nothing once warm.
 struct HartreeWork {
@@ -201,6 +210,11 @@ struct HartreeWork {
   DevBuf q;        // FP32 [(i, j)][(t, c)]
   int64_t q_layout[3] = {0, 0, 0};   // (rows, K, padded rank) the zeroed Q was laid out for
   DevBuf amax;     // FP32 group maxima of the operands (the tensor-core slicing grid)
+  DevBuf planes;   // slices of the operands
+  DevBuf gauss;    // FP64 weighted Gaussians of one direction, [(t, i)][q]
+  DevBuf fd;       // FP64 factors of one direction, [(t, i)][a]
+  DevBuf ozpart;
+  OzWork oz;       // their FP64 product
   DevBuf err;      // int: a bounded wait of the tensor-core kernel ran out
 };
 
@@ -212,15 +226,7 @@ struct DensityWork {
   DevBuf p2;       // FP32 [s][j][i][c]
   DevBuf w;        // FP32 weights 2 f_s
   DevBuf amax;     // FP32 group maxima of the operands (the tensor-core slicing grid)
-};
-
-// Work buffers of the FP64 tensor-core GEMM (ozgemm.cu), grow-only.
-struct OzWork {
-  DevBuf planes;   // digit planes of the operands
-  DevBuf exp;      // row scales of the operands
-  DevBuf kexp;     // K scales (padded to whole chunks)
-  DevBuf diag;     // sums of d3^2 of the rows of X^T X
-  DevBuf err;      // error word
+  DevBuf planes;   // slices of the operands
 };
 
 struct Csr {
