@@ -268,20 +268,17 @@ def run_ours(args, rank, world):
     n = s.N
     peak, peak_kind = peaks()
     roof = {}
-    # blocks wider than 256 states run as one tcgen05 launch per 256-column
-    # block: the roofline unit is one degree over the whole block
-    blocks = -(-k // 256) if k > 256 else 1
+    # a degree is one launch of its kernel, over all column blocks
     for kind, vsz in (("umma_fp32", 4), ("tc_fp32", 4), ("umma_bf16", 2), ("tc_bf16", 2)):
         ms, cnt = op.kernel_time(kind)
         if cnt == 0:
             continue
-        nb = blocks if kind.startswith("umma") else 1
-        per = ms / (cnt / nb) / 1e3          # seconds per degree
+        per = ms / cnt / 1e3                 # seconds per degree
         # algorithmic bytes of one degree: H in CSR form at the degree's value
         # width (value + int32 column per nonzero, row pointers), Y read, X read,
         # Ynew written
         bytes_deg = nnz * (vsz + 4) + 4 * (n + 1) + 3 * n * k * vsz
-        roof[kind] = {"launch_ms": ms / cnt, "launches": cnt, "launches_per_degree": nb,
+        roof[kind] = {"launch_ms": ms / cnt, "launches": cnt, "launches_per_degree": 1,
                       "degree_ms": per * 1e3, "bytes_per_degree": bytes_deg,
                       "flops_per_degree": 2.0 * nnz * k, "achieved": bytes_deg / per / 1e9}
     stages = {}
@@ -340,7 +337,7 @@ def run_ours(args, rank, world):
     if rank == 0:
         r32 = roof.get("umma_fp32") or roof["tc_fp32"]
         kb = "umma_bf16" if "umma_bf16" in roof else ("tc_bf16" if "tc_bf16" in roof else None)
-        kname = ("k_cheb_umma (one FP32 filter degree: tcgen05 SpMM, three-term BF16 "
+        kname = ("k_cheb_umma (one FP32 filter degree: tcgen05 SpMM, two-term FP16 "
                  "split, fused with the recurrence)" if "umma_fp32" in roof else
                  "k_cheb_tc<float, 5> (one FP32 filter degree: 3xTF32 mma.sync SpMM fused "
                  "with the recurrence)")

@@ -136,7 +136,7 @@ ttg_status ttg_op_elapsed_ms(ttg_op* op, int32_t slot0, int32_t slot1, float* ms
  * (no host wait per launch).  ttg_op_kernel_time synchronises the stream and
  * returns the total milliseconds and the launch count of one kind since
  * timing was switched on; enable = 0 switches it off and clears the totals. */
-#define TTG_KT_UMMA_FP32 0   /* tcgen05 FP32 degree (three-term BF16 split) */
+#define TTG_KT_UMMA_FP32 0   /* tcgen05 FP32 degree (two-term FP16 split) */
 #define TTG_KT_TC_FP32 1     /* mma.sync FP32 degree (3xTF32) */
 #define TTG_KT_TC_BF16 2     /* mma.sync BF16 degree */
 #define TTG_KT_ROWGROUP 3    /* CUDA-core row-group degree (any precision) */

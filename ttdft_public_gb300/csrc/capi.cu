@@ -199,15 +199,15 @@ ttg_status ttg_op_create_tucker(int64_t n, const int64_t* h_row_ptr, const int32
   const char* dis = getenv("TTG_DISABLE_TC");
   op->tc_disabled = dis && dis[0] == '1';
   if (!op->tc_disabled) {
-    // the mma.sync tiles serve block widths that are not multiples of 16;
-    // an op for wide blocks of multiples of 16 (the tcgen05 degrees run them
-    // in column blocks) does without them and their memory
+    // the mma.sync tiles serve BF16 degrees of widths that are not multiples
+    // of 16; an op for wide blocks of multiples of 16 (the tcgen05 degrees run
+    // them in column blocks) does without them and their memory
     if (!(max_k > 256 && max_k % 16 == 0)) {
       s = build_tiles(op, n, h_row_ptr, h_col, h_val, nproj, c_row_ptr, c_col, c_val,
                       tucker_ranks);
       if (s != TTG_OK) return fail(s);
     }
-    s = build_umma_tiles(op, n, h_row_ptr, h_col, h_val, nproj, c_row_ptr, c_col, c_val,
+    s = build_umma_tiles(op, n, h_row_ptr, h_col, h_val, nproj, c_row_ptr, c_col, c_val, d,
                          tucker_ranks);
     if (s != TTG_OK) return fail(s);
   }
@@ -444,11 +444,11 @@ ttg_status ttg_cheb_filter(ttg_op* op, ttg_block* X, int32_t m, double a, double
   if (cur != TTG_PREC_FP64) TTG_TRY(launch_convert(op, TTG_PREC_FP64, cur, X->x.p, xb, op->n, k));
   // degree 1: Y = (sigma1/e) (H X - c X)
   double alpha = sigma1 / e, beta = -c * alpha;
-  TTG_TRY(launch_proj_w(op, cur, xb, k));
-  TTG_TRY(launch_cheb_step(op, cur, xb, nullptr, yb, k, alpha, beta, 0.0));
+  TTG_TRY(launch_degree(op, cur, true, xb, nullptr, yb, k, alpha, beta, 0.0));
   for (int d = 2; d <= steps; ++d) {
     const int p = prec_of(d);
-    if (p != cur) {
+    const bool first = p != cur;
+    if (first) {
       void *nx, *ny;
       TTG_TRY(bufs_for(p, &nx, &ny));
       if (cur == TTG_PREC_FP64) {
@@ -474,8 +474,7 @@ ttg_status ttg_cheb_filter(ttg_op* op, ttg_block* X, int32_t m, double a, double
     alpha = 2.0 * sigma2 / e;
     beta = -c * alpha;
     const double delta = -sigma * sigma2;
-    TTG_TRY(launch_proj_w(op, cur, yb, k));
-    TTG_TRY(launch_cheb_step(op, cur, yb, xb, xb, k, alpha, beta, delta));
+    TTG_TRY(launch_degree(op, cur, first, yb, xb, xb, k, alpha, beta, delta));
     std::swap(xb, yb);
     sigma = sigma2;
   }
@@ -497,7 +496,7 @@ ttg_status ttg_apply_h(ttg_op* op, const ttg_block* X, ttg_block* HX) {
   if (X->k != HX->k || X == HX) return TTG_BAD_ARG;
   ttg_block* Xm = const_cast<ttg_block*>(X);   // its projector rows are scratch
   TTG_TRY(launch_proj_w(op, TTG_PREC_FP64, Xm->x.p, X->k));
-  TTG_TRY(launch_cheb_step(op, TTG_PREC_FP64, Xm->x.p, nullptr, HX->x.p, X->k, 1.0, 0.0, 0.0));
+  TTG_TRY(launch_cheb_step(op, TTG_PREC_FP64, true, Xm->x.p, nullptr, HX->x.p, X->k, 1.0, 0.0, 0.0));
   return TTG_OK;
 }
 
@@ -631,7 +630,7 @@ ttg_status ttg_rayleigh_ritz(ttg_op* op, ttg_block* X, int32_t rotate, double* w
   if (op->rr_prec == TTG_PREC_DF64)
     TTG_TRY(launch_apply_df64(op, X->x.as<double>(), op->w64.as<double>(), k));
   else
-    TTG_TRY(launch_cheb_step(op, TTG_PREC_FP64, X->x.p, nullptr, op->w64.p, k, 1.0, 0.0, 0.0));
+    TTG_TRY(launch_cheb_step(op, TTG_PREC_FP64, true, X->x.p, nullptr, op->w64.p, k, 1.0, 0.0, 0.0));
   TTG_TRY(kt_end(op));
   TTG_TRY(kt_begin(op, TTG_KT_RR_GRAM));
   TTG_TRY(gram_fp64(op, X->x.as<double>(), op->w64.as<double>(), k, op->kk0.as<double>(), true));
@@ -690,7 +689,7 @@ ttg_status ttg_lanczos_bounds(ttg_op* op, const double* v0_host, int32_t max_ite
   double* ab = op->scal.as<double>() + kScalLanczos;
   for (int it = 0; it < max_iter; ++it) {
     TTG_TRY(launch_proj_w(op, TTG_PREC_FP64, v, 1));
-    TTG_TRY(launch_cheb_step(op, TTG_PREC_FP64, v, nullptr, hv, 1, 1.0, 0.0, 0.0));
+    TTG_TRY(launch_cheb_step(op, TTG_PREC_FP64, true, v, nullptr, hv, 1, 1.0, 0.0, 0.0));
     TTG_TRY(lanczos_step(op, v, vp, hv, ab, it));
   }
   std::vector<double> abh(2 * max_iter);

@@ -67,7 +67,10 @@ struct UpdateArgs {
   const int* umma_pos;        // slot of the entry within its 128-row tile
   const int* umma_row;        // tile * 128 + lane of each row
   const int64_t* umma_tptr;   // slot offset of each tile (multiples of 16)
-  __nv_bfloat16* u16;         // the tiles' three BF16 planes (2048 elements apart)
+  __nv_bfloat16* u16;         // the tiles' BF16 plane
+  __half* h16;                // and their two FP16 planes (2048 elements apart)
+  const float* rscale;        // inverse scale of each tile row's FP16 planes
+  float* rmax;                // largest new |value| of each tile row
   int64_t n;
 };
 
@@ -93,6 +96,9 @@ __global__ void __launch_bounds__(256) k_update_values(const UpdateArgs a) {
   const double* MX = DZ + rz * rz;
   const double* MY = MX + rx * rx;
   const double* MZ = MY + ry * ry;
+  const int ur = a.u16 ? a.umma_row[row] : 0;
+  const float up = a.u16 ? 1.f / a.rscale[ur] : 1.f;       // a power of two
+  float hmax = 0.f;
   for (int64_t e = a.row_ptr[row] + lane; e < a.row_ptr[row + 1]; e += 32) {
     const int J = a.col[e];
     const int xJ = J % rx, yJ = (J / rx) % ry, zJ = J / (rx * ry);
@@ -125,37 +131,38 @@ __global__ void __launch_bounds__(256) k_update_values(const UpdateArgs a) {
     // value index in the row groups: (group slot offset + slot) * 8 + row in group
     const int64_t p = (a.rg_gptr[row >> 3] + a.rg_pos[e]) * 8 + (row & 7);
     a.v64[p] = val;
-    if (a.vdf) {
-      const float h = __double2float_rn(val);
-      a.vdf[p] = make_float2(h, __double2float_rn(val - (double)h));
-    }
-    if (a.v32) a.v32[p] = (float)val;
+    const float h = __double2float_rn(val);
+    if (a.vdf) a.vdf[p] = make_float2(h, __double2float_rn(val - (double)h));
+    if (a.v32) a.v32[p] = h;
     if (a.v16) a.v16[p] = __double2bfloat16(val);
     if (a.t32) {
       // fragment order of spmm_tc.cu: TF32 lane 4g+(j%4), element j/4;
       // BF16 lane 4g+((j%8)/2), element (j%2) + 2*(j/8)
       const int base = a.tile_base[e];
       const int j = a.tile_slot[e];
-      a.t32[(int64_t)(base + (j & 3)) * 4 + (j >> 2)] = (float)val;
+      a.t32[(int64_t)(base + (j & 3)) * 4 + (j >> 2)] = h;
       a.t16[(int64_t)(base + ((j & 7) >> 1)) * 4 + (j & 1) + 2 * (j >> 3)] = __double2bfloat16(val);
     }
     if (a.u16) {
-      // three BF16 terms, as the tile builder splits them
-      // element in plane 0: chunk (tile's first + slot / 16), canonical K-major
+      // the BF16 value and two FP16 terms of the scaled one, as the tile
+      // builder has them: chunk (tile's first + slot / 16), canonical K-major
       // position of (lane, slot % 16) within the chunk's 128 x 16 plane
-      const int ur = a.umma_row[row];
       const int m = ur & 127, sl = a.umma_pos[e];
       const int64_t chunk = a.umma_tptr[ur >> 7] / 16 + (sl >> 4);
       const int s16 = sl & 15;
-      __nv_bfloat16* u = a.u16 + chunk * 6144 + ((m >> 3) * 128 + (s16 >> 3) * 64 + (m & 7) * 8 +
-                                                 (s16 & 7));
-      const __nv_bfloat16 h0 = __float2bfloat16_rn((float)val);
-      const double r1 = val - (double)__bfloat162float(h0);
-      const __nv_bfloat16 h1 = __float2bfloat16_rn((float)r1);
-      u[0] = h0;
-      u[2048] = h1;
-      u[4096] = __float2bfloat16_rn((float)(r1 - (double)__bfloat162float(h1)));
+      const int at = (m >> 3) * 128 + (s16 >> 3) * 64 + (m & 7) * 8 + (s16 & 7);
+      a.u16[chunk * 2048 + at] = __float2bfloat16_rn(h);
+      const float v = h * up;
+      const __half v0 = __float2half_rn(v);
+      __half* u = a.h16 + chunk * 4096 + at;
+      u[0] = v0;
+      u[2048] = __float2half_rn(v - __half2float(v0));
+      if (fabsf(h) <= 3.402823466e38f) hmax = fmaxf(hmax, fabsf(h));
     }
+  }
+  if (a.u16) {
+    for (int o = 16; o > 0; o >>= 1) hmax = fmaxf(hmax, __shfl_xor_sync(0xffffffffu, hmax, o));
+    if (lane == 0) a.rmax[ur] = hmax;
   }
 }
 
@@ -381,6 +388,9 @@ ttg_status update_from_tables(ttg_op* op, const UpdateLayout& L) {
   a.umma_row = P.umma_row.as<int>();
   a.umma_tptr = op->umma.tptr.as<int64_t>();
   a.u16 = op->umma.n_tiles > 0 && P.umma_pos.p ? op->umma.hpl.as<__nv_bfloat16>() : nullptr;
+  a.h16 = reinterpret_cast<__half*>(op->umma.fp16);
+  a.rscale = op->umma.rscale.as<float>();
+  a.rmax = op->umma.rmax.as<float>();
   a.n = op->n;
   if (op->nnz_h == 0) return TTG_OK;           // no entry to update
   const int nxg = (rx + 7) / 8;
@@ -433,7 +443,7 @@ ttg_status update_from_tables(ttg_op* op, const UpdateLayout& L) {
     k_update_values<<<(unsigned)((int64_t)ry * nxg * rz), 256, 0, st>>>(a); TTG_COUNT();
     TTG_LAUNCHED(op);
   }
-  return TTG_OK;
+  return a.u16 ? launch_umma_rescale(op) : TTG_OK;
 }
 
 }  // namespace

@@ -863,26 +863,18 @@ static ttg_status launch_f64(ttg_op* op, const void* src, const void* xold, void
   return kt_end(op);
 }
 
-ttg_status launch_cheb_step(ttg_op* op, int prec, const void* src, const void* xold, void* dst,
-                            int k, double alpha, double beta, double delta) {
+ttg_status launch_degree(ttg_op* op, int prec, bool first, void* src, const void* xold, void* dst,
+                         int k, double alpha, double beta, double delta) {
+  // the FP32 tcgen05 degree forms W with its planes of the block
+  if (prec != TTG_PREC_FP32 || !umma_supported(op, prec, k)) TTG_TRY(launch_proj_w(op, prec, src, k));
+  return launch_cheb_step(op, prec, first, src, xold, dst, k, alpha, beta, delta);
+}
+
+ttg_status launch_cheb_step(ttg_op* op, int prec, bool first, const void* src, const void* xold,
+                            void* dst, int k, double alpha, double beta, double delta) {
   if (k <= 0 || k > op->max_k) return TTG_BAD_ARG;
   if (umma_supported(op, prec, k))
-    return launch_cheb_umma(op, prec, src, xold, dst, k, alpha, beta, delta);
-  // blocks wider than one MMA (N <= 256): the tcgen05 degree over column
-  // blocks of at most 256 states, each re-reading H (the reference's
-  // num_X_blocks, ChebyShevFilter.cc:97-170, splits its columns the same way)
-  if (k > 256 && k % 16 == 0 && umma_supported(op, prec, 256)) {
-    const int nblk = (k + 255) / 256;
-    const int kb = ((k + nblk - 1) / nblk + 15) / 16 * 16;
-    const size_t elem = prec == TTG_PREC_FP32 ? 4 : 2;
-    for (int c0 = 0; c0 < k; c0 += kb) {
-      const int kk = std::min(kb, k - c0);
-      TTG_TRY(launch_cheb_umma(op, prec, static_cast<const char*>(src) + c0 * elem,
-                               xold ? static_cast<const char*>(xold) + c0 * elem : nullptr,
-                               static_cast<char*>(dst) + c0 * elem, kk, alpha, beta, delta));
-    }
-    return TTG_OK;
-  }
+    return launch_cheb_umma(op, prec, first, src, xold, dst, k, alpha, beta, delta);
   if (tc_supported(op, prec, k))
     return launch_cheb_tc(op, prec, src, xold, dst, k, alpha, beta, delta);
   if (prec == TTG_PREC_FP64) {

@@ -120,10 +120,10 @@ struct TileOp {
   DevBuf v16;      // bf16,  [chunk][8 n-tiles][32 lanes][4]
 };
 
-// 128-row tiles for the tcgen05 filter degrees (spmm_umma.cu): H as three
-// BF16 planes per 16-slot chunk in the MMA operand layout (FP32 degrees use
-// all three, BF16 degrees plane 0), and the block's three BF16 planes that
-// the FP32 degrees gather.
+// 128-row tiles for the tcgen05 filter degrees (spmm_umma.cu): H per 16-slot
+// chunk in the MMA operand layout, one BF16 plane (BF16 degrees) and two FP16
+// planes of its scaled rows (FP32 degrees), and the block's two FP16 planes
+// that the FP32 degrees gather.
 struct UmmaOp {
   int64_t n_tiles = 0;
   int64_t slots = 0;
@@ -131,8 +131,20 @@ struct UmmaOp {
   DevBuf tcol;     // int32 [slots]
   DevBuf rowmap;   // int32 [n_tiles*128], -1 = padding
   DevBuf order;    // int32 [n_tiles], launch order: most chunks first
-  DevBuf hpl;      // bf16 [chunk][3][128 x 16]
-  DevBuf xpl;      // bf16 [3][n + nproj][k]
+  DevBuf hpl;      // bf16 [chunk][128 x 16], then fp16 [chunk][2][128 x 16]
+  uint16_t* fp16 = nullptr;   // the FP16 part of hpl
+  DevBuf xpl;      // fp16 [2][n + nproj][k rounded up to 16]
+  int ctas = 0;    // of a launch
+  DevBuf lptr;     // int32 [ctas+1], tiles of each CTA in
+  DevBuf litem;    // int32 [n_tiles]
+  DevBuf rscale;   // float [n_tiles*128]: inverse scale of each row
+  DevBuf rcmax;    // float [n_tiles*128]: largest scaled entry of C^T in it
+  DevBuf rmax;     // float [n_tiles*128]: largest entry of H written by the last update
+  DevBuf wscale;   // float [nproj]: scale of each projector's W
+  DevBuf cval;     // float [nnz_c]: C with the inverse of it
+  DevBuf cmax;     // uint32 [2][ld]: largest |value| of each block column (bits)
+  DevBuf ticket;   // int [nproj][column groups]: finished parts of W
+  int cside = 0;   // half of cmax that holds the current degree's
   DevBuf err;      // int: a bounded wait of the kernel ran out
 };
 
@@ -297,8 +309,12 @@ ttg_status kt_end(ttg_op* op);
 ttg_status build_row_groups(ttg_op* op, int64_t n, const int64_t* hp, const int32_t* hc,
                             const double* hv, int32_t nproj, const int64_t* cp,
                             const int32_t* cc, const double* cv, const double* d);
-ttg_status launch_cheb_step(ttg_op* op, int prec, const void* src, const void* xold,
+// first: not the degree after another of the same precision (of one filter)
+ttg_status launch_cheb_step(ttg_op* op, int prec, bool first, const void* src, const void* xold,
                             void* dst, int k, double alpha, double beta, double delta);
+// the projectors' W of src (its rows n..) and the degree
+ttg_status launch_degree(ttg_op* op, int prec, bool first, void* src, const void* xold, void* dst,
+                         int k, double alpha, double beta, double delta);
 ttg_status launch_proj_w(ttg_op* op, int prec, void* src, int k);
 ttg_status launch_apply_df64(ttg_op* op, const double* src, double* dst, int k);
 
@@ -310,10 +326,12 @@ bool tc_supported(const ttg_op* op, int prec, int k);
 // spmm_umma.cu
 ttg_status build_umma_tiles(ttg_op* op, int64_t n, const int64_t* hp, const int32_t* hc,
                             const double* hv, int32_t nproj, const int64_t* cp, const int32_t* cc,
-                            const double* cv, const int32_t* dims);
+                            const double* cv, const double* d, const int32_t* dims);
 bool umma_supported(const ttg_op* op, int prec, int k);
-ttg_status launch_cheb_umma(ttg_op* op, int prec, const void* src, const void* xold, void* dst,
-                            int k, double alpha, double beta, double delta);
+// first: not the degree after another of the same precision on the same op
+ttg_status launch_cheb_umma(ttg_op* op, int prec, bool first, const void* src, const void* xold,
+                            void* dst, int k, double alpha, double beta, double delta);
+ttg_status launch_umma_rescale(ttg_op* op);
 ttg_status umma_check_error(ttg_op* op);
 ttg_status launch_cheb_tc(ttg_op* op, int prec, const void* src, const void* xold, void* dst,
                           int k, double alpha, double beta, double delta);
