@@ -46,8 +46,10 @@
 //    have an issuing thread (warps 1 and 3): while one half waits for its eight
 //    epilogue warps to empty its accumulators, the other's MMAs have the tensor
 //    pipe, and the half that is ahead by then stays so.  One thread for both
-//    spent a third of its time in the commits (330 cycles each).  A chunk
-//    costs 36 KB of copies for 2 x 336 MMA cycles.
+//    spent a third of its time in the commits (330 cycles each).  They are
+//    elected (elect_one): the MMAs of a 512,000 x 1,200 orthonormalisation
+//    took 35.6 ms under `lane == 0`, 33.1 now.  A chunk costs 36 KB of copies
+//    for 2 x 336 MMA cycles.
 //  - warp 0, one thread: the copies (few and large: 18 copies of 1 to 4 KB a
 //    chunk took four times as long, at 85 ns each); warp 2, one thread: waits
 //    for a chunk's copies in order and publishes the count (a thread that
@@ -502,7 +504,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_mma(const __grid_constant__ 
   } else if (warp == 1 || warp == 3) {
     // ---- MMAs of one half: digit i of A times digits 0 .. 5 - i of B in one
     const int h = warp >> 1;
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t base0 = su32(smem), dcol = tmem + (uint32_t)(h * kHalfCols);
       uint32_t avail = 0, q = 0, gr = 0;                  // chunks, groups of this half
       for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {

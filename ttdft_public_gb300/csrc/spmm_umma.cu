@@ -167,13 +167,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity) {
   return false;
 }
 
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(p));
-  return p != 0;
-}
-
 __device__ __forceinline__ int mbar_test(uint64_t* b, uint32_t parity) {
   uint32_t ok;
   asm volatile(

@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tg_mma(const __grid_constant__ 
   } else if (warp == 1 || warp == 3) {
     // ---- MMAs of every other group into accumulator buffer b
     const int b = warp >> 1;
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t base0 = su32(smem), dcol = tmem + (uint32_t)(b * kBufCols);
       uint32_t avail = 0, gg = 0;                    // groups over all tiles
       for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
