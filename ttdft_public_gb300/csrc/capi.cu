@@ -627,10 +627,14 @@ ttg_status ttg_rayleigh_ritz(ttg_op* op, ttg_block* X, int32_t rotate, double* w
   // HX into w64 (FP64 values), then P = X^T HX
   TTG_TRY(kt_begin(op, TTG_KT_RR_HX));
   TTG_TRY(launch_proj_w(op, TTG_PREC_FP64, X->x.p, k));
-  if (op->rr_prec == TTG_PREC_DF64)
-    TTG_TRY(launch_apply_df64(op, X->x.as<double>(), op->w64.as<double>(), k));
-  else
+  if (op->rr_prec == TTG_PREC_DF64) {
+    ttg_status s = TTG_OOM;
+    if (oz_apply_supported(op, k)) s = launch_oz_apply(op, X->x.as<double>(), op->w64.as<double>(), k);
+    if (s == TTG_OOM) s = launch_apply_df64(op, X->x.as<double>(), op->w64.as<double>(), k);
+    TTG_TRY(s);
+  } else {
     TTG_TRY(launch_cheb_step(op, TTG_PREC_FP64, true, X->x.p, nullptr, op->w64.p, k, 1.0, 0.0, 0.0));
+  }
   TTG_TRY(kt_end(op));
   TTG_TRY(kt_begin(op, TTG_KT_RR_GRAM));
   TTG_TRY(gram_fp64(op, X->x.as<double>(), op->w64.as<double>(), k, op->kk0.as<double>(), true));

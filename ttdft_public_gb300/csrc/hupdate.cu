@@ -392,6 +392,7 @@ ttg_status update_from_tables(ttg_op* op, const UpdateLayout& L) {
   a.rscale = op->umma.rscale.as<float>();
   a.rmax = op->umma.rmax.as<float>();
   a.n = op->n;
+  op->ozrows.cut = false;
   if (op->nnz_h == 0) return TTG_OK;           // no entry to update
   const int nxg = (rx + 7) / 8;
   UpdatePlan& plan = P.plan;

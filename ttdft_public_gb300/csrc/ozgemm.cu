@@ -955,3 +955,632 @@ ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C,
 ttg_status ozgemm_error(ttg_op* op) { return ozgemm_error(op->stream, op->oz); }
 
 }  // namespace ttg
+
+// ------------------------------------------------------------- H X in FP64 ----
+//
+// The Rayleigh-Ritz product H X (eigensolver/MultTm.cu computes it in FP64) on
+// the tiles of the filter degrees (spmm_umma.cu: 128 rows, their sorted column
+// union in chunks of 16 slots), with the digits, levels and folds of k_oz_mma,
+// but seven of them: a row of H holds values far below its diagonal, and with
+// six its eigenvectors were off by twice what double-FP32 sums had (4.2e-10
+// against 2.3e-10).  A is a tile's rows of H, cut once per operator and set of
+// values into a 28 KB block a chunk; B are the gathered rows of X, cut before
+// each product and laid out row by row, for 32 states seven digits of 64 bytes
+// each (512 bytes with the place of an eighth).  Two such groups of a row are
+// an item's columns, and digit i of H times digits 0 .. 6-i of a group is one
+// MMA, as in k_oz_mma.  (Level 6 may pass 2^24 and lose its last place, 2^-64
+// of the product of the two scales.)
+// Bound: the MMAs' shared-memory reads and the copies (42 KB a chunk and 64
+// states through L2).  k_apply_df64 (spmm.cu) -> this, 64,000 functions: 160
+// states 14.8 -> 4.6 ms, 40 states 6.3 -> 1.7 ms; 1,728 functions, 16 states 0.47
+// -> 0.07 ms; H is cut in about 3 ms at 64,000 functions.  It is faster at every
+// width; the other kernel is left where there are no tiles or no room.
+
+namespace ttg {
+namespace {
+
+constexpr int kApThreads = 768;                       // 24 warps, the last four gather
+constexpr int kApGather = 4;
+constexpr int kApDigits = 7, kApLevels = 7;
+constexpr int kApH = kApDigits * kPlA;                // 28 KB: H's digits of a chunk
+constexpr int kApAtom = 16 * 128;                     // 16 slots x 128 bytes (two digits of 32 states)
+constexpr int kApAtoms = (kApDigits + 1) / 2;         // of a group
+constexpr int kApRows = 2 * kApAtoms * kApAtom;       // 16 KB: the gathered digits of a chunk
+constexpr int kApStages = 5;
+constexpr int kApSmem = kApStages * (kApH + kApRows) + 1024;
+constexpr int kXGroup = kApAtoms * 128;               // 512 bytes: a row's digits of 32 states
+constexpr int kApCols = kApLevels * OZ_H;             // 224
+
+// Seven balanced base-256 digits of v 2^(8 - e), rounded to 48 fractional bits;
+// as digits6, which has 40.
+__device__ __forceinline__ void digits7(double v, int e, float* d) {
+  const int hi = __double2hiint(v);
+  const uint32_t lo = (uint32_t)__double2loint(v);
+  const int E = (hi >> 20) & 0x7FF;
+  if (E == 0x7FF) {
+#pragma unroll
+    for (int i = 0; i < kApDigits; ++i) d[i] = __int_as_float(0x7fc00000);
+    return;
+  }
+  unsigned long long X = 0;
+  if (E > 0) {
+    const unsigned long long M =
+        ((unsigned long long)((hi & 0xFFFFF) | 0x100000) << 32) | lo;
+    // v 2^(8-e) 2^48 = M 2^(E - 1075 + 56 - e); |v| < 2^e makes the shift >= -3
+    const int rs = 1075 - 56 + e - E;
+    if (rs <= 0) X = M << -rs;
+    else if (rs < 63) X = (M + (1ull << (rs - 1))) >> rs;
+  }
+  // balanced digits, lowest first (see digits6), from the two 32-bit halves
+  int t = (int)(uint32_t)(X & 0xFFFFFFu), g[kApDigits];
+  g[6] = ((t + 128) & 255) - 128; t = (t + 128) >> 8;
+  g[5] = ((t + 128) & 255) - 128; t = (t + 128) >> 8;
+  g[4] = ((t + 128) & 255) - 128; t = (t + 128) >> 8;
+  t += (int)((X >> 24) & 0xFFFFFFu);
+  g[3] = ((t + 128) & 255) - 128; t = (t + 128) >> 8;
+  g[2] = ((t + 128) & 255) - 128; t = (t + 128) >> 8;
+  g[1] = ((t + 128) & 255) - 128; t = (t + 128) >> 8;
+  g[0] = t + (int)(X >> 48);                            // 0 .. 256
+  const int sm = hi >> 31;                              // 0 or -1
+#pragma unroll
+  for (int i = 0; i < kApDigits; ++i) d[i] = (float)((g[i] ^ sm) - sm);
+}
+
+// B operand (slots x states, states contiguous) in the 128-byte swizzle layout,
+// pieces of 128 bytes x 16 slots 2 KB apart (spmm_umma.cu)
+__device__ __forceinline__ uint64_t gathered_desc(uint32_t addr) {
+  uint64_t d = (uint64_t)((addr >> 4) & 0x3FFF);
+  d |= (uint64_t)(kApAtom >> 4) << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+
+// tile * 128 + lane of each row
+__global__ void k_oz_tile_rows(const int* __restrict__ rowmap, int64_t n, int* __restrict__ urow) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n && rowmap[i] >= 0) urow[rowmap[i]] = (int)i;
+}
+
+struct OzCut {
+  const int64_t* gptr;        // row groups: slots, columns, values
+  const int* gcol;
+  const double* v64;
+  const int64_t* tptr;        // tiles
+  const int* tcol;
+  const int* urow;
+  int* he;                    // largest biased exponent of each tile row
+  unsigned char* hd;          // digit blocks, zero
+  int64_t n;
+};
+
+// A block takes a row group, a thread every 32nd slot of one of its rows: the
+// row's scale, then its values' digits, each at the place that its column has
+// in the list of the row's tile (both lists are sorted: a search from the place
+// of the value before).
+__global__ void __launch_bounds__(256) k_oz_cut_rows(const OzCut a) {
+  __shared__ int top[8];
+  const int64_t s0 = a.gptr[blockIdx.x];
+  const int ns = (int)(a.gptr[blockIdx.x + 1] - s0), r = threadIdx.x & 7;
+  const int64_t row = (int64_t)blockIdx.x * 8 + r;
+  if (threadIdx.x < 8) top[r] = 0;
+  __syncthreads();
+  int m = 0;
+  for (int s = threadIdx.x >> 3; s < ns; s += 32)
+    m = max(m, (__double2hiint(__ldg(a.v64 + (s0 + s) * 8 + r)) >> 20) & 0x7FF);
+  atomicMax(&top[r], m);
+  __syncthreads();
+  if (row >= a.n) return;
+  const int ur = a.urow[row], lane = ur & 127, e = exp_of_bits(top[r]);
+  if (threadIdx.x < 8) a.he[ur] = top[r];
+  const int64_t t0 = a.tptr[ur >> 7];
+  const int nt = (int)(a.tptr[(ur >> 7) + 1] - t0);
+  unsigned char* out = a.hd + t0 / OZ_K * kApH + (lane >> 3) * 256 + (lane & 7) * 16;
+  int from = 0;
+  for (int s = threadIdx.x >> 3; s < ns; s += 32) {
+    const double v = __ldg(a.v64 + (s0 + s) * 8 + r);
+    if (((__double2hiint(v) & 0x7fffffff) | __double2loint(v)) == 0) continue;
+    const int col = __ldg(a.gcol + s0 + s);
+    int lo = from, hi = nt;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (__ldg(a.tcol + t0 + mid) < col) lo = mid + 1;
+      else hi = mid;
+    }
+    from = lo;
+    float d[kApDigits];
+    digits7(v, e, d);
+    unsigned char* o = out + (int64_t)(lo >> 4) * kApH + ((lo >> 3) & 1) * 128 + (lo & 7) * 2;
+#pragma unroll
+    for (int i = 0; i < kApDigits; ++i)
+      *reinterpret_cast<__nv_bfloat16*>(o + i * kPlA) = __float2bfloat16_rn(d[i]);
+  }
+}
+
+// Digits of the block's rows: eight states of a row a thread.
+__global__ void __launch_bounds__(256) k_oz_cut_states(const double* __restrict__ x, int64_t rows,
+                                                       int k, int64_t ld, int groups,
+                                                       const int* __restrict__ xe,
+                                                       unsigned char* __restrict__ xd) {
+  const int64_t total = rows * groups * 4;
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total;
+       i += (int64_t)gridDim.x * 256) {
+    const int64_t r = i / (groups * 4);
+    const int c = (int)(i - r * (groups * 4)) * 8;
+    const double* p = x + r * ld + c;
+    double v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      double2 q = make_double2(0.0, 0.0);
+      if (c + j + 1 < k) q = __ldg(reinterpret_cast<const double2*>(p + j));   // ld is a multiple of 8
+      else if (c + j < k) q.x = __ldg(p + j);
+      v[j] = q.x;
+      v[j + 1] = q.y;
+    }
+    uint32_t w[kApDigits][4];
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      float d0[kApDigits], d1[kApDigits];
+      digits7(v[j], c + j < k ? exp_of_bits(__ldg(xe + c + j)) : 0, d0);
+      digits7(v[j + 1], c + j + 1 < k ? exp_of_bits(__ldg(xe + c + j + 1)) : 0, d1);
+#pragma unroll
+      for (int d = 0; d < kApDigits; ++d) w[d][j / 2] = pack_bf16(d0[d], d1[d]);
+    }
+    unsigned char* o = xd + (r * groups + (c >> 5)) * kXGroup + (c & 31) * 2;
+#pragma unroll
+    for (int d = 0; d < kApDigits; ++d)
+      *reinterpret_cast<uint4*>(o + d * (OZ_H * 2)) = make_uint4(w[d][0], w[d][1], w[d][2], w[d][3]);
+  }
+}
+
+struct OzApply {
+  const int64_t* tptr;
+  const int* tcol;
+  const int* rowmap;
+  const int* lptr;            // tiles of each of `ctas` CTAs (spmm_umma.cu)
+  const int* litem;
+  int ctas, par, nblk;        // column blocks of 64 states
+  const unsigned char* hd;
+  const int* he;
+  const unsigned char* xd;
+  const int* xe;
+  int groups;                 // of 32 states in a row of xd
+  double* dst;
+  int64_t ld;
+  int k;
+  int* err;
+};
+
+// the CTA's items, as in k_cheb_umma; f returns false to stop
+template <typename F>
+__device__ __forceinline__ void apply_items(const OzApply& a, F f) {
+  const int q = blockIdx.x / a.ctas, g = blockIdx.x - q * a.ctas;
+  bool flip = false;
+  for (int b = q; b < a.nblk; b += a.par, flip = !flip) {
+    const int j = flip ? a.ctas - 1 - g : g, e = __ldg(a.lptr + j + 1);
+    for (int i = __ldg(a.lptr + j); i < e; ++i)
+      if (!f(__ldg(a.litem + i), b)) return;
+  }
+}
+
+// seven 4-column tensor-memory loads `step` columns apart and one wait
+__device__ __forceinline__ void tmem_ld4x7(uint32_t a, uint32_t step, float (*v)[4]) {
+  uint32_t r[28];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%28];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%4,%5,%6,%7}, [%29];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8,%9,%10,%11}, [%30];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%12,%13,%14,%15}, [%31];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%16,%17,%18,%19}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%20,%21,%22,%23}, [%33];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%24,%25,%26,%27}, [%34];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
+        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
+        "=r"(r[26]), "=r"(r[27])
+      : "r"(a), "r"(a + step), "r"(a + 2 * step), "r"(a + 3 * step), "r"(a + 4 * step),
+        "r"(a + 5 * step), "r"(a + 6 * step)
+      : "memory");
+#pragma unroll
+  for (int L = 0; L < kApLevels; ++L)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[L][j] = __uint_as_float(r[L * 4 + j]);
+}
+
+__global__ void __launch_bounds__(kApThreads, 1) k_oz_apply(const OzApply a) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = smem_raw + ((1024 - (su32(smem_raw) & 1023)) & 1023);
+  unsigned char* hring = smem + kApStages * kApRows;
+  __shared__ __align__(8) uint64_t full[kApStages], empty[kApStages];
+  __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2];
+  __shared__ __align__(8) uint64_t fin[2];
+  __shared__ uint32_t tmem_slot;
+  __shared__ uint32_t landed;                                 // chunks whose copies are there
+  __shared__ int abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 ::"r"(su32(&tmem_slot)), "r"(kTmemCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 32) {
+    for (int s = 0; s < kApStages; ++s) {
+      bar_init(&full[s], 2);                                  // H's copy, the gathering warp
+      bar_init(&empty[s], 2);
+    }
+    for (int b = 0; b < 2; ++b) {
+      bar_init(&acc_full[b], 1);
+      bar_init(&acc_empty[b], kEpiWarps);
+      bar_init(&fin[b], 1);
+    }
+    landed = 0;
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_slot;
+  volatile int* abrt = &abort_flag;
+  bool ok = true;
+
+  if (warp == 0) {
+    // ---- H: the digit block of chunk q into stage q % kApStages
+    if (lane == 0) {
+      uint64_t pol_stream;
+      asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_stream));
+      uint32_t q = 0;
+      apply_items(a, [&](int tile, int) {
+        const int64_t c0 = __ldg(a.tptr + tile) / OZ_K, c1 = __ldg(a.tptr + tile + 1) / OZ_K;
+        for (int64_t c = c0; c < c1; ++c, ++q) {
+          const int s = q % kApStages;
+          if (q >= kApStages && !bar_wait(&empty[s], (q / kApStages - 1) & 1, abrt, 0)) {
+            ok = false;
+            return false;
+          }
+          const uint32_t fb = su32(&full[s]);
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb),
+                       "r"(kApH) : "memory");
+          asm volatile(
+              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
+              " [%0], [%1], %2, [%3], %4;"
+              ::"r"(su32(hring + s * kApH)), "l"(a.hd + c * kApH), "r"(kApH), "r"(fb),
+                "l"(pol_stream) : "memory");
+        }
+        return true;
+      });
+      // on abort, let the copies already issued land: the gathering warps
+      // arrive for theirs before they stop
+      if (!ok)
+        for (uint32_t r = (q > kApStages ? q - kApStages : 0); r < q; ++r)
+          bar_drain(&full[r % kApStages], (r / kApStages) & 1);
+    }
+  } else if (warp == 2) {
+    // ---- chunks landed, in order
+    if (lane == 0) {
+      uint32_t q = 0;
+      apply_items(a, [&](int tile, int) {
+        const int nq = (int)((__ldg(a.tptr + tile + 1) - __ldg(a.tptr + tile)) / OZ_K);
+        for (int c = 0; c < nq; ++c, ++q) {
+          if (!bar_wait(&full[q % kApStages], (q / kApStages) & 1, abrt, 0)) {
+            ok = false;
+            return false;
+          }
+          asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(su32(&landed)),
+                       "r"(q + 1) : "memory");
+        }
+        return true;
+      });
+    }
+  } else if (warp == 1 || warp == 3) {
+    // ---- MMAs of one group of 32 states
+    const int h = warp >> 1;
+    if (elect_one()) {
+      const uint32_t hbase = su32(hring), xbase = su32(smem) + (uint32_t)(h * kApAtoms * kApAtom);
+      const uint32_t dcol = tmem + (uint32_t)(h * kApCols);
+      uint32_t avail = 0, q = 0, gr = 0;                  // chunks, exact sums of this half
+      apply_items(a, [&](int tile, int b) {
+        const int nq = (int)((__ldg(a.tptr + tile + 1) - __ldg(a.tptr + tile)) / OZ_K);
+        const bool on = (2 * b + h) * OZ_H < a.k;
+        for (int j = 0; j < nq; ++j, ++q) {
+          const int c = j % kGroupChunks, s = q % kApStages;
+          if (on && c == 0 && gr > 0 && !bar_wait(&acc_empty[h], (gr - 1) & 1, abrt, 0)) {
+            ok = false;
+            return false;
+          }
+          for (int i = 0; i < kTcMaxWait && avail <= q; ++i) {
+            asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(avail)
+                         : "r"(su32(&landed)) : "memory");
+            if (avail > q || *abrt) break;
+          }
+          if (avail <= q) {
+            ok = false;
+            *abrt = 1;
+            return false;
+          }
+          if (!on) {
+            bar_arrive(&empty[s]);
+            continue;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint64_t db = gathered_desc(xbase + (uint32_t)(s * kApRows));
+#pragma unroll
+          for (int i = 0; i < kApDigits; ++i) {
+            const uint64_t da = kmajor_desc(hbase + (uint32_t)(s * kApH + i * kPlA));
+            const uint32_t acc = (c > 0 || i > 0) ? 1u : 0u;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                ::"r"(dcol + (uint32_t)(i * OZ_H)), "l"(da), "l"(db),
+                  "r"(idesc_oz(OZ_H * (kApDigits - i)) | (1u << 16)), "r"(acc));
+          }
+          asm volatile(
+              "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+              ::"r"(su32(&empty[s])) : "memory");
+          if (c == kGroupChunks - 1 || j == nq - 1) {
+            asm volatile(
+                "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                ::"r"(su32(&acc_full[h])) : "memory");
+            ++gr;
+          }
+        }
+        return true;
+      });
+      asm volatile(
+          "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+          ::"r"(su32(&fin[h])) : "memory");
+      bar_drain(&fin[h], 0);
+    }
+  } else if (warp >= kEpiWarp0 + 2 * kEpiWarps) {
+    // ---- gathered rows, chunk q to warp q % kApGather (see k_cheb_umma)
+    const int pw = warp - kEpiWarp0 - 2 * kEpiWarps, lr = lane >> 3, lj = lane & 7;
+    uint64_t pol_keep;
+    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol_keep));
+    const uint32_t sw0 = (uint32_t)(lr * 128 + ((lj ^ lr) << 4));
+    const uint32_t sw1 = (uint32_t)((4 + lr) * 128 + ((lj ^ (4 + lr)) << 4));
+    const int64_t xrow = (int64_t)a.groups * kXGroup;
+    int pending = -1;                                         // stage of the chunk in flight
+    auto land = [&]() {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) bar_arrive(&full[pending]);
+      pending = -1;
+    };
+    uint32_t q0 = 0, q = pw;
+    apply_items(a, [&](int tile, int b) {
+      const int64_t t0 = __ldg(a.tptr + tile);
+      const int nq = (int)((__ldg(a.tptr + tile + 1) - t0) / OZ_K);
+      const int atoms = (2 * b + 1) * OZ_H < a.k ? 2 * kApAtoms : kApAtoms;
+      const int* colp = a.tcol + t0 + (lane & 15);
+      const unsigned char* xb = a.xd + (int64_t)b * 2 * kXGroup + 16 * lj;
+      const uint32_t end = q0 + (uint32_t)nq;
+      int next = q < end ? __ldg(colp + (int64_t)(q - q0) * OZ_K) : 0;
+      for (; q < end; q += kApGather) {
+        const int mine = next;
+        next = q + kApGather < end ? __ldg(colp + (int64_t)(q + kApGather - q0) * OZ_K) : 0;
+        const unsigned char* xs[4];
+#pragma unroll
+        for (int rq = 0; rq < 4; ++rq)
+          xs[rq] = xb + (int64_t)__shfl_sync(0xffffffffu, mine, 4 * rq + lr) * xrow;
+        const int s = q % kApStages;
+        if (q >= kApStages) {
+          const uint32_t par = (q / kApStages - 1) & 1;
+          int is = 0;
+          if (lane == 0) is = bar_test(&empty[s], par);
+          is = __shfl_sync(0xffffffffu, is, 0);
+          if (!is) {
+            if (pending >= 0) {
+              asm volatile("cp.async.wait_group 0;" ::: "memory");
+              land();
+            }
+            bool w = true;
+            if (lane == 0) w = bar_wait(&empty[s], par, abrt, 0);
+            ok = __shfl_sync(0xffffffffu, w, 0);
+            if (!ok) return false;
+          }
+        }
+        const uint32_t sb = su32(smem) + (uint32_t)(s * kApRows);
+#pragma unroll
+        for (int rq = 0; rq < 4; ++rq) {
+          const uint32_t drow = sb + (rq & 1 ? sw1 : sw0) + (rq >> 1) * 1024;
+#pragma unroll
+          for (int t = 0; t < 2 * kApAtoms; ++t)
+            if (t < atoms && (t % kApAtoms < kApAtoms - 1 || lj < 4))       // no eighth digit
+              asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;"
+                           ::"r"(drow + (uint32_t)(t * kApAtom)), "l"(xs[rq] + t * 128), "l"(pol_keep)
+                           : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (pending >= 0) {
+          asm volatile("cp.async.wait_group 1;" ::: "memory");
+          land();
+        }
+        pending = s;
+      }
+      q0 = end;
+      return true;
+    });
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (pending >= 0) land();
+  } else {
+    // ---- folds of a group of states, as in k_oz_mma, four columns at a time
+    const int h = (warp - kEpiWarp0) / kEpiWarps, qd = warp & 3;
+    const int cb = (((warp - kEpiWarp0) >> 2) & 1) * OZ_E;
+    const uint32_t acol = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(h * kApCols + cb);
+    uint32_t gr = 0;
+    apply_items(a, [&](int tile, int b) {
+      const int col0 = (2 * b + h) * OZ_H + cb;
+      if ((2 * b + h) * OZ_H >= a.k) return true;
+      const int nq = (int)((__ldg(a.tptr + tile + 1) - __ldg(a.tptr + tile)) / OZ_K);
+      const int ng = (nq + kGroupChunks - 1) / kGroupChunks;
+      float hi[OZ_E], lo[OZ_E];
+#pragma unroll
+      for (int c = 0; c < OZ_E; ++c) { hi[c] = 0.f; lo[c] = 0.f; }
+      for (int t = 0; t < ng; ++t, ++gr) {
+        bool wt = true;
+        if (lane == 0) wt = bar_wait(&acc_full[h], gr & 1, abrt, 32);
+        ok = __shfl_sync(0xffffffffu, wt, 0);
+        if (!ok) return false;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int cc = 0; cc < OZ_E; cc += 4) {
+          float S[kApLevels][4];
+          tmem_ld4x7(acol + cc, OZ_H, S);
+          if (cc + 4 == OZ_E) {              // the last loads are in registers: release the buffer
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) bar_arrive(&acc_empty[h]);
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            float f = S[0][i], l = 0.f;
+            float sc = 1.f / 256.f;
+#pragma unroll
+            for (int L = 1; L < kApLevels; ++L, sc *= (1.f / 256.f)) {
+              const float u = S[L][i] * sc;
+              const float h2 = f + u;
+              const float bv = h2 - f;
+              l += (f - (h2 - bv)) + (u - bv);
+              f = h2;
+            }
+            const float sum = hi[cc + i] + f;
+            const float bv = sum - hi[cc + i];
+            lo[cc + i] += (hi[cc + i] - (sum - bv)) + (f - bv) + l;
+            hi[cc + i] = sum;
+          }
+        }
+      }
+      const int64_t ur = (int64_t)tile * OZ_M + qd * 32 + lane;
+      const int row = __ldg(a.rowmap + ur);
+      if (row < 0) return true;
+      const int em = exp_of_bits(__ldg(a.he + ur)) - 16;
+      double* o = a.dst + row * a.ld + col0;
+#pragma unroll
+      for (int c = 0; c < OZ_E; c += 2) {
+        double v[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          v[u] = scaled_sum(hi[c + u], lo[c + u],
+                            em + exp_of_bits(__ldg(a.xe + min(col0 + c + u, a.k - 1))));
+        if (col0 + c + 1 < a.k)
+          *reinterpret_cast<double2*>(o + c) = make_double2(v[0], v[1]);
+        else if (col0 + c < a.k)
+          o[c] = v[0];
+      }
+      return true;
+    });
+  }
+  __syncwarp();
+  if (!ok) {
+    *abrt = 1;
+    atomicExch(a.err, 1);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+}
+
+}  // namespace
+
+bool oz_apply_supported(const ttg_op* op, int k) {
+  const UmmaOp& U = op->umma;
+  if (U.n_tiles == 0 || op->tc_disabled || op->rg.n_groups == 0) return false;
+  return k > 0;
+}
+
+// dst = H src; src's rows n .. hold W.  TTG_OOM (before any work): no room.
+ttg_status launch_oz_apply(ttg_op* op, const double* src, double* dst, int k) {
+  UmmaOp& U = op->umma;
+  OzRows& Z = op->ozrows;
+  cudaStream_t st = op->stream;
+  const int64_t chunks = U.slots / OZ_K, trows = U.n_tiles * OZ_M;
+  const int64_t rows = op->n + (op->C.nnz > 0 ? op->nproj : 0);
+  const int groups = (k + OZ_H - 1) / OZ_H;
+  auto grow = [&](DevBuf& b, size_t need) -> ttg_status {
+    if (b.bytes >= need) return TTG_OK;
+    const size_t had = b.bytes;
+    TTG_TRY(b.alloc(need));
+    op->device_bytes += (int64_t)need - (int64_t)had;
+    return TTG_OK;
+  };
+  if (!Z.hd.p) {
+    // at most a sixteenth of the memory
+    size_t free = 0, total = 0;
+    TTG_CUDA_TRY(cudaMemGetInfo(&free, &total));
+    if ((size_t)chunks * kApH > total / 16) return TTG_OOM;
+  }
+  TTG_TRY(grow(Z.hd, std::max<size_t>((size_t)chunks * kApH, 16)));
+  if (grow(Z.xd, (size_t)rows * groups * kXGroup) != TTG_OK) {
+    op->device_bytes -= (int64_t)Z.hd.bytes;
+    Z.hd.release();
+    Z.cut = false;
+    return TTG_OOM;
+  }
+  TTG_TRY(grow(Z.xe, (size_t)op->ld * sizeof(int)));
+  if (!op->oz.err.p) {
+    TTG_TRY(op->oz.err.alloc(sizeof(int)));
+    TTG_CUDA_TRY(cudaMemsetAsync(op->oz.err.p, 0, sizeof(int), st));
+  }
+  if (!Z.urow.p) {
+    TTG_TRY(grow(Z.urow, (size_t)op->n * sizeof(int)));
+    k_oz_tile_rows<<<(unsigned)((trows + 255) / 256), 256, 0, st>>>(U.rowmap.as<int>(), trows,
+                                                                  Z.urow.as<int>()); TTG_COUNT();
+    TTG_LAUNCHED(op);
+  }
+  if (!Z.he.p) TTG_TRY(grow(Z.he, (size_t)trows * sizeof(int)));
+  if (!Z.cut) {
+    TTG_CUDA_TRY(cudaMemsetAsync(Z.hd.p, 0, Z.hd.bytes, st));
+    TTG_CUDA_TRY(cudaMemsetAsync(Z.he.p, 0, Z.he.bytes, st));
+    const OzCut c{op->rg.gptr.as<int64_t>(), op->rg.gcol.as<int>(), op->rg.v64.as<double>(),
+                  U.tptr.as<int64_t>(), U.tcol.as<int>(), Z.urow.as<int>(), Z.he.as<int>(),
+                  Z.hd.as<unsigned char>(), op->n};
+    k_oz_cut_rows<<<(unsigned)op->rg.n_groups, 256, 0, st>>>(c); TTG_COUNT();
+    TTG_LAUNCHED(op);
+    Z.cut = true;
+  }
+  TTG_CUDA_TRY(cudaMemsetAsync(Z.xe.p, 0, (size_t)k * sizeof(int), st));
+  OzSlices S{};
+  S.o[0] = OzOperand{src, k, rows, 1, op->ld};
+  S.ebits[0] = Z.xe.as<int>();
+  const int64_t kb = std::max<int64_t>(64, (rows + 255) / 256);
+  k_rowexp_rows<<<dim3((unsigned)((k + 31) / 32), (unsigned)((rows + kb - 1) / kb), 1), dim3(32, 8), 0,
+                  st>>>(S, kb, nullptr, 0); TTG_COUNT();
+  TTG_LAUNCHED(op);
+  k_oz_cut_states<<<(unsigned)std::min<int64_t>((rows * groups * 4 + 255) / 256, 152 * 16), 256, 0, st>>>(
+      src, rows, k, op->ld, groups, Z.xe.as<int>(), Z.xd.as<unsigned char>()); TTG_COUNT();
+  TTG_LAUNCHED(op);
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  std::call_once(once, [] {
+    attr = cudaFuncSetAttribute(k_oz_apply, cudaFuncAttributeMaxDynamicSharedMemorySize, kApSmem);
+  });
+  if (attr != cudaSuccess) return TTG_CUDA_ERR;
+  OzApply a{};
+  a.tptr = U.tptr.as<int64_t>();
+  a.tcol = U.tcol.as<int>();
+  a.rowmap = U.rowmap.as<int>();
+  a.lptr = U.lptr.as<int>();
+  a.litem = U.litem.as<int>();
+  a.nblk = (k + OZ_N - 1) / OZ_N;
+  a.ctas = U.ctas;
+  a.par = std::max(1, std::min(a.nblk, kSMs / U.ctas));
+  a.hd = Z.hd.as<unsigned char>();
+  a.he = Z.he.as<int>();
+  a.xd = Z.xd.as<unsigned char>();
+  a.xe = Z.xe.as<int>();
+  a.groups = groups;
+  a.dst = dst;
+  a.ld = op->ld;
+  a.k = k;
+  a.err = op->oz.err.as<int>();
+  k_oz_apply<<<(unsigned)(a.ctas * a.par), kApThreads, kApSmem, st>>>(a); TTG_COUNT();
+  TTG_LAUNCHED(op);
+  return TTG_OK;
+}
+
+}  // namespace ttg

@@ -344,6 +344,8 @@ __global__ void __launch_bounds__(32 * kGroupRows) k_cheb_f64(
 // runs FP32 at many times its FP64 rate, so this carries the Rayleigh-Ritz
 // product H X at FP64-level accuracy several times faster than FP64 FMAs.
 // Source rows are float2 (hi, lo) pairs; H slots are float2 pairs too.
+// Used where launch_oz_apply (ozgemm.cu, three to seven times as fast) has no
+// tiles or no memory for H's digits.
 template <int G>
 __global__ void __launch_bounds__(512) k_apply_df64(
     const int64_t* __restrict__ gptr, const int* __restrict__ gcol,

@@ -226,6 +226,17 @@ struct OzWork {
   DevBuf err;      // error word
 };
 
+// H X in FP64 on the tensor cores (ozgemm.cu): the digits of H on the tiles of
+// UmmaOp, and of the block.
+struct OzRows {
+  DevBuf hd;       // [chunk][7][128 x 16] bf16
+  DevBuf he;       // int32 [n_tiles*128]: largest biased exponent of each row
+  DevBuf urow;     // int32 [n]: tile * 128 + lane of each row
+  DevBuf xd;       // bf16 [n + nproj][groups of 32 states][8][32], the last unused
+  DevBuf xe;       // int32 [k]: largest biased exponent of each column
+  bool cut = false;   // hd holds the digits of the current values
+};
+
 // Work buffers of the Hartree kernel expansion (tensor.cu), grow-only and
 // owned by the operator, so the SCF's calls allocate nothing once warm.
 struct HartreeWork {
@@ -290,6 +301,7 @@ struct ttg_op {
   ttg::DevBuf kk3;            // eigensolver scratch (k*k + 6k doubles)
   ttg::DevBuf chol;           // blocked Cholesky: the diagonal before factorisation
   ttg::OzWork oz;             // FP64 tensor-core GEMM
+  ttg::OzRows ozrows;         // FP64 tensor-core H X
   ttg::DevBuf eigbuf;         // eigensolver refinement (5 k*k doubles)
   ttg::DevBuf eigf;           // FP32 tridiagonalisation scratch
   ttg::DevBuf partial;        // split-K partials for the Gram
@@ -330,6 +342,9 @@ ttg_status launch_degree(ttg_op* op, int prec, bool first, void* src, const void
                          int k, double alpha, double beta, double delta);
 ttg_status launch_proj_w(ttg_op* op, int prec, void* src, int k);
 ttg_status launch_apply_df64(ttg_op* op, const double* src, double* dst, int k);
+// ozgemm.cu: the same product on the tensor cores; TTG_OOM: no room for H's digits
+bool oz_apply_supported(const ttg_op* op, int k);
+ttg_status launch_oz_apply(ttg_op* op, const double* src, double* dst, int k);
 
 // spmm_tc.cu
 ttg_status build_tiles(ttg_op* op, int64_t n, const int64_t* hp, const int32_t* hc,
