@@ -25,8 +25,8 @@
 // |dz| a pair needs a prefix of them, and with the (y, x) pairs sorted by w, tiles
 // of 128 of them share a prefix: one ragged FP64 GEMM on the tensor cores (a few
 // GB of values at most at a time, in slabs of y), from which the entries are
-// gathered.  64 atoms: 24.6 -> 12.9 ms in all, 9.1 of them the gather and the scattered
-// writes into the formats.  The per-entry sum stays for
+// gathered.  64 atoms: 24.6 -> 12.1 ms in all, 5.9 of
+// them the gather and the scattered writes into the formats.  The per-entry sum stays for
 // operators that the plan does not fit and where the tensor cores are off.
 
 #include <algorithm>
@@ -51,9 +51,7 @@ struct UpdateArgs {
   const double* PZp;          // [zp][c]
   int rc;                     // Tucker rank of the potential along z
   const double* G;            // values of the slab's (y, x) pairs by z pairs, or null
-  const int* where;           // position of a (y, x) pair in the slab
-  const int64_t* base;        // of each 128 pairs: offset of their values
-  const int* ld;              // and columns
+  const int* where;           // offset of a (y, x) pair's values
   const int* zq;              // position of a z pair
   int y0;                     // first y of the slab
   int64_t nxp;
@@ -82,6 +80,12 @@ __device__ __forceinline__ int pair_index(int i, int j, int bw) {
 // A block updates eight rows, neighbours in x (one row group where rx is a
 // multiple of 8), a warp each; blocks run through z first, whose rows gather
 // neighbouring values of the same (y, x) pairs.
+// An entry's value is at the end of a chain of loads (column, the pair's
+// offset, value), and the kernel is bound by their latency (FP64 pipe 30 %, L2
+// 25 %, HBM 2.7 TB/s at 28^3 functions).  So the chain runs ahead: while an entry
+// is computed and stored, the value of the lane's next one, the offset of the
+// one after and the column of the third are on their way.  64 atoms: 9.1 ms
+// without it, now 5.9.
 __global__ void __launch_bounds__(256) k_update_values(const UpdateArgs a) {
   const int lane = threadIdx.x & 31;
   const int nxg = (a.rx + 7) >> 3;
@@ -90,65 +94,91 @@ __global__ void __launch_bounds__(256) k_update_values(const UpdateArgs a) {
   if (xI >= a.rx) return;
   const int64_t row = xI + (int64_t)a.rx * (yI + (int64_t)a.ry * zI);
   const int rx = a.rx, ry = a.ry, rz = a.rz;
-  const double* DX = a.kin;
-  const double* DY = DX + rx * rx;
-  const double* DZ = DY + ry * ry;
-  const double* MX = DZ + rz * rz;
-  const double* MY = MX + rx * rx;
-  const double* MZ = MY + ry * ry;
-  const int ur = a.u16 ? a.umma_row[row] : 0;
+  const double* DX = a.kin + xI * rx;
+  const double* DY = a.kin + rx * rx + yI * ry;
+  const double* DZ = a.kin + rx * rx + ry * ry + zI * rz;
+  const int64_t mass = (int64_t)rx * rx + (int64_t)ry * ry + (int64_t)rz * rz;
+  const double* MX = DX + mass;
+  const double* MY = DY + mass;
+  const double* MZ = DZ + mass;
+  const int ur = a.u16 ? __ldg(a.umma_row + row) : 0;
+  const int64_t chunk0 = a.u16 ? __ldg(a.umma_tptr + (ur >> 7)) / 16 : 0;
   const float up = a.u16 ? 1.f / a.rscale[ur] : 1.f;       // a power of two
+  const int64_t rg0 = __ldg(a.rg_gptr + (row >> 3)) * 8 + (row & 7);
+  const int64_t e1 = __ldg(a.row_ptr + row + 1);
   float hmax = 0.f;
-  for (int64_t e = a.row_ptr[row] + lane; e < a.row_ptr[row + 1]; e += 32) {
-    const int J = a.col[e];
-    const int xJ = J % rx, yJ = (J / rx) % ry, zJ = J / (rx * ry);
-    const double dx = DX[xI * rx + xJ], mx = MX[xI * rx + xJ];
-    const double dy = DY[yI * ry + yJ], my = MY[yI * ry + yJ];
-    const double dz = DZ[zI * rz + zJ], mz = MZ[zI * rz + zJ];
+  auto column = [&](int64_t e) { return e < e1 ? __ldg(a.col + e) : -1; };
+  // offset of column J's value in G (0 where there is none)
+  auto offset = [&](int J, int& zq) {
+    if (J < 0 || !a.G) return zq = 0;
+    const int yx = J / rx, xJ = J - yx * rx, zJ = yx / ry, yJ = yx - zJ * ry;
+    zq = __ldg(a.zq + pair_index(zI, zJ, a.bw[2]));
+    return __ldg(a.where + (int64_t)pair_index(yI, yJ, a.bw[1]) * a.nxp + pair_index(xI, xJ, a.bw[0]));
+  };
+  int64_t e = __ldg(a.row_ptr + row) + lane;
+  int J0 = column(e), J1 = column(e + 32), J2 = column(e + 64);
+  int z0, z1;
+  int o0 = offset(J0, z0), o1 = offset(J1, z1);
+  double g0 = J0 >= 0 && a.G ? __ldg(a.G + o0 + z0) : 0.0;
+  for (; e < e1; e += 32) {
+    const double g1 = J1 >= 0 && a.G ? __ldg(a.G + o1 + z1) : 0.0;
+    int z2;
+    const int o2 = offset(J2, z2), J3 = column(e + 96), J = J0;
+    const int rg = __ldg(a.rg_pos + e), sl = a.u16 ? __ldg(a.umma_pos + e) : 0;
+    const int base = a.t16 ? __ldg(a.tile_base + e) : 0, j = a.t16 ? __ldg(a.tile_slot + e) : 0;
+    const int yxJ = J / rx, xJ = J - yxJ * rx, zJ = yxJ / ry, yJ = yxJ - zJ * ry;
+    const double dx = __ldg(DX + xJ), mx = __ldg(MX + xJ);
+    const double dy = __ldg(DY + yJ), my = __ldg(MY + yJ);
+    const double dz = __ldg(DZ + zJ), mz = __ldg(MZ + zJ);
     double val = 0.5 * (dx * my * mz + mx * dy * mz + mx * my * dz);
-    const int xp = pair_index(xI, xJ, a.bw[0]);
-    const int yp = pair_index(yI, yJ, a.bw[1]);
-    const int zp = pair_index(zI, zJ, a.bw[2]);
     if (a.G) {
-      const int p = __ldg(a.where + (int64_t)yp * a.nxp + xp), t = p >> 7;
-      val += __ldg(a.G + __ldg(a.base + t) + (int64_t)(p & 127) * __ldg(a.ld + t) + __ldg(a.zq + zp));
-    } else if (xp >= 0 && yp >= 0 && zp >= 0) {
-      const double* t2 = a.T2 + ((int64_t)yp * a.nxp + xp) * a.rc;
-      const double* pz = a.PZp + (int64_t)zp * a.rc;
-      // four independent partial sums: the FP64 FMA chain of one sum would
-      // otherwise serialise the rc terms of every entry
-      double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-      int c = 0;
-      for (; c + 3 < a.rc; c += 4) {
-        s0 = fma(pz[c], t2[c], s0);
-        s1 = fma(pz[c + 1], t2[c + 1], s1);
-        s2 = fma(pz[c + 2], t2[c + 2], s2);
-        s3 = fma(pz[c + 3], t2[c + 3], s3);
+      val += g0;
+    } else {
+      const int xp = pair_index(xI, xJ, a.bw[0]);
+      const int yp = pair_index(yI, yJ, a.bw[1]);
+      const int zp = pair_index(zI, zJ, a.bw[2]);
+      if (xp >= 0 && yp >= 0 && zp >= 0) {
+        const double* t2 = a.T2 + ((int64_t)yp * a.nxp + xp) * a.rc;
+        const double* pz = a.PZp + (int64_t)zp * a.rc;
+        // four independent partial sums: the FP64 FMA chain of one sum would
+        // otherwise serialise the rc terms of every entry
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+        int c = 0;
+        for (; c + 3 < a.rc; c += 4) {
+          s0 = fma(pz[c], t2[c], s0);
+          s1 = fma(pz[c + 1], t2[c + 1], s1);
+          s2 = fma(pz[c + 2], t2[c + 2], s2);
+          s3 = fma(pz[c + 3], t2[c + 3], s3);
+        }
+        for (; c < a.rc; ++c) s0 = fma(pz[c], t2[c], s0);
+        val += (s0 + s1) + (s2 + s3);
       }
-      for (; c < a.rc; ++c) s0 = fma(pz[c], t2[c], s0);
-      val += (s0 + s1) + (s2 + s3);
     }
+    J0 = J1;
+    J1 = J2;
+    J2 = J3;
+    o1 = o2;
+    z1 = z2;
+    g0 = g1;
     // value index in the row groups: (group slot offset + slot) * 8 + row in group
-    const int64_t p = (a.rg_gptr[row >> 3] + a.rg_pos[e]) * 8 + (row & 7);
+    const int64_t p = rg0 + (int64_t)rg * 8;
     a.v64[p] = val;
     const float h = __double2float_rn(val);
     if (a.vdf) a.vdf[p] = make_float2(h, __double2float_rn(val - (double)h));
     if (a.v32) a.v32[p] = h;
     if (a.v16) a.v16[p] = __double2bfloat16(val);
-    if (a.t32) {
+    if (a.t16) {
       // fragment order of spmm_tc.cu: TF32 lane 4g+(j%4), element j/4;
       // BF16 lane 4g+((j%8)/2), element (j%2) + 2*(j/8)
-      const int base = a.tile_base[e];
-      const int j = a.tile_slot[e];
-      a.t32[(int64_t)(base + (j & 3)) * 4 + (j >> 2)] = h;
+      if (a.t32) a.t32[(int64_t)(base + (j & 3)) * 4 + (j >> 2)] = h;
       a.t16[(int64_t)(base + ((j & 7) >> 1)) * 4 + (j & 1) + 2 * (j >> 3)] = __double2bfloat16(val);
     }
     if (a.u16) {
       // the BF16 value and two FP16 terms of the scaled one, as the tile
       // builder has them: chunk (tile's first + slot / 16), canonical K-major
       // position of (lane, slot % 16) within the chunk's 128 x 16 plane
-      const int m = ur & 127, sl = a.umma_pos[e];
-      const int64_t chunk = a.umma_tptr[ur >> 7] / 16 + (sl >> 4);
+      const int m = ur & 127;
+      const int64_t chunk = chunk0 + (sl >> 4);
       const int s16 = sl & 15;
       const int at = (m >> 3) * 128 + (s16 >> 3) * 64 + (m & 7) * 8 + (s16 & 7);
       a.u16[chunk * 2048 + at] = __float2bfloat16_rn(h);
@@ -285,7 +315,7 @@ ttg_status make_plan(ttg_op* op, const UpdateArgs& a, int64_t nxp, int64_t nyp, 
           s.items += (cols[w] + 63) / 64;
           off += 128 * (int64_t)cols[w];
         }
-        where[i] = s.pairs++;
+        where[i] = (int)(base.back() + (int64_t)(s.pairs++ % 128) * ld.back());
         pairs.push_back(i);
       }
     first.push_back(s.items);
@@ -381,8 +411,8 @@ ttg_status update_from_tables(ttg_op* op, const UpdateLayout& L) {
   a.vdf = op->rg.vdf.as<float2>();
   a.v32 = op->rg.v32.as<float>();
   a.v16 = op->rg.v16.as<__nv_bfloat16>();
-  a.t32 = op->tiles.n_tiles > 0 && P.tile_base.p ? op->tiles.v32.as<float>() : nullptr;
-  a.t16 = op->tiles.v16.as<__nv_bfloat16>();
+  a.t32 = op->tiles.v32.as<float>();
+  a.t16 = op->tiles.n_tiles > 0 && P.tile_base.p ? op->tiles.v16.as<__nv_bfloat16>() : nullptr;
   a.rg_gptr = op->rg.gptr.as<int64_t>();
   a.umma_pos = P.umma_pos.as<int>();
   a.umma_row = P.umma_row.as<int>();
@@ -421,12 +451,11 @@ ttg_status update_from_tables(ttg_op* op, const UpdateLayout& L) {
     for (size_t i = 0; i < plan.slabs.size(); ++i) {
       const UpdatePlan::Slab& sl = plan.slabs[i];
       if (sl.pairs == 0) continue;
-      a.base = plan.base.as<int64_t>() + sl.tile0;
-      a.ld = plan.ld.as<int>() + sl.tile0;
       a.y0 = sl.y0;
       OzOperand t2{w + off_t2, sl.pairs, rc, rc, 1};
       t2.idx = plan.pairs.as<int>() + sl.pair0;
-      const OzRagged R{plan.first.as<int>() + sl.tile0 + i, a.base, a.ld, sl.items};
+      const OzRagged R{plan.first.as<int>() + sl.tile0 + i, plan.base.as<int64_t>() + sl.tile0,
+                       plan.ld.as<int>() + sl.tile0, sl.items};
       const ttg_status gs = ozgemm(op, t2, pz, P.values.as<double>(), OzLayout{0, 1}, false, false,
                                    nullptr, &R);
       if (gs == TTG_OOM && i == 0) {

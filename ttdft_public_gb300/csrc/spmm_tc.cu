@@ -326,7 +326,9 @@ ttg_status build_tiles(ttg_op* op, int64_t n, const int64_t* hp, const int32_t* 
   const int64_t nchunk = slots / CS;
   std::vector<int32_t> tcol(std::max<int64_t>(slots, CS), 0);
   // per chunk and n-tile: 32 lanes x 4 values
-  std::vector<float> v32((size_t)std::max<int64_t>(nchunk, 1) * 8 * 32 * 4, 0.f);
+  // the tcgen05 tiles run every FP32 width that these would
+  const bool fp32 = !umma_enabled();
+  std::vector<float> v32(fp32 ? (size_t)std::max<int64_t>(nchunk, 1) * 8 * 32 * 4 : 0, 0.f);
   std::vector<uint16_t> v16((size_t)std::max<int64_t>(nchunk, 1) * 8 * 32 * 4, 0);
   // for value updates: per H_loc entry, the lane base ((chunk*8 + n-tile)*32 + 4g)
   // of its fragment and its slot within the 16-slot chunk
@@ -373,10 +375,12 @@ ttg_status build_tiles(ttg_op* op, int64_t n, const int64_t* hp, const int32_t* 
             const size_t o = (((size_t)(c0 + c) * 8 + nt) * 32 + l) * 4;
             auto H = [&](int sl) { return dense[(size_t)(c * CS + sl) * TR + row]; };
             // TF32 m16n8k8 B fragment: (k=q, n=g), (k=q+4, n=g), for k8 steps 0 and 1
-            v32[o + 0] = (float)H(q);
-            v32[o + 1] = (float)H(q + 4);
-            v32[o + 2] = (float)H(8 + q);
-            v32[o + 3] = (float)H(8 + q + 4);
+            if (fp32) {
+              v32[o + 0] = (float)H(q);
+              v32[o + 1] = (float)H(q + 4);
+              v32[o + 2] = (float)H(8 + q);
+              v32[o + 3] = (float)H(8 + q + 4);
+            }
             // BF16 m16n8k16 B fragment: (k=2q,2q+1; n=g), (k=2q+8,2q+9; n=g)
             v16[o + 0] = host_bf16(H(2 * q));
             v16[o + 1] = host_bf16(H(2 * q + 1));
@@ -391,13 +395,14 @@ ttg_status build_tiles(ttg_op* op, int64_t n, const int64_t* hp, const int32_t* 
   TTG_TRY(T.tptr.alloc((ntiles + 1) * sizeof(int64_t)));
   TTG_TRY(T.tcol.alloc(tcol.size() * sizeof(int32_t)));
   TTG_TRY(T.rowmap.alloc(rowmap.size() * sizeof(int32_t)));
-  TTG_TRY(T.v32.alloc(v32.size() * sizeof(float)));
+  if (fp32) TTG_TRY(T.v32.alloc(v32.size() * sizeof(float)));
   TTG_TRY(T.v16.alloc(v16.size() * sizeof(uint16_t)));
   TTG_CUDA_TRY(cudaMemcpyAsync(T.tptr.p, tptr.data(), T.tptr.bytes, cudaMemcpyHostToDevice, op->stream));
   TTG_CUDA_TRY(cudaMemcpyAsync(T.tcol.p, tcol.data(), T.tcol.bytes, cudaMemcpyHostToDevice, op->stream));
   TTG_CUDA_TRY(cudaMemcpyAsync(T.rowmap.p, rowmap.data(), T.rowmap.bytes, cudaMemcpyHostToDevice,
                                op->stream));
-  TTG_CUDA_TRY(cudaMemcpyAsync(T.v32.p, v32.data(), T.v32.bytes, cudaMemcpyHostToDevice, op->stream));
+  if (fp32)
+    TTG_CUDA_TRY(cudaMemcpyAsync(T.v32.p, v32.data(), T.v32.bytes, cudaMemcpyHostToDevice, op->stream));
   TTG_CUDA_TRY(cudaMemcpyAsync(T.v16.p, v16.data(), T.v16.bytes, cudaMemcpyHostToDevice, op->stream));
   if (keep && hp[n] > 0) {
     Pattern& P = op->pattern;
@@ -432,7 +437,7 @@ static ttg_status launch_tc_t(ttg_op* op, const void* hval, const void* src, con
 
 bool tc_supported(const ttg_op* op, int prec, int k) {
   if (op->tiles.n_tiles == 0 || op->tc_disabled) return false;
-  if (prec == TTG_PREC_FP32) return k % 4 == 0;
+  if (prec == TTG_PREC_FP32) return k % 4 == 0 && op->tiles.v32.p;
   if (prec == TTG_PREC_BF16) return k % 8 == 0;
   return false;
 }

@@ -968,17 +968,17 @@ void raise_max(float& m, float v) {
   if (v <= 3.402823466e38f && v > m) m = v;
 }
 
-int umma_disabled_by_env() {
-  const char* e = getenv("TTG_DISABLE_UMMA");
-  return e && e[0] == '1';
-}
-
 }  // namespace
+
+bool umma_enabled() {
+  const char* e = getenv("TTG_DISABLE_UMMA");
+  return !(e && e[0] == '1');
+}
 
 ttg_status build_umma_tiles(ttg_op* op, int64_t n, const int64_t* hp, const int32_t* hc,
                             const double* hv, int32_t nproj, const int64_t* cp, const int32_t* cc,
                             const double* cv, const double* d, const int32_t* dims) {
-  if (umma_disabled_by_env()) return TTG_OK;
+  if (!umma_enabled()) return TTG_OK;
   std::vector<int32_t> rowmap;
   int64_t ntiles;
   if (dims && dims[0] > 0 && dims[1] > 0 && dims[2] > 0 &&

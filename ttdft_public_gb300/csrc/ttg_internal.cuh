@@ -129,7 +129,7 @@ struct TileOp {
   DevBuf tptr;     // int64 [n_tiles+1], slot offsets (multiples of 16)
   DevBuf tcol;     // int32 [slots]
   DevBuf rowmap;   // int32 [n_tiles*64], -1 = padding
-  DevBuf v32;      // float, [chunk][8 n-tiles][32 lanes][4]
+  DevBuf v32;      // float, [chunk][8 n-tiles][32 lanes][4]; none beside tcgen05 tiles
   DevBuf v16;      // bf16,  [chunk][8 n-tiles][32 lanes][4]
 };
 
@@ -175,7 +175,7 @@ struct UpdatePlan {
   std::vector<Slab> slabs;
   int64_t out_max = 0;        // values of the largest slab
   DevBuf pairs;      // int32 per slab pair: yp nxp + xp
-  DevBuf where;      // int32 [nyp nxp]: position of the pair in its slab, -1 if unused
+  DevBuf where;      // int32 [nyp nxp]: offset of the pair's values in its slab, -1 if unused
   DevBuf first;      // int32 per slab, tiles + 1: prefix sums of column tiles
   DevBuf base;       // int64 per tile: offset of its values
   DevBuf ld;         // int32 per tile: its columns
@@ -352,6 +352,7 @@ ttg_status build_tiles(ttg_op* op, int64_t n, const int64_t* hp, const int32_t* 
                        const double* cv, const int32_t* dims);
 bool tc_supported(const ttg_op* op, int prec, int k);
 // spmm_umma.cu
+bool umma_enabled();   // TTG_DISABLE_UMMA is not set
 ttg_status build_umma_tiles(ttg_op* op, int64_t n, const int64_t* hp, const int32_t* hc,
                             const double* hv, int32_t nproj, const int64_t* cp, const int32_t* cc,
                             const double* cv, const double* d, const int32_t* dims);
