@@ -765,13 +765,13 @@ struct PrepareArgs {
 // What an FP32 degree needs of its block, in one launch: the two FP16 planes
 // of the scaled columns, and of W_a = sum_J Cd[a,J] Y[J,:] (rows n + a).
 // The first blocks sum `chunk` entries of a projector for 64 states (an eighth
-// of them a warp, 16 loads in flight); the last of a projector's blocks adds
+// of them a warp, eight loads in flight); the last of a projector's blocks adds
 // the parts in order and writes the planes.  The other blocks
 // split the rows, 8 states a thread.  Bound: the projectors' gathered rows
 // (L2) and the block read and written once.
-constexpr int kPrepAhead = 16;
-constexpr int kPrepChunk = 8 * kPrepAhead;       // the smallest chunk
-__global__ void __launch_bounds__(256) k_umma_prepare(const PrepareArgs a) {
+constexpr int kPrepAhead = 8;
+constexpr int kPrepChunk = 128;                  // the smallest chunk
+__global__ void __launch_bounds__(256, 5) k_umma_prepare(const PrepareArgs a) {
   const int tid = threadIdx.x;
   if ((int)blockIdx.x < a.proj_blocks) {
     __shared__ float2 red[8][32];
@@ -849,28 +849,42 @@ __global__ void __launch_bounds__(256) k_umma_prepare(const PrepareArgs a) {
   if (b0 == 0)
     for (int c = tid; c < a.k; c += 256) a.cmax_next[c] = 0u;
   const int kg = a.kp >> 3;
-  const int64_t total = a.n * kg;
-  for (int64_t i = b0 * 256 + tid; i < total; i += nb * 256) {
-    const int64_t r = total <= INT_MAX ? (int64_t)((uint32_t)i / (uint32_t)kg) : i / kg;
-    const int c = (int)(i - r * kg) * 8;
-    uint4 hi, lo;
-    __half* h = reinterpret_cast<__half*>(&hi);
-    __half* l = reinterpret_cast<__half*>(&lo);
+  const int64_t total = a.n * kg, step = nb * 256;
+  // two items (8 states of a row) at a time
+  for (int64_t i = b0 * 256 + tid; i < total; i += 2 * step) {
+    float4 v[2][2];
+    int c[2];
 #pragma unroll
-    for (int q = 0; q < 8; q += 4) {
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      uint4 m = make_uint4(0u, 0u, 0u, 0u);
-      if (c + q < a.k) {                              // k is a multiple of 4
-        v = *reinterpret_cast<const float4*>(a.src + r * a.ld + c + q);
-        m = *reinterpret_cast<const uint4*>(a.cmax + c + q);
+    for (int u = 0; u < 2; ++u) {
+      const int64_t at = i + u * step;
+      const int64_t r = total <= INT_MAX ? (int64_t)((uint32_t)at / (uint32_t)kg) : at / kg;
+      c[u] = (int)(at - r * kg) * 8;
+      v[u][0] = v[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (at < total) {                               // k is a multiple of 4
+        const float* p = a.src + r * a.ld + c[u];
+        if (c[u] < a.k) v[u][0] = *reinterpret_cast<const float4*>(p);
+        if (c[u] + 4 < a.k) v[u][1] = *reinterpret_cast<const float4*>(p + 4);
       }
-      split_half(v.x * scale_up(m.x), h[q], l[q]);
-      split_half(v.y * scale_up(m.y), h[q + 1], l[q + 1]);
-      split_half(v.z * scale_up(m.z), h[q + 2], l[q + 2]);
-      split_half(v.w * scale_up(m.w), h[q + 3], l[q + 3]);
     }
-    *reinterpret_cast<uint4*>(a.pl + i * 8) = hi;
-    *reinterpret_cast<uint4*>(a.pl + a.pstride + i * 8) = lo;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int64_t at = i + u * step;
+      if (at >= total) break;
+      uint4 hi, lo;
+      __half* h = reinterpret_cast<__half*>(&hi);
+      __half* l = reinterpret_cast<__half*>(&lo);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        uint4 m = make_uint4(0u, 0u, 0u, 0u);
+        if (c[u] + 4 * q < a.k) m = __ldg(reinterpret_cast<const uint4*>(a.cmax + c[u] + 4 * q));
+        split_half(v[u][q].x * scale_up(m.x), h[4 * q], l[4 * q]);
+        split_half(v[u][q].y * scale_up(m.y), h[4 * q + 1], l[4 * q + 1]);
+        split_half(v[u][q].z * scale_up(m.z), h[4 * q + 2], l[4 * q + 2]);
+        split_half(v[u][q].w * scale_up(m.w), h[4 * q + 3], l[4 * q + 3]);
+      }
+      *reinterpret_cast<uint4*>(a.pl + at * 8) = hi;
+      *reinterpret_cast<uint4*>(a.pl + a.pstride + at * 8) = lo;
+    }
   }
 }
 
