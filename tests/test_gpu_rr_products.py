@@ -13,10 +13,12 @@ from ttdft_public_gb300 import api, system
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n, k", [(300, 32), (1000, 33), (1000, 64), (1000, 97), (20100, 160), (20100, 40)])
-def test_ritz_values(n, k):
+# the last: about 380,000 chunks of H, more than are held at a time
+@pytest.mark.parametrize("n, k, band", [(300, 32, 150), (1000, 33, 150), (1000, 64, 150), (1000, 97, 150),
+                                        (20100, 160, 150), (20100, 40, 150), (260000, 32, 1500)])
+def test_ritz_values(n, k, band):
     rng = np.random.default_rng(n + k)
-    col = np.clip(np.arange(n)[:, None] + rng.integers(-150, 150, (n, 15)), 0, n - 1)
+    col = np.clip(np.arange(n)[:, None] + rng.integers(-band, band, (n, 15)), 0, n - 1)
     M = sp.csr_matrix((rng.standard_normal(n * 15), (np.repeat(np.arange(n), 15), col.ravel())), shape=(n, n))
     M = M + M.T
     d = 10.0 ** rng.uniform(-2, 2, n)

@@ -69,6 +69,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <vector>
 #include <mutex>
 
 #include "ttg_internal.cuh"
@@ -1051,8 +1052,9 @@ struct OzCut {
   const int* tcol;
   const int* urow;
   int* he;                    // largest biased exponent of each tile row
-  unsigned char* hd;          // digit blocks, zero
+  unsigned char* hd;          // digit blocks of tiles [t0, t1), zero
   int64_t n;
+  int t0, t1;
 };
 
 // A block takes a row group, a thread every 32nd slot of one of its rows: the
@@ -1061,9 +1063,16 @@ struct OzCut {
 // of the value before).
 __global__ void __launch_bounds__(256) k_oz_cut_rows(const OzCut a) {
   __shared__ int top[8];
+  const int64_t first = (int64_t)blockIdx.x * 8;
+  bool any = false;                              // the same for all threads
+  for (int64_t i = first; i < min(first + 8, a.n); ++i) {
+    const int t = __ldg(a.urow + i) >> 7;
+    any |= t >= a.t0 && t < a.t1;
+  }
+  if (!any) return;
   const int64_t s0 = a.gptr[blockIdx.x];
   const int ns = (int)(a.gptr[blockIdx.x + 1] - s0), r = threadIdx.x & 7;
-  const int64_t row = (int64_t)blockIdx.x * 8 + r;
+  const int64_t row = first + r;
   if (threadIdx.x < 8) top[r] = 0;
   __syncthreads();
   int m = 0;
@@ -1073,10 +1082,11 @@ __global__ void __launch_bounds__(256) k_oz_cut_rows(const OzCut a) {
   __syncthreads();
   if (row >= a.n) return;
   const int ur = a.urow[row], lane = ur & 127, e = exp_of_bits(top[r]);
+  if ((ur >> 7) < a.t0 || (ur >> 7) >= a.t1) return;
   if (threadIdx.x < 8) a.he[ur] = top[r];
   const int64_t t0 = a.tptr[ur >> 7];
   const int nt = (int)(a.tptr[(ur >> 7) + 1] - t0);
-  unsigned char* out = a.hd + t0 / OZ_K * kApH + (lane >> 3) * 256 + (lane & 7) * 16;
+  unsigned char* out = a.hd + (t0 - a.tptr[a.t0]) / OZ_K * kApH + (lane >> 3) * 256 + (lane & 7) * 16;
   int from = 0;
   for (int s = threadIdx.x >> 3; s < ns; s += 32) {
     const double v = __ldg(a.v64 + (s0 + s) * 8 + r);
@@ -1141,6 +1151,7 @@ struct OzApply {
   const int* lptr;            // tiles of each of `ctas` CTAs (spmm_umma.cu)
   const int* litem;
   int ctas, par, nblk;        // column blocks of 64 states
+  int t0, t1;                 // tiles whose digits hd holds
   const unsigned char* hd;
   const int* he;
   const unsigned char* xd;
@@ -1159,8 +1170,10 @@ __device__ __forceinline__ void apply_items(const OzApply& a, F f) {
   bool flip = false;
   for (int b = q; b < a.nblk; b += a.par, flip = !flip) {
     const int j = flip ? a.ctas - 1 - g : g, e = __ldg(a.lptr + j + 1);
-    for (int i = __ldg(a.lptr + j); i < e; ++i)
-      if (!f(__ldg(a.litem + i), b)) return;
+    for (int i = __ldg(a.lptr + j); i < e; ++i) {
+      const int tile = __ldg(a.litem + i);
+      if (tile >= a.t0 && tile < a.t1 && !f(tile, b)) return;
+    }
   }
 }
 
@@ -1234,8 +1247,9 @@ __global__ void __launch_bounds__(kApThreads, 1) k_oz_apply(const OzApply a) {
       uint64_t pol_stream;
       asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_stream));
       uint32_t q = 0;
+      const int64_t h0 = __ldg(a.tptr + a.t0) / OZ_K;
       apply_items(a, [&](int tile, int) {
-        const int64_t c0 = __ldg(a.tptr + tile) / OZ_K, c1 = __ldg(a.tptr + tile + 1) / OZ_K;
+        const int64_t c0 = __ldg(a.tptr + tile) / OZ_K - h0, c1 = __ldg(a.tptr + tile + 1) / OZ_K - h0;
         for (int64_t c = c0; c < c1; ++c, ++q) {
           const int s = q % kApStages;
           if (q >= kApStages && !bar_wait(&empty[s], (q / kApStages - 1) & 1, abrt, 0)) {
@@ -1493,12 +1507,16 @@ bool oz_apply_supported(const ttg_op* op, int k) {
   return k > 0;
 }
 
-// dst = H src; src's rows n .. hold W.  TTG_OOM (before any work): no room.
+// dst = H src; src's rows n .. hold W.  H's digits are cut for slabs of tiles
+// that fit into a 32nd of the memory: the whole operator up to about 64,000
+// functions, whose digits are then kept for the next product with the same
+// values; a larger one is cut again for every product (a tenth of its time).
+// TTG_OOM (before any work): no room.
 ttg_status launch_oz_apply(ttg_op* op, const double* src, double* dst, int k) {
   UmmaOp& U = op->umma;
   OzRows& Z = op->ozrows;
   cudaStream_t st = op->stream;
-  const int64_t chunks = U.slots / OZ_K, trows = U.n_tiles * OZ_M;
+  const int64_t trows = U.n_tiles * OZ_M;
   const int64_t rows = op->n + (op->C.nnz > 0 ? op->nproj : 0);
   const int groups = (k + OZ_H - 1) / OZ_H;
   auto grow = [&](DevBuf& b, size_t need) -> ttg_status {
@@ -1508,13 +1526,25 @@ ttg_status launch_oz_apply(ttg_op* op, const double* src, double* dst, int k) {
     op->device_bytes += (int64_t)need - (int64_t)had;
     return TTG_OK;
   };
-  if (!Z.hd.p) {
-    // at most a sixteenth of the memory
+  if (Z.slabs.empty()) {
     size_t free = 0, total = 0;
     TTG_CUDA_TRY(cudaMemGetInfo(&free, &total));
-    if ((size_t)chunks * kApH > total / 16) return TTG_OOM;
+    const int64_t most = std::max<int64_t>((int64_t)(total / 32 / kApH), 1);
+    std::vector<int64_t> tp(U.n_tiles + 1);
+    TTG_CUDA_TRY(cudaMemcpyAsync(tp.data(), U.tptr.p, tp.size() * 8, cudaMemcpyDeviceToHost, st));
+    TTG_CUDA_TRY(cudaStreamSynchronize(st));
+    std::vector<int> slabs(1, 0);
+    for (int64_t t = 0; t < U.n_tiles; ++t) {
+      if ((tp[t + 1] - tp[t]) / OZ_K > most) return TTG_OOM;
+      if ((tp[t + 1] - tp[slabs.back()]) / OZ_K > most) slabs.push_back((int)t);
+    }
+    slabs.push_back((int)U.n_tiles);
+    Z.most = 0;
+    for (size_t i = 1; i < slabs.size(); ++i)
+      Z.most = std::max<int64_t>(Z.most, (tp[slabs[i]] - tp[slabs[i - 1]]) / OZ_K);
+    Z.slabs = slabs;
   }
-  TTG_TRY(grow(Z.hd, std::max<size_t>((size_t)chunks * kApH, 16)));
+  TTG_TRY(grow(Z.hd, std::max<size_t>((size_t)Z.most * kApH, 16)));
   if (grow(Z.xd, (size_t)rows * groups * kXGroup) != TTG_OK) {
     op->device_bytes -= (int64_t)Z.hd.bytes;
     Z.hd.release();
@@ -1533,16 +1563,6 @@ ttg_status launch_oz_apply(ttg_op* op, const double* src, double* dst, int k) {
     TTG_LAUNCHED(op);
   }
   if (!Z.he.p) TTG_TRY(grow(Z.he, (size_t)trows * sizeof(int)));
-  if (!Z.cut) {
-    TTG_CUDA_TRY(cudaMemsetAsync(Z.hd.p, 0, Z.hd.bytes, st));
-    TTG_CUDA_TRY(cudaMemsetAsync(Z.he.p, 0, Z.he.bytes, st));
-    const OzCut c{op->rg.gptr.as<int64_t>(), op->rg.gcol.as<int>(), op->rg.v64.as<double>(),
-                  U.tptr.as<int64_t>(), U.tcol.as<int>(), Z.urow.as<int>(), Z.he.as<int>(),
-                  Z.hd.as<unsigned char>(), op->n};
-    k_oz_cut_rows<<<(unsigned)op->rg.n_groups, 256, 0, st>>>(c); TTG_COUNT();
-    TTG_LAUNCHED(op);
-    Z.cut = true;
-  }
   TTG_CUDA_TRY(cudaMemsetAsync(Z.xe.p, 0, (size_t)k * sizeof(int), st));
   OzSlices S{};
   S.o[0] = OzOperand{src, k, rows, 1, op->ld};
@@ -1578,8 +1598,23 @@ ttg_status launch_oz_apply(ttg_op* op, const double* src, double* dst, int k) {
   a.ld = op->ld;
   a.k = k;
   a.err = op->oz.err.as<int>();
-  k_oz_apply<<<(unsigned)(a.ctas * a.par), kApThreads, kApSmem, st>>>(a); TTG_COUNT();
-  TTG_LAUNCHED(op);
+  for (size_t i = 1; i < Z.slabs.size(); ++i) {
+    a.t0 = Z.slabs[i - 1];
+    a.t1 = Z.slabs[i];
+    if (!Z.cut) {
+      TTG_CUDA_TRY(cudaMemsetAsync(Z.hd.p, 0, Z.hd.bytes, st));
+      TTG_CUDA_TRY(cudaMemsetAsync(Z.he.as<int>() + (int64_t)a.t0 * OZ_M, 0,
+                                   (size_t)(a.t1 - a.t0) * OZ_M * sizeof(int), st));
+      const OzCut c{op->rg.gptr.as<int64_t>(), op->rg.gcol.as<int>(), op->rg.v64.as<double>(),
+                    U.tptr.as<int64_t>(), U.tcol.as<int>(), Z.urow.as<int>(), Z.he.as<int>(),
+                    Z.hd.as<unsigned char>(), op->n, a.t0, a.t1};
+      k_oz_cut_rows<<<(unsigned)op->rg.n_groups, 256, 0, st>>>(c); TTG_COUNT();
+      TTG_LAUNCHED(op);
+      Z.cut = Z.slabs.size() == 2;
+    }
+    k_oz_apply<<<(unsigned)(a.ctas * a.par), kApThreads, kApSmem, st>>>(a); TTG_COUNT();
+    TTG_LAUNCHED(op);
+  }
   return TTG_OK;
 }
 

@@ -229,12 +229,14 @@ struct OzWork {
 // H X in FP64 on the tensor cores (ozgemm.cu): the digits of H on the tiles of
 // UmmaOp, and of the block.
 struct OzRows {
-  DevBuf hd;       // [chunk][7][128 x 16] bf16
+  DevBuf hd;       // [chunk of a slab][7][128 x 16] bf16
   DevBuf he;       // int32 [n_tiles*128]: largest biased exponent of each row
   DevBuf urow;     // int32 [n]: tile * 128 + lane of each row
   DevBuf xd;       // bf16 [n + nproj][groups of 32 states][8][32], the last unused
   DevBuf xe;       // int32 [k]: largest biased exponent of each column
-  bool cut = false;   // hd holds the digits of the current values
+  std::vector<int> slabs;   // first tiles of the slabs, and the number of tiles
+  int64_t most = 0;   // chunks of the largest
+  bool cut = false;   // hd holds the digits of the current values (one slab)
 };
 
 // Work buffers of the Hartree kernel expansion (tensor.cu), grow-only and
