@@ -68,7 +68,7 @@ SCF_SETTINGS = {
 # the 64-atom operator with its 160-column block (profile_workload --workload
 # atoms64 --prec fp32 --degrees 1): bytes / 3,760,928 slots; scaled to the
 # timed operator's slots
-TRAFFIC_PER_SLOT_UMMA = (3.11e9 + 31.32e6) / 3760928
+TRAFFIC_PER_SLOT_UMMA = (2.036e9 + 24.67e6) / 3760928
 MAX_ITER = 60
 MEASURED_PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
 FALLBACK_HBM_GBS = 6800.0
@@ -345,7 +345,7 @@ def run_ours(args, rank, world):
             "metric": METRIC, "value": sec_per_iter, "unit": "s/SCF-iter", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": sec_per_iter * 1e3,
             "higher_is_better": False, "scaling": "weak", "vs_baseline": None,
-            "dtype": "bf16/fp32 filter, fp64 Rayleigh-Ritz (double-fp32 arithmetic), exact-sliced bf16 tensor-core Hartree and density, fp64 grids",
+            "dtype": "bf16/fp32 filter, fp64 Rayleigh-Ritz and Hartree and density on exact-sliced bf16 tensor-core products, fp64 grids",
             "data": "synthetic (seeded atoms)",
             "config": {"workload": f"{WORKLOAD}: full SCF iteration (mixed filter)",
                        "N": n, "states": k, "degree": m, "bf16_degrees": m // 4,

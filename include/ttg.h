@@ -43,7 +43,8 @@ typedef enum {
   TTG_PREC_FP64 = 0,   /* H and the block in FP64, FP64 accumulation */
   TTG_PREC_FP32 = 1,   /* H and the block in FP32, FP32 accumulation */
   TTG_PREC_BF16 = 2,   /* H and the block stored in BF16, FP32 accumulation */
-  TTG_PREC_DF64 = 3    /* FP64 values as pairs of FP32 (~47 bits) on the FP32 pipes */
+  TTG_PREC_DF64 = 3    /* FP64 values as exact digits on the tensor cores, summed in pairs
+                          of FP32, or as pairs of FP32 on the FP32 pipes (~47 bits) */
 } ttg_prec;
 
 /* Precision schedule of one Chebyshev filter call: the first `n_low` degrees
@@ -113,7 +114,8 @@ ttg_status ttg_op_create_tucker(int64_t n, const int64_t* h_row_ptr, const int32
                                 const int32_t* c_col, const double* c_val, const double* d,
                                 const int32_t* tucker_ranks, int32_t max_k, ttg_op** out);
 /* Arithmetic of the H X product inside ttg_rayleigh_ritz / ttg_chfsi_pass:
- * TTG_PREC_DF64 (default: FP64-level accuracy at the FP32 rate) or
+ * TTG_PREC_DF64 (default: FP64-level accuracy, on the tensor cores where the
+ * operator has tcgen05 tiles and its digits fit in memory) or
  * TTG_PREC_FP64 (native FP64, the reference's arithmetic). */
 ttg_status ttg_op_set_rr_precision(ttg_op* op, int32_t prec);
 /* Replaces AX::free_mata_on_device / AX::~AX (eigensolver/MultCuda.cu:673-717). */

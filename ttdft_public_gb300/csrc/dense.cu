@@ -21,9 +21,9 @@
 //                  (main.cc:1239-1272).
 //
 // FP64 throughout: these are the quantities the method keeps in double.  The
-// two N x k GEMMs (the Gram X^T Y and the rotation X Q) read and write FP64
-// and compute in double-FP32 on the FP32 pipe (about 48 bits; FP64 runs at
-// a small fraction of the FP32 rate on this part).
+// two N x k GEMMs here (the Gram X^T Y and the rotation X Q) are the fallback of
+// ozgemm.cu: FP64 in and out, double-FP32 on the FP32 pipe (about 48 bits; FP64
+// runs at a small fraction of the FP32 rate on this part).
 
 #include <algorithm>
 #include <cmath>

@@ -22,7 +22,8 @@
 //                          computeRhoIn (dft/AndersonMixing.cc:267-316).
 //
 // Fields are x-fastest n1 x n2 x n3 arrays in device memory owned by the
-// caller.  The mode products and Gram matrices are one strided-batched GEMM
+// caller.  The mode products and Gram matrices run on the tensor cores
+// (ozgemm.cu) from 1e8 flops on; smaller ones are one strided-batched GEMM
 // kernel (FP64 in and out, double-FP32 arithmetic on the FP32 pipe) with a
 // fixed-order split-K reduction in FP64 (bitwise reproducible).
 

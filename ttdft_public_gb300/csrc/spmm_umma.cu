@@ -61,17 +61,18 @@
 // accumulators meet in shared memory and every CTA finishes its share of the
 // rows.  BF16 degrees keep one CTA a tile: their sums are rounded to 8 bits at
 // every degree, so the order of a sum is part of the result.
-// What bounds it: the round trip of a stage through its barriers (about 3,000
-// clocks, a ring of 4 or 5 stages) and the issue of the MMAs; without any copy
-// the 64-atom FP32 degree takes 5 % less.  HBM's floor is H read once.
+// What bounds it (clock counts of its threads): at 160 states a stage takes 670
+// clocks, in which H streams at 6.9 TB/s over the SMs: HBM, plus the CTAs'
+// uneven ends; at 240 states a column block 820, of which the MMAs need 720.
+// Stages of half the size: 520 instead of 400 us and 1,130 instead of 1,018.
 // One degree, three-term split with a CTA a tile -> now:
 //   64,000 functions, 160 states, FP32: 728 -> 400 us (H's 2.0 GB: 294 us)
 //   the same, BF16: 396 -> 183 us (147 us)
 //   32,768 functions, 1,200 states, FP32: 2,425 -> 1,018 us
 //   1,728 functions, 24 states, FP32 (clusters of 4): 63 (mma.sync) -> 11 us
-// Of these, a stage of several chunks and two terms gave 728 -> 514, the
-// epilogue beside the next item's MMAs 514 -> 430, the elected MMA thread and
-// addresses made before the wait the rest.
+// Of these, a stage of several chunks and two terms gave 728 -> 514; the
+// epilogue beside the next item's MMAs (22 % of the kernel until then), the
+// elected MMA thread and addresses made before the wait the rest.
 // Every wait (mbarrier or the ready count) is bounded; a wait that runs out
 // sets an error word.
 

@@ -377,7 +377,8 @@ ttg_status hartree_error(ttg_op* op);
 #ifdef __CUDACC__
 // Double-FP32 ("df64") arithmetic: a value is an unevaluated sum hi + lo of
 // two floats (about 48 significant bits).  FP64 runs at ~1.25 TFLOP/s on
-// this part and FP32 at ~80, so the FP64 GEMMs run on the FP32 pipe in df64:
+// this part and FP32 at ~80, so the FP64 GEMMs that are too small for the
+// tensor cores (ozgemm.cu), or fall back from them, run on the FP32 pipe in df64:
 // one df64 multiply-add is 11 FP32 instructions (Dekker/Knuth error-free
 // product and sum), about 5x the FP64 rate.  The product's lo x lo term
 // (2^-48 relative) is dropped.

@@ -9,7 +9,7 @@
 
 Builds the workload's operator, uploads a random block and runs `degrees`
 filter degrees per listed precision (one fused SpMM launch each) and, with
---rr, one Rayleigh-Ritz projection (the df64 SpMM, Gram and eigensolve).  Few
+--rr, one Rayleigh-Ritz projection (H X, Gram and eigensolve).  Few
 launches and no timing loop, so that an ncu capture of it stays small.  With
 --scf N it runs N iterations of the SCF loop instead (for launch lists),
 with --hartree N N evaluations of the standalone Hartree contraction."""
