@@ -46,7 +46,7 @@
 //    have an issuing thread (warps 1 and 3): while one half waits for its eight
 //    epilogue warps to empty its accumulators, the other's MMAs have the tensor
 //    pipe, and the half that is ahead by then stays so.  One thread for both
-//    spent a third of its time in the commits (330 cycles each).  They are
+//    spent a third of its time in the commits (330 cycles each then).  They are
 //    elected (elect_one): the MMAs of a 512,000 x 1,200 orthonormalisation
 //    took 35.6 ms under `lane == 0`, 33.1 now.  A chunk costs 36 KB of copies
 //    for 2 x 336 MMA cycles.

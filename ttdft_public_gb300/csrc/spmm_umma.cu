@@ -14,9 +14,9 @@
 // is left below 2^-22 |v| (and below 2^-31 of the row's or 2^-39 of the
 // column's largest value, where v1 runs out of exponents).  The product is
 // accumulated in FP32 from v0w0, v0w1 and v1w0; v1w1 is below 2^-22 |v w|.
-// An accumulation step of the tensor core truncates, which is where the error
-// of a degree comes from: three steps per 16 slots instead of the six of a
-// three-term BF16 split.  Relative error of 8 degrees against FP64, before and
+// An accumulation step of the tensor core truncates, the larger part of a
+// degree's error: three steps per 16 slots instead of the six of a three-term
+// BF16 split.  Relative error of 8 degrees against FP64, before and
 // now: 1.3e-5 and 3.7e-6 (1,728 functions, 24 states), 1.8e-5 and 9.7e-6 (8,000,
 // 160), 2.2e-5 and 1.9e-5 (64,000, 400).
 //  - Block columns: the largest |Y| of each column comes from the epilogue of
@@ -38,27 +38,27 @@
 //    many tiles), in the MN-major operand layout with the 128-byte swizzle:
 //    8 lanes read one whole 128-byte piece of a row, so one instruction moves
 //    four rows.
-// A stage is SC = 2 chunks (FP32) or 4 (BF16): the commit of a stage's MMAs
-// costs the issuing thread about 330 clocks whatever it commits, and the
-// round trip of a stage through its barriers is paid once for all of it.
-// Warp roles (one CTA per SM):
-//  - warp 0, one thread: the H copies, up to a whole ring ahead;
-//  - warps 3-12: the row gathers, whole chunks in turn, two chunks of each warp
-//    in flight; a warp waits for its own copies and fences them for the async
-//    proxy before it arrives;
-//  - warp 2, one thread: waits for each stage's "full" mbarrier in order and
+// A stage is SC = 2 chunks (FP32) or 4 (BF16): its commit and the round trip
+// through its barriers are paid once for all of it.
+// Persistent CTAs, one per SM, each with a list of tiles (each_item).  Roles:
+//  - warp 4, one thread: the H copies, up to a whole ring ahead;
+//  - warps 7-16: the row gathers, whole chunks in turn; a warp waits for its
+//    own copies and fences them for the async proxy before it arrives;
+//  - warp 6, one thread: waits for each stage's "full" mbarrier in order and
 //    publishes the count of ready stages in shared memory;
-//  - warp 1, one thread: three MMAs (one for BF16) a chunk and one commit (to
-//    the stage's "done" mbarrier) per stage.  It never waits on an mbarrier
-//    itself: such a wait queues behind its outstanding MMAs (about 0.1 us).
-// After the last stage warps 0-3 (one per 32 TMEM lanes) read the accumulator
-// from tensor memory and apply the recurrence in FP32.
-// Blocks wider than one MMA (N <= 256) run as column blocks in one launch, the
-// tiles of one block after those of the one before, so that only the last
-// block's tail leaves SMs idle.
+//  - warp 5, one elected thread: three MMAs (one for BF16) a chunk and one
+//    commit (to the stage's "done" mbarrier) per stage.  Between the stages of
+//    an item it waits on no mbarrier: such a wait queues behind its
+//    outstanding MMAs (about 0.1 us);
+//  - warps 0-3 (one per 32 TMEM lanes): read an item's accumulator from tensor
+//    memory and apply the recurrence in FP32, while the next item's MMAs fill
+//    the other accumulator.
+// Blocks wider than one MMA (N <= 256) are column blocks of one launch, a CTA's
+// tiles of one block after those of the one before, with its list exchanged for
+// one from the other end of the order of loads in every second one.
 // Few tiles (FP32): where the tiles would leave half of the SMs without work,
-// a cluster of 2, 4 or 8 CTAs shares a tile, each a part of its chunks; the
-// accumulators meet in shared memory and every CTA finishes its share of the
+// a cluster of 2, 4 or 8 CTAs (as many as are resident at once) shares a tile,
+// each a part of its chunks; the accumulators meet in shared memory and every CTA finishes its share of the
 // rows.  BF16 degrees keep one CTA a tile: their sums are rounded to 8 bits at
 // every degree, so the order of a sum is part of the result.
 // What bounds it (clock counts of its threads): at 160 states a stage takes 670

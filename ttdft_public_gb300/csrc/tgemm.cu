@@ -39,7 +39,7 @@
 //    128 columns for p = 0, 1, 2, three MMAs a chunk instead of eight.
 //  - Two accumulator buffers (2 x 256 tensor-memory columns), each with an
 //    issuing thread (warps 1 and 3) that takes every other group: one issues
-//    while the other is held up in its commits (330 cycles each).
+//    while the other is held up in its commits.  They are elected (elect_one).
 //  - warp 0, one thread: the copies (TMA); warp 2, one thread: waits for a
 //    chunk's copies in order and publishes the count;
 //  - warps 4-19 (four per 32 TMEM lanes, 16 columns each): combine the levels
