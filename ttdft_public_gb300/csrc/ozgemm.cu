@@ -1317,7 +1317,12 @@ __global__ void __launch_bounds__(kApThreads, 1) k_oz_apply(const OzApply a) {
             return false;
           }
           if (!on) {
-            bar_arrive(&empty[s]);
+            // this thread's MMAs of the block before may still run: the commit
+            // frees the stage after them, so that `empty` completes in the order
+            // of the chunks, which the gathering warps' parity waits need
+            asm volatile(
+                "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                ::"r"(su32(&empty[s])) : "memory");
             continue;
           }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
