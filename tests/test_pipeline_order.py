@@ -3,9 +3,12 @@ role for any time: a ring of stages, warps that fill them by turns, a thread tha
 come later but in order per issuing thread.
 
 A parity wait sees only whether the phase before the running one had that parity: a waiter more than one phase off,
-on either side, reads the wrong answer.  The rules that keep the waiters within a phase:
+on either side, reads the wrong answer.  Two rules keep the waiters within a phase:
  - k_oz_apply (csrc/ozgemm.cu): `empty` has to complete in the order of the chunks.  The issuing thread of a group
-   without states frees a stage by a commit, behind its own earlier MMAs, and not by an arrival of its own."""
+   without states frees a stage by a commit, behind its own earlier MMAs, and not by an arrival of its own.
+ - k_cheb_umma (csrc/spmm_umma.cu): a stage of a tile's last chunks has slots without one.  Their warps arrive for
+   them as for the others; where the copying thread does so in their place, the MMAs can run past a warp that is late,
+   and the phase that it waits for is then read as not yet there."""
 import random
 
 import pytest
@@ -98,6 +101,46 @@ def apply_pipeline(rng, blocks, chunks, commit):
     return run(agents, rng) and not early
 
 
+def filter_pipeline(rng, items, stages, sc, warps, own):
+    """k_cheb_umma on one CTA: tiles of items[i] chunks, stages of sc chunks."""
+    full, done = [Barrier(1 + sc) for _ in range(stages)], [Barrier(1) for _ in range(stages)]
+    slots = []                                            # chunk or no chunk, whole stages an item
+    for n in items:
+        slots += [True] * n + [False] * (-n % sc)
+    early, queue, last = [], [], {"ended": False}
+
+    def copies():
+        for g in range(len(slots) // sc):
+            if g >= stages:
+                yield lambda s=g % stages, p=g // stages - 1: done[s].test(p)
+            if not own:
+                for j in range(sc):
+                    if not slots[g * sc + j]:
+                        full[g % stages].arrive()
+            full[g % stages].arrive()
+            yield
+
+    def gather(w):
+        for t in range(w, len(slots), warps):
+            g = t // sc
+            if g >= stages:
+                yield lambda s=g % stages, p=g // stages - 1: done[s].test(p)
+            if done[g % stages].phases < g // stages:
+                early.append(t)
+            yield
+            if slots[t] or own:
+                full[g % stages].arrive()
+
+    def mma():
+        for g in range(len(slots) // sc):
+            yield lambda s=g % stages, p=g // stages: full[s].test(p)
+            queue.append(done[g % stages])
+        last["ended"] = True
+
+    agents = [copies(), mma(), completions(queue, last)] + [gather(w) for w in range(warps)]
+    return run(agents, rng) and not early
+
+
 BLOCKS = [[True, False], [True, True, False], [False, True, False, True]]
 
 
@@ -108,3 +151,16 @@ def test_absent_group_frees_stages_in_order(blocks):
 
 def test_absent_group_without_a_commit_is_read_too_early():
     assert not all(apply_pipeline(random.Random(i), b, 23, commit=False) for b in BLOCKS for i in range(150))
+
+
+# FP32 (two chunks a stage) and BF16 (four) rings; tiles of nine chunks give a warp two empty slots in a row
+RINGS = [(5, 2, 10, [9] * 12), (4, 2, 8, [7, 7, 1, 15, 7, 7, 7, 30]), (5, 4, 10, [9, 5, 17, 1, 2, 3, 13, 13, 13])]
+
+
+@pytest.mark.parametrize("stages, sc, warps, items", RINGS)
+def test_empty_slots_are_filled_by_their_warps(stages, sc, warps, items):
+    assert all(filter_pipeline(random.Random(i), items, stages, sc, warps, own=True) for i in range(150))
+
+
+def test_empty_slots_filled_by_the_copies_can_stop_a_late_warp():
+    assert not all(filter_pipeline(random.Random(i), r[3], *r[:3], own=False) for r in RINGS for i in range(150))

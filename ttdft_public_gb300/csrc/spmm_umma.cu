@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(kThreads)
   // those the H blocks
   unsigned char* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
   // full[s]: the H copy by bytes and an arrival each from the H thread and the
-  // warps that gather the stage's chunks; done[s]: its MMAs have read it
+  // warps of the stage's slots; done[s]: its MMAs have read it
   __shared__ __align__(8) uint64_t full[kMaxStages], done[kMaxStages];
   // accumulators: an item's MMAs are done, its sums have been read
   __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2];
@@ -367,9 +367,6 @@ __global__ void __launch_bounds__(kThreads)
           if (lap > 0) ok &= mbar_wait(&done[s], (lap - 1) & 1);
           const uint32_t fb = smem_u32(&full[s]);
           const int nc = min(SC, it.nch - c);
-          // a last stage of fewer chunks: arrive for the missing gathers
-          for (int j = nc; j < SC; ++j)
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(fb) : "memory");
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb),
                        "r"(nc * HC) : "memory");
           asm volatile(
@@ -446,9 +443,14 @@ __global__ void __launch_bounds__(kThreads)
               __syncwarp();
             }
           }
-          // a slot without a chunk is waited for as well: a warp's wait, a
-          // ring earlier at most, is what keeps the parity of this one unambiguous
-          if (c >= it.nch) continue;
+          // a slot without a chunk (an item's last stage) is waited for and
+          // arrived for as well: a warp's wait, a ring earlier at most, and the
+          // MMAs' wait for the warp are what keep the parity unambiguous
+          if (c >= it.nch) {
+            if (lane == 0)
+              asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[s])) : "memory");
+            continue;
+          }
 #pragma unroll
           for (int rq = 0; rq < 4; ++rq) {
             const uint32_t drow = sb + (rq & 1 ? sw1 : sw0) + (rq >> 1) * 1024;
