@@ -124,7 +124,11 @@ ttg_status ttg_op_info(const ttg_op* op, ttg_op_info_t* info);
 /* The op's cudaStream_t, as an opaque pointer, for callers that overlap work. */
 void* ttg_op_stream(ttg_op* op);
 /* Waits for the op's stream; TTG_TIMEOUT if a bounded wait inside a
- * tensor-memory filter kernel ran out since the last check. */
+ * tensor-memory kernel (filter degree, FP64 GEMM, H X, Hartree or density
+ * product) ran out since the last check.  Entry points that hand results to
+ * the host check the FP64 kernels themselves; those that leave their results
+ * on the device (ttg_cheb_filter, ttg_op_update_potential_device,
+ * ttg_hartree_device, ttg_density_device) report here. */
 ttg_status ttg_op_sync(ttg_op* op);
 /* Device-side timing on the op's stream (slot 0..15). */
 ttg_status ttg_op_record(ttg_op* op, int32_t slot);

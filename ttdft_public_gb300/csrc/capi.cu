@@ -32,11 +32,12 @@ size_t block_bytes(const ttg_op* op, size_t elem) {
   return (size_t)(op->n + op->nproj) * (size_t)op->ld * elem;
 }
 
+// Waits for the stream; the FP64 tensor-core kernels' error comes before the
+// status that their results led to.
 ttg_status read_status(ttg_op* op, int* host_status) {
   TTG_CUDA_TRY(cudaMemcpyAsync(host_status, op->status.p, sizeof(int), cudaMemcpyDeviceToHost,
                                op->stream));
-  TTG_CUDA_TRY(cudaStreamSynchronize(op->stream));
-  return TTG_OK;
+  return ozgemm_error(op);
 }
 
 ttg_status check_block(const ttg_op* op, const ttg_block* b) {
@@ -219,6 +220,10 @@ ttg_status ttg_op_create_tucker(int64_t n, const int64_t* h_row_ptr, const int32
   if ((s = ensure(op->scal, (kScalJacobi + 4 * (kmax + 2) + kmax) * 8, op)) != TTG_OK)
     return fail(s);
   if ((s = ensure(op->status, 64, op)) != TTG_OK) return fail(s);
+  if (cudaHostAlloc(&op->oz.word, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) !=
+      cudaSuccess)
+    return fail(TTG_OOM);
+  *op->oz.word = 0;
   if ((s = ensure(op->w64, block_bytes(op, 8), op)) != TTG_OK) return fail(s);
   if (cudaMemsetAsync(op->status.p, 0, 64, op->stream) != cudaSuccess) return fail(TTG_CUDA_ERR);
   if (cudaStreamSynchronize(op->stream) != cudaSuccess) return fail(TTG_CUDA_ERR);
@@ -313,9 +318,8 @@ ttg_status ttg_op_set_rr_precision(ttg_op* op, int32_t prec) {
 
 ttg_status ttg_op_sync(ttg_op* op) {
   if (!op) return TTG_BAD_ARG;
-  TTG_CUDA_TRY(cudaStreamSynchronize(op->stream));
+  TTG_TRY(ozgemm_error(op));             // waits for the stream
   TTG_TRY(umma_check_error(op));
-  TTG_TRY(ozgemm_error(op));
   return hartree_error(op);
 }
 
@@ -509,7 +513,7 @@ ttg_status ttg_gram(ttg_op* op, const ttg_block* X, const ttg_block* Y, double* 
   if (s_host) {
     TTG_CUDA_TRY(cudaMemcpyAsync(s_host, op->kk0.p, (size_t)k * k * 8, cudaMemcpyDeviceToHost,
                                  op->stream));
-    TTG_CUDA_TRY(cudaStreamSynchronize(op->stream));
+    return ozgemm_error(op);
   }
   return TTG_OK;
 }
@@ -537,7 +541,7 @@ ttg_status chol_qr_step(ttg_op* op, ttg_block* X, bool shifted) {
     TTG_TRY(unit_scale_shift(op, S, d, k, 1e-8, bad));
     int nbad = 0;
     TTG_CUDA_TRY(cudaMemcpyAsync(&nbad, bad, sizeof(int), cudaMemcpyDeviceToHost, op->stream));
-    TTG_CUDA_TRY(cudaStreamSynchronize(op->stream));
+    TTG_TRY(ozgemm_error(op));
     if (nbad) {
       fprintf(stderr, "ttg: Cholesky-QR: %d of %d columns have a zero or non-finite norm\n",
               nbad, k);
@@ -616,8 +620,7 @@ ttg_status ttg_syev(ttg_op* op, int32_t k, const double* a_host, double* w_host,
   if (v_host)
     TTG_CUDA_TRY(cudaMemcpyAsync(v_host, op->kk1.p, (size_t)k * k * 8, cudaMemcpyDeviceToHost,
                                  op->stream));
-  TTG_CUDA_TRY(cudaStreamSynchronize(op->stream));
-  return TTG_OK;
+  return ozgemm_error(op);
 }
 
 ttg_status ttg_rayleigh_ritz(ttg_op* op, ttg_block* X, int32_t rotate, double* w_host,
@@ -655,8 +658,7 @@ ttg_status ttg_rayleigh_ritz(ttg_op* op, ttg_block* X, int32_t rotate, double* w
   if (q_host)
     TTG_CUDA_TRY(cudaMemcpyAsync(q_host, op->kk1.p, (size_t)k * k * 8, cudaMemcpyDeviceToHost,
                                  op->stream));
-  if (w_host || q_host) TTG_CUDA_TRY(cudaStreamSynchronize(op->stream));
-  return TTG_OK;
+  return w_host || q_host ? ozgemm_error(op) : TTG_OK;
 }
 
 ttg_status ttg_rotate(ttg_op* op, ttg_block* X, const double* q_host) {
@@ -668,9 +670,7 @@ ttg_status ttg_rotate(ttg_op* op, ttg_block* X, const double* q_host) {
   TTG_TRY(product_fp64(op, X->x.as<double>(), op->kk1.as<double>(), op->w64.as<double>(), k, 0,
                        false));
   std::swap(op->w64.p, X->x.p);
-  TTG_CUDA_TRY(cudaStreamSynchronize(op->stream));
-  TTG_TRY(ozgemm_error(op));
-  return TTG_OK;
+  return ozgemm_error(op);
 }
 
 ttg_status ttg_lanczos_bounds(ttg_op* op, const double* v0_host, int32_t max_iter,

@@ -535,7 +535,6 @@ ttg_status ttg_op_update_potential(ttg_op* op, const int32_t* pot_ranks, const d
   TTG_CUDA_TRY(cudaMemcpyAsync(w + L.off_z, hz.data(), hz.size() * 8, cudaMemcpyHostToDevice, st));
   TTG_CUDA_TRY(cudaMemcpyAsync(w + L.off_g, G, ncore * 8, cudaMemcpyHostToDevice, st));
   TTG_TRY(update_from_tables(op, L));
-  TTG_CUDA_TRY(cudaStreamSynchronize(st));
   return ozgemm_error(op);
 }
 

@@ -747,6 +747,26 @@ ttg_status row_exps(cudaStream_t st, const OzSlices& S, int nz, const int* kexp,
   return TTG_OK;
 }
 
+ttg_status error_word(cudaStream_t st, OzWork& ws, int** err) {
+  if (!ws.word && !ws.err.p) {
+    TTG_TRY(ws.err.alloc(sizeof(int)));
+    TTG_CUDA_TRY(cudaMemsetAsync(ws.err.p, 0, sizeof(int), st));
+  }
+  *err = ws.word ? ws.word : ws.err.as<int>();
+  return TTG_OK;
+}
+
+// TTG_FAKE_TIMEOUT=1 (tests of the callers): the error word as a kernel whose
+// wait ran out leaves it.
+__global__ void k_oz_fake_timeout(int* err) { atomicExch(err, 1); }
+
+ttg_status fake_timeout(cudaStream_t st, int* err) {
+  if (!getenv("TTG_FAKE_TIMEOUT")) return TTG_OK;
+  k_oz_fake_timeout<<<1, 1, 0, st>>>(err);
+  TTG_CUDA_TRY(cudaGetLastError());
+  return TTG_OK;
+}
+
 ttg_status slice(cudaStream_t st, const OzSlices& S, int nz, int64_t r0, int64_t rpad, int64_t k0,
                  int64_t chunks, const int* kexp, int ksign, unsigned long long* diag = nullptr) {
   if (chunks <= 0) return TTG_OK;
@@ -817,13 +837,10 @@ ttg_status ozgemm(cudaStream_t st, OzWork& ws, DevBuf& partial_buf, const OzOper
     diag = ws.diag.as<unsigned long long>();
     TTG_CUDA_TRY(cudaMemsetAsync(diag, 0, (size_t)M * 8, st));
   }
-  if (!ws.err.p) {
-    TTG_TRY(ws.err.alloc(sizeof(int)));
-    TTG_CUDA_TRY(cudaMemsetAsync(ws.err.p, 0, sizeof(int), st));
-  }
+  int* err = nullptr;
+  TTG_TRY(error_word(st, ws, &err));
   int* ea = ws.exp.as<int>();
   int* eb = same ? ea : ea + M;
-  int* err = ws.err.as<int>();
   // K scales: the row scales of kscale_of (a view whose rows are the K
   // index), A scaled by 2^-f_k and B by 2^f_k; the buffer is padded with zeros
   // to whole chunks
@@ -931,16 +948,18 @@ ttg_status ozgemm(cudaStream_t st, OzWork& ws, DevBuf& partial_buf, const OzOper
         out.p, (int)nsplit, (int)M, (int)N, sym ? 1 : 0, diag, ea, C, c.rs, c.cs); TTG_COUNT();
     TTG_CUDA_TRY(cudaGetLastError());
   }
-  return TTG_OK;
+  return fake_timeout(st, err);
 }
 
 ttg_status ozgemm_error(cudaStream_t st, OzWork& ws) {
-  if (!ws.err.p) return TTG_OK;
   int e = 0;
-  TTG_CUDA_TRY(cudaMemcpyAsync(&e, ws.err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+  if (ws.err.p)
+    TTG_CUDA_TRY(cudaMemcpyAsync(&e, ws.err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   TTG_CUDA_TRY(cudaStreamSynchronize(st));
+  if (ws.word) e = *static_cast<volatile int*>(ws.word);
   if (e) {
-    TTG_CUDA_TRY(cudaMemsetAsync(ws.err.p, 0, sizeof(int), st));
+    if (ws.word) *static_cast<volatile int*>(ws.word) = 0;
+    else TTG_CUDA_TRY(cudaMemsetAsync(ws.err.p, 0, sizeof(int), st));
     fprintf(stderr, "ttg: FP64 tensor-core GEMM: %s\n",
             e == 3 ? "a copy barrier out of phase" : "a bounded wait ran out");
     return e == 3 ? TTG_CUDA_ERR : TTG_TIMEOUT;
@@ -1557,10 +1576,8 @@ ttg_status launch_oz_apply(ttg_op* op, const double* src, double* dst, int k) {
     return TTG_OOM;
   }
   TTG_TRY(grow(Z.xe, (size_t)op->ld * sizeof(int)));
-  if (!op->oz.err.p) {
-    TTG_TRY(op->oz.err.alloc(sizeof(int)));
-    TTG_CUDA_TRY(cudaMemsetAsync(op->oz.err.p, 0, sizeof(int), st));
-  }
+  int* err = nullptr;
+  TTG_TRY(error_word(st, op->oz, &err));
   if (!Z.urow.p) {
     TTG_TRY(grow(Z.urow, (size_t)op->n * sizeof(int)));
     k_oz_tile_rows<<<(unsigned)((trows + 255) / 256), 256, 0, st>>>(U.rowmap.as<int>(), trows,
@@ -1602,7 +1619,7 @@ ttg_status launch_oz_apply(ttg_op* op, const double* src, double* dst, int k) {
   a.dst = dst;
   a.ld = op->ld;
   a.k = k;
-  a.err = op->oz.err.as<int>();
+  a.err = err;
   for (size_t i = 1; i < Z.slabs.size(); ++i) {
     a.t0 = Z.slabs[i - 1];
     a.t1 = Z.slabs[i];
@@ -1620,7 +1637,7 @@ ttg_status launch_oz_apply(ttg_op* op, const double* src, double* dst, int k) {
     k_oz_apply<<<(unsigned)(a.ctas * a.par), kApThreads, kApSmem, st>>>(a); TTG_COUNT();
     TTG_LAUNCHED(op);
   }
-  return TTG_OK;
+  return fake_timeout(st, err);
 }
 
 }  // namespace ttg

@@ -657,7 +657,7 @@ ttg_status ttg_tucker_sthosvd(ttg_op* op, const double* t_dev, const int32_t* di
     TTG_CUDA_TRY(cudaMemcpyAsync(w.data(), wdev, rcap * 8, cudaMemcpyDeviceToHost, st));
     TTG_CUDA_TRY(cudaMemcpyAsync(&w[rcap], tdev, 8, cudaMemcpyDeviceToHost, st));
     TTG_CUDA_TRY(cudaMemcpyAsync(&stat, op->status.p, 4, cudaMemcpyDeviceToHost, st));
-    TTG_CUDA_TRY(cudaStreamSynchronize(st));
+    TTG_TRY(ozgemm_error(op));
     if (stat) return TTG_NOT_CONVERGED;
     const double trace = w[rcap];
     // the first trace is ||T||^2: threshold eps^2 ||T||^2 / 3 per mode
@@ -679,7 +679,6 @@ ttg_status ttg_tucker_sthosvd(ttg_op* op, const double* t_dev, const int32_t* di
     cur_t = to;
     cur[d] = r;
   }
-  TTG_CUDA_TRY(cudaStreamSynchronize(st));
   return ozgemm_error(op);
 }
 
@@ -722,7 +721,6 @@ ttg_status ttg_tucker_reconstruct(const double* core_dev, const int32_t* ranks,
     }
     if (s != TTG_OK) return s;
   }
-  TTG_CUDA_TRY(cudaStreamSynchronize(S.s));
   return ozgemm_error(S.s, w);
 }
 

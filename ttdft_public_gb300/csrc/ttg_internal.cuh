@@ -223,7 +223,15 @@ struct OzWork {
   DevBuf exp;      // row scales of the operands
   DevBuf kexp;     // K scales (padded to whole chunks)
   DevBuf diag;     // sums of d3^2 of the rows of X^T X
-  DevBuf err;      // error word
+  DevBuf err;      // error word, where there is no `word`
+  // An operator's error word: pinned host memory that the kernels write to
+  // where a wait runs out, so that whoever has waited for the stream reads it
+  // without a copy of its own.
+  int* word = nullptr;
+  OzWork() = default;
+  OzWork(const OzWork&) = delete;
+  OzWork& operator=(const OzWork&) = delete;
+  ~OzWork() { if (word) cudaFreeHost(word); }
 };
 
 // H X in FP64 on the tensor cores (ozgemm.cu): the digits of H on the tiles of
@@ -473,7 +481,9 @@ ttg_status ozgemm(cudaStream_t st, OzWork& w, DevBuf& partial, const OzOperand& 
 ttg_status ozgemm(ttg_op* op, const OzOperand& A, const OzOperand& B, double* C, OzLayout c,
                   bool sym, bool b_lower = false, const OzOperand* kscale_of = nullptr,
                   const OzRagged* ragged = nullptr);
-// Reads and clears the tensor-core GEMM's error word (synchronises).
+// Waits for the stream, reads and clears the tensor-core GEMM's error word.
+// Entry points that hand results to the host return this in the place of a
+// plain wait.
 ttg_status ozgemm_error(cudaStream_t st, OzWork& w);
 ttg_status ozgemm_error(ttg_op* op);
 
