@@ -236,8 +236,11 @@ __global__ void __launch_bounds__(256) k_pair_width(const UpdateArgs a, int* __r
   }
 }
 
-// Most values of a slab (8 bytes each).
-constexpr int64_t kSlabValues = (int64_t)1 << 28;
+// Most values of a slab (8 bytes each); TTG_UPDATE_SLAB_VALUES sets another limit.
+int64_t slab_values() {
+  const char* e = getenv("TTG_UPDATE_SLAB_VALUES");
+  return e ? std::max<int64_t>(atoll(e), 1) : (int64_t)1 << 28;
+}
 
 ttg_status upload_vec(cudaStream_t st, DevBuf& b, const void* p, size_t bytes) {
   TTG_TRY(b.alloc(std::max<size_t>(bytes, 16)));
@@ -277,7 +280,7 @@ ttg_status make_plan(ttg_op* op, const UpdateArgs& a, int64_t nxp, int64_t nyp, 
     cols[d] = ((int)zlist.size() + 1) / 2 * 2;
   }
   L.nq = (int)zlist.size();
-  const int64_t max_rows = ozgemm_ragged_rows(rc, L.nq);
+  const int64_t max_rows = L.max_rows = ozgemm_ragged_rows(rc, L.nq), max_values = slab_values();
   std::vector<int> pairs, where(nxp * nyp, -1), first, ld;
   std::vector<int64_t> base;
   for (int y0 = 0; y0 < ry;) {
@@ -292,12 +295,12 @@ ttg_status make_plan(ttg_op* op, const UpdateArgs& a, int64_t nxp, int64_t nyp, 
           v += cols[width[i]];
         }
       v += 128 * (int64_t)cols[bz];          // a tile's columns are its widest pair's
-      if (cnt + c > max_rows || vals + v > kSlabValues) break;
+      if (cnt + c > max_rows || vals + v > max_values) break;
       cnt += c;
       vals += v;
     }
-    if (y1 == y0) {
-      L = UpdatePlan();
+    if (y1 == y0) {                          // no plan for these
+      L.slabs.clear();
       L.made = true;
       return TTG_OK;
     }
@@ -427,21 +430,24 @@ ttg_status update_from_tables(ttg_op* op, const UpdateLayout& L) {
   const int nxg = (rx + 7) / 8;
   UpdatePlan& plan = P.plan;
   const bool oz = ozgemm_supported(g1, p1);
-  // the plan's slabs hold for the rank it was made for and smaller ones
-  for (const UpdatePlan::Slab& sl : plan.slabs)
-    if (sl.pairs > ozgemm_ragged_rows(rc, plan.nq)) plan.made = false;
+  // the plan's slabs hold for the rank it was made for and smaller ones; a rank
+  // without a plan says nothing about smaller ones
+  const int64_t max_rows = ozgemm_ragged_rows(rc, plan.nq);
+  int64_t most = 0;                            // pairs of a slab
+  for (const UpdatePlan::Slab& sl : plan.slabs) most = std::max<int64_t>(most, sl.pairs);
+  if (most > max_rows || (plan.slabs.empty() && max_rows > plan.max_rows)) plan.made = false;
   if (oz && !plan.made) {
     const ttg_status ps = make_plan(op, a, nxp, nyp, rc);
-    if (ps == TTG_OOM) {
-      plan = UpdatePlan();
-      plan.made = true;
-    } else if (ps != TTG_OK) {
-      return ps;
-    }
+    if (ps == TTG_OOM) plan = UpdatePlan();    // this time without one
+    else if (ps != TTG_OK) return ps;
+    most = 0;
+    for (const UpdatePlan::Slab& sl : plan.slabs) most = std::max<int64_t>(most, sl.pairs);
   }
+  // all workspaces before the first new value: H is then updated as a whole
   bool ragged = oz && !plan.slabs.empty();
   if (ragged && P.values.bytes < (size_t)plan.out_max * 8 && P.values.alloc(plan.out_max * 8) != TTG_OK)
     ragged = false;
+  if (ragged && ozgemm_reserve(op, most, plan.nq, rc) != TTG_OK) ragged = false;
   if (ragged) {
     a.G = P.values.as<double>();
     a.where = plan.where.as<int>();
@@ -456,13 +462,7 @@ ttg_status update_from_tables(ttg_op* op, const UpdateLayout& L) {
       t2.idx = plan.pairs.as<int>() + sl.pair0;
       const OzRagged R{plan.first.as<int>() + sl.tile0 + i, plan.base.as<int64_t>() + sl.tile0,
                        plan.ld.as<int>() + sl.tile0, sl.items};
-      const ttg_status gs = ozgemm(op, t2, pz, P.values.as<double>(), OzLayout{0, 1}, false, false,
-                                   nullptr, &R);
-      if (gs == TTG_OOM && i == 0) {
-        ragged = false;
-        break;
-      }
-      if (gs != TTG_OK) return gs;
+      TTG_TRY(ozgemm(op, t2, pz, P.values.as<double>(), OzLayout{0, 1}, false, false, nullptr, &R));
       k_update_values<<<(unsigned)((int64_t)(sl.y1 - sl.y0) * nxg * rz), 256, 0, st>>>(a); TTG_COUNT();
       TTG_LAUNCHED(op);
     }

@@ -787,6 +787,16 @@ int64_t ozgemm_ragged_rows(int64_t K, int64_t N) {
   return std::max<int64_t>(0, (kPlaneBudget - rup(N, kRowPad) * row) / row / kRowPad * kRowPad);
 }
 
+ttg_status ozgemm_reserve(ttg_op* op, int64_t M, int64_t N, int64_t K) {
+  OzWork& w = op->oz;
+  const int64_t row = (K + OZ_K - 1) / OZ_K * kDigits * 32;
+  const size_t planes = (size_t)((rup(M, kRowPad) + rup(N, kRowPad)) * row);
+  const size_t exps = (size_t)(M + N) * sizeof(int);
+  if (w.planes.bytes < planes) TTG_TRY(w.planes.alloc(planes));
+  if (w.exp.bytes < exps) TTG_TRY(w.exp.alloc(exps));
+  return TTG_OK;
+}
+
 bool ozgemm_supported(const OzOperand& A, const OzOperand& B) {
   if (getenv("TTG_DISABLE_OZGEMM")) return false;
   return A.p && B.p && A.rows > 0 && B.rows > 0 && A.kext > 0 && A.kext == B.kext &&

@@ -33,6 +33,9 @@ namespace ttg {
 ttg_status DevBuf::alloc(size_t n) {
   release();
   if (n == 0) return TTG_OK;
+  // TTG_ALLOC_LIMIT (tests of what a call does without room): larger ones fail
+  const char* limit = getenv("TTG_ALLOC_LIMIT");
+  if (limit && n > (size_t)atoll(limit)) return TTG_OOM;
   cudaError_t e = cudaMalloc(&p, n);
   if (e != cudaSuccess) {
     p = nullptr;

@@ -165,7 +165,8 @@ struct UmmaOp {
 // coordinate, and within a slab its (y, x) index pairs by falling half-width in
 // z, in tiles of 128.
 struct UpdatePlan {
-  bool made = false;
+  bool made = false;          // for slabs of up to max_rows pairs; without slabs
+  int64_t max_rows = 0;       // where the pairs of one y are more
   int nq = 0;                 // z pairs |dz| <= bw in the order of |dz|
   struct Slab {
     int y0, y1;
@@ -462,6 +463,8 @@ struct OzRagged {
 };
 // The most rows of A, of K values, that a ragged product takes with N rows of B.
 int64_t ozgemm_ragged_rows(int64_t K, int64_t N);
+// Room for ragged products of up to M rows of A: they return no TTG_OOM then.
+ttg_status ozgemm_reserve(ttg_op* op, int64_t M, int64_t N, int64_t K);
 // Whether ozgemm takes these operands (sizes; off with TTG_DISABLE_OZGEMM);
 // callers fall back to the double-FP32 CUDA-core GEMMs.
 bool ozgemm_supported(const OzOperand& A, const OzOperand& B);
