@@ -44,6 +44,13 @@ ttg_status grow(DevBuf& b, size_t bytes) {
   return b.alloc(bytes);
 }
 
+// Room for the largest of the products that share `planes`, made before the
+// first of them; without it each makes what it can (tgemm).
+void grow_planes(DevBuf& planes, std::initializer_list<int64_t> bytes) {
+  const int64_t need = std::max(bytes);
+  if (planes.bytes < (size_t)need) planes.alloc(need);
+}
+
 struct Scratch {
   std::vector<void*> ptrs;
   ~Scratch() {
@@ -297,9 +304,9 @@ ttg_status hartree_tc(cudaStream_t st, HartreeWork& w, const HartreeIn& in, doub
   const TOperand A3{w.q.as<float>(), qrows, kt, kt, 0, 0, am_q};
   const TOperand B3{w.F[2].as<float>(), nz, kt, kt, 0, 0, am_f[2]};
   const int kg1 = (rx + 15) / 16, kg2 = (ry + 15) / 16, kg3 = (int)(ktt / 16);
-  TTG_TRY(grow(w.planes, std::max({tgemm_plane_bytes(TG_STORE_F32, A1, B1, K, 1, kg1),
-                                   tgemm_plane_bytes(TG_STORE_F32, A2, B2, K, 1, kg2),
-                                   tgemm_plane_bytes(TG_SUM_F64, A3, B3, 1, K, kg3)})));
+  grow_planes(w.planes, {tgemm_plane_bytes(TG_STORE_F32, A1, B1, K, 1, kg1),
+                         tgemm_plane_bytes(TG_STORE_F32, A2, B2, K, 1, kg2),
+                         tgemm_plane_bytes(TG_SUM_F64, A3, B3, 1, K, kg3)});
   // 1) P_t[(i, c)][b] = sum_a G[(b, c)][a] Fx_t[i][a]      rows (b, c) x cols i, batch t
   TOut o1{w.p2.p, ry, 1, ryp, (int64_t)rz * ryp, (int64_t)nx * rz * ryp};
   o1.omax = am_p;
@@ -403,9 +410,9 @@ ttg_status density_tc(ttg_op* op, const ttg_block* X, const double* occ, int rx,
     const TOperand A3{D.p2.as<float>(), (int64_t)nx * ny, rz, rzp, sc, (int64_t)ny * nx * rzp, am_2};
     const TOperand B3{D.uf[2].as<float>(), nz, rz, rzp, 0, 0, dm + 2};
     const int kg1 = (rx + 15) / 16, kg2 = (ry + 15) / 16, kg3 = (rz + 15) / 16;
-    TTG_TRY(grow(D.planes, std::max({tgemm_plane_bytes(TG_STORE_F32, A1, B1, sc, 1, kg1),
-                                     tgemm_plane_bytes(TG_STORE_F32, A2, B2, sc, 1, kg2),
-                                     tgemm_plane_bytes(TG_SQSUM_F64, A3, B3, 1, sc, kg3)})));
+    grow_planes(D.planes, {tgemm_plane_bytes(TG_STORE_F32, A1, B1, sc, 1, kg1),
+                           tgemm_plane_bytes(TG_STORE_F32, A2, B2, sc, 1, kg2),
+                           tgemm_plane_bytes(TG_SQSUM_F64, A3, B3, 1, sc, kg3)});
     // 1) P1[s][i][c][b] = sum_a X_s[(b, c)][a] Ux[i][a]       rows (b, c), cols i, batch s
     TOut o1{D.p1.p, ry, 1, ryp, (int64_t)rz * ryp, (int64_t)rz * nx * ryp};
     o1.omax = am_1;

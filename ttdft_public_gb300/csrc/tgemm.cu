@@ -529,7 +529,8 @@ struct TPlan {
   int64_t slab, bytes_b, bytes;     // A's blocks at a time, plane bytes
 };
 
-TPlan plan_of(int mode, const TOperand& A, const TOperand& B, int Z, int G, int kg) {
+TPlan plan_of(int mode, const TOperand& A, const TOperand& B, int Z, int G, int kg,
+              int64_t budget = kPlaneBudget) {
   TPlan P;
   P.chunks = mode == TG_SQSUM_F64 ? kg : G * kg;
   P.za = mode == TG_SQSUM_F64 ? G : A.batch > 0 ? Z : 1;
@@ -539,7 +540,7 @@ TPlan plan_of(int mode, const TOperand& A, const TOperand& B, int Z, int G, int 
   const int64_t per_block = P.za * P.chunks * kBlock;
   P.bytes_b = P.zb * P.bb * P.chunks * kBlock;
   P.slab = std::max<int64_t>(
-      1, std::min(P.ab, (kPlaneBudget - std::min(P.bytes_b, kPlaneBudget / 2)) / per_block));
+      1, std::min(P.ab, (budget - std::min(P.bytes_b, budget / 2)) / per_block));
   P.bytes = P.slab * per_block + P.bytes_b;
   return P;
 }
@@ -599,10 +600,17 @@ ttg_status tgemm(cudaStream_t st, int mode, const TOperand& A, const TOperand& B
   if ((A.batch > 0 && A.batch < Z) || (B.batch > 0 && B.batch < Z)) return TTG_BAD_ARG;
   if (A.rows > INT32_MAX || B.rows > INT32_MAX) return TTG_BAD_ARG;
   if (!operand_ok(A) || !operand_ok(B)) return TTG_BAD_ARG;
-  const TPlan P = plan_of(mode, A, B, Z, G, kg);
+  TPlan P = plan_of(mode, A, B, Z, G, kg);
   const int chunks = P.chunks;
   if ((P.slab * P.za + P.bb * P.zb) * chunks > INT32_MAX) return TTG_BAD_ARG;
-  if (planes.bytes < (size_t)P.bytes) TTG_TRY(planes.alloc(P.bytes));
+  // smaller slabs where there is no room for these
+  for (int64_t budget = kPlaneBudget; planes.bytes < (size_t)P.bytes;) {
+    const ttg_status s = planes.alloc(P.bytes);
+    if (s == TTG_OK) break;
+    if (s != TTG_OOM || P.slab == 1) return s;
+    while (budget > 1 && plan_of(mode, A, B, Z, G, kg, budget).slab >= P.slab) budget /= 2;
+    P = plan_of(mode, A, B, Z, G, kg, budget);
+  }
   unsigned char* pb = planes.as<unsigned char>();
   unsigned char* pa = pb + P.bytes_b;
   const int by_chunk = mode == TG_SUM_F64 ? kg : 0;

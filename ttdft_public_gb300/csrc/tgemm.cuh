@@ -47,7 +47,8 @@ enum TgemmMode {
 // at most 192 values per group.  `err` is a device int set to 1 when a
 // bounded wait ran out, to 2 when a store fell outside out.limit, to 3 when
 // a copy barrier was found out of phase (the kernel stops issuing work).
-// `planes`: grow-only work buffer of the operands' slices (at most about 1 GiB).
+// `planes`: grow-only work buffer of the operands' slices (at most about 1 GiB;
+// less where that does not fit, with more slabs of A's rows).
 ttg_status tgemm(cudaStream_t st, int mode, const TOperand& A, const TOperand& B, int Z, int G,
                  int kg, const TOut& out, int* err, DevBuf& planes);
 
