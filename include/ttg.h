@@ -71,7 +71,8 @@ typedef struct {
   int64_t n_groups;
   int64_t stored_cols;    /* merged column slots over all groups */
   double fill;            /* (nnz_h + nnz_c^T) / (group_rows * stored_cols) */
-  int64_t device_bytes;   /* HBM held by the operator */
+  int64_t device_bytes;   /* HBM held by the operator, its workspaces included (blocks are
+                             their own) */
   int64_t launches;       /* kernels this op has launched so far */
   int64_t n_tiles;        /* 64-row tiles of the tensor-core format (0: none) */
   int64_t tile_slots;     /* merged column slots over all tiles */

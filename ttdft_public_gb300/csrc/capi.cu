@@ -20,12 +20,40 @@ namespace {
 
 int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 
-ttg_status ensure(DevBuf& b, size_t bytes, ttg_op* op) {
-  if (b.bytes >= bytes) return TTG_OK;
-  const size_t old = b.bytes;
-  TTG_TRY(b.alloc(bytes));
-  op->device_bytes += (int64_t)bytes - (int64_t)old;
-  return TTG_OK;
+ttg_status ensure(DevBuf& b, size_t bytes) {
+  return b.bytes >= bytes ? TTG_OK : b.alloc(bytes);
+}
+
+// Device memory of an operator: its formats of H, working blocks and workspaces.
+int64_t device_bytes(const ttg_op* op) {
+  const RowGroups& G = op->rg;
+  const TileOp& T = op->tiles;
+  const UmmaOp& U = op->umma;
+  const Pattern& P = op->pattern;
+  const UpdatePlan& L = P.plan;
+  const HartreeWork& h = op->hw;
+  const DensityWork& d = op->dw;
+  const OzRows& Z = op->ozrows;
+  const DevBuf* all[] = {
+      &G.gptr, &G.gcol, &G.v64, &G.v32, &G.v16, &G.vdf,
+      &T.tptr, &T.tcol, &T.rowmap, &T.v32, &T.v16,
+      &U.tptr, &U.tcol, &U.rowmap, &U.order, &U.hpl, &U.xpl, &U.lptr, &U.litem, &U.rscale, &U.rcmax,
+      &U.rmax, &U.wscale, &U.cval, &U.cmax, &U.ticket, &U.err,
+      &P.row_ptr, &P.col, &P.rg_pos, &P.tile_base, &P.tile_slot, &P.umma_pos, &P.umma_row, &P.kin,
+      &P.work, &P.work2, &P.values,
+      &L.pairs, &L.where, &L.first, &L.base, &L.ld, &L.zq, &L.zlist,
+      &op->C.ptr, &op->C.col, &op->C.val, &op->C.val32,
+      &op->w32a, &op->w32b, &op->w16a, &op->w16b, &op->w64, &op->wdf, &op->wpart,
+      &op->kk0, &op->kk1, &op->kk2, &op->kk3, &op->chol, &op->eigbuf, &op->eigf, &op->partial,
+      &op->sth_a, &op->sth_b, &op->sth_part, &op->sth_part2, &op->sth_w, &op->scal, &op->status,
+      &Z.hd, &Z.he, &Z.urow, &Z.xd, &Z.xe,
+      &h.F[0], &h.F[1], &h.F[2], &h.gf, &h.p2, &h.q, &h.amax, &h.planes, &h.gauss, &h.fd, &h.ozpart, &h.err,
+      &d.uf[0], &d.uf[1], &d.uf[2], &d.xt, &d.p1, &d.p2, &d.w, &d.amax, &d.planes};
+  int64_t sum = 0;
+  for (const DevBuf* b : all) sum += (int64_t)b->bytes;
+  for (const OzWork* w : {&op->oz, &h.oz})
+    for (const DevBuf* b : {&w->planes, &w->exp, &w->kexp, &w->diag, &w->err}) sum += (int64_t)b->bytes;
+  return sum;
 }
 
 size_t block_bytes(const ttg_op* op, size_t elem) {
@@ -213,18 +241,18 @@ ttg_status ttg_op_create_tucker(int64_t n, const int64_t* h_row_ptr, const int32
     if (s != TTG_OK) return fail(s);
   }
   const int64_t kmax = std::max<int64_t>(max_k, kMaxLanczos);
-  if ((s = ensure(op->kk0, kmax * kmax * 8, op)) != TTG_OK) return fail(s);
-  if ((s = ensure(op->kk1, kmax * kmax * 8, op)) != TTG_OK) return fail(s);
-  if ((s = ensure(op->kk2, kmax * kmax * 8, op)) != TTG_OK) return fail(s);
-  if ((s = ensure(op->kk3, (kmax * kmax + 6 * kmax + 64) * 8, op)) != TTG_OK) return fail(s);
-  if ((s = ensure(op->scal, (kScalJacobi + 4 * (kmax + 2) + kmax) * 8, op)) != TTG_OK)
+  if ((s = ensure(op->kk0, kmax * kmax * 8)) != TTG_OK) return fail(s);
+  if ((s = ensure(op->kk1, kmax * kmax * 8)) != TTG_OK) return fail(s);
+  if ((s = ensure(op->kk2, kmax * kmax * 8)) != TTG_OK) return fail(s);
+  if ((s = ensure(op->kk3, (kmax * kmax + 6 * kmax + 64) * 8)) != TTG_OK) return fail(s);
+  if ((s = ensure(op->scal, (kScalJacobi + 4 * (kmax + 2) + kmax) * 8)) != TTG_OK)
     return fail(s);
-  if ((s = ensure(op->status, 64, op)) != TTG_OK) return fail(s);
+  if ((s = ensure(op->status, 64)) != TTG_OK) return fail(s);
   if (cudaHostAlloc(&op->oz.word, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) !=
       cudaSuccess)
     return fail(TTG_OOM);
   *op->oz.word = 0;
-  if ((s = ensure(op->w64, block_bytes(op, 8), op)) != TTG_OK) return fail(s);
+  if ((s = ensure(op->w64, block_bytes(op, 8))) != TTG_OK) return fail(s);
   if (cudaMemsetAsync(op->status.p, 0, 64, op->stream) != cudaSuccess) return fail(TTG_CUDA_ERR);
   if (cudaStreamSynchronize(op->stream) != cudaSuccess) return fail(TTG_CUDA_ERR);
   *out = op;
@@ -295,7 +323,7 @@ ttg_status ttg_op_info(const ttg_op* op, ttg_op_info_t* info) {
   info->fill = op->rg.slots > 0
                    ? (double)(op->nnz_h + op->nnz_c) / ((double)kGroupRows * op->rg.slots)
                    : 0.0;
-  info->device_bytes = op->device_bytes;
+  info->device_bytes = device_bytes(op);
   info->launches = op->launches;
   info->n_tiles = op->tiles.n_tiles;
   info->tile_slots = op->tiles.slots;
@@ -430,13 +458,13 @@ ttg_status ttg_cheb_filter(ttg_op* op, ttg_block* X, int32_t m, double a, double
       *x = X->x.p;
       *y = op->w64.p;
     } else if (p == TTG_PREC_FP32) {
-      TTG_TRY(ensure(op->w32a, block_bytes(op, 4), op));
-      TTG_TRY(ensure(op->w32b, block_bytes(op, 4), op));
+      TTG_TRY(ensure(op->w32a, block_bytes(op, 4)));
+      TTG_TRY(ensure(op->w32b, block_bytes(op, 4)));
       *x = op->w32a.p;
       *y = op->w32b.p;
     } else {
-      TTG_TRY(ensure(op->w16a, block_bytes(op, 2), op));
-      TTG_TRY(ensure(op->w16b, block_bytes(op, 2), op));
+      TTG_TRY(ensure(op->w16a, block_bytes(op, 2)));
+      TTG_TRY(ensure(op->w16b, block_bytes(op, 2)));
       *x = op->w16a.p;
       *y = op->w16b.p;
     }

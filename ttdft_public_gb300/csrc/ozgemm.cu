@@ -1554,11 +1554,7 @@ ttg_status launch_oz_apply(ttg_op* op, const double* src, double* dst, int k) {
   const int64_t rows = op->n + (op->C.nnz > 0 ? op->nproj : 0);
   const int groups = (k + OZ_H - 1) / OZ_H;
   auto grow = [&](DevBuf& b, size_t need) -> ttg_status {
-    if (b.bytes >= need) return TTG_OK;
-    const size_t had = b.bytes;
-    TTG_TRY(b.alloc(need));
-    op->device_bytes += (int64_t)need - (int64_t)had;
-    return TTG_OK;
+    return b.bytes >= need ? TTG_OK : b.alloc(need);
   };
   if (Z.slabs.empty()) {
     size_t free = 0, total = 0;
@@ -1580,7 +1576,6 @@ ttg_status launch_oz_apply(ttg_op* op, const double* src, double* dst, int k) {
   }
   TTG_TRY(grow(Z.hd, std::max<size_t>((size_t)Z.most * kApH, 16)));
   if (grow(Z.xd, (size_t)rows * groups * kXGroup) != TTG_OK) {
-    op->device_bytes -= (int64_t)Z.hd.bytes;
     Z.hd.release();
     Z.cut = false;
     return TTG_OOM;

@@ -780,12 +780,9 @@ ttg_status build_row_groups(ttg_op* op, int64_t n, const int64_t* hp, const int3
                                  op->stream));
     TTG_CUDA_TRY(cudaMemcpyAsync(P.rg_pos.p, rgpos.data(), hp[n] * sizeof(int32_t),
                                  cudaMemcpyHostToDevice, op->stream));
-    op->device_bytes += P.row_ptr.bytes + P.col.bytes + P.rg_pos.bytes;
   }
   // host vectors above are freed on return: wait for the copies
   TTG_CUDA_TRY(cudaStreamSynchronize(op->stream));
-  op->device_bytes += rg.gptr.bytes + rg.gcol.bytes + rg.v64.bytes + C.ptr.bytes + C.col.bytes +
-                      C.val.bytes;
   return TTG_OK;
 }
 
@@ -800,18 +797,15 @@ static ttg_status rg_values(ttg_op* op, int prec, void** out) {
     TTG_TRY(rg.v32.alloc(cnt * sizeof(float)));
     k_convert_vals<float><<<grid, 256, 0, op->stream>>>(rg.v64.as<double>(), rg.v32.as<float>(), cnt); TTG_COUNT();
     TTG_LAUNCHED(op);
-    op->device_bytes += rg.v32.bytes;
   } else if (prec == TTG_PREC_BF16 && !rg.v16.p) {
     TTG_TRY(rg.v16.alloc(cnt * sizeof(__nv_bfloat16)));
     k_convert_vals<__nv_bfloat16><<<grid, 256, 0, op->stream>>>(rg.v64.as<double>(),
                                                                rg.v16.as<__nv_bfloat16>(), cnt); TTG_COUNT();
     TTG_LAUNCHED(op);
-    op->device_bytes += rg.v16.bytes;
   } else if (prec == TTG_PREC_DF64 && !rg.vdf.p) {
     TTG_TRY(rg.vdf.alloc(cnt * sizeof(float2)));
     k_split_vals<<<grid, 256, 0, op->stream>>>(rg.v64.as<double>(), rg.vdf.as<float2>(), cnt); TTG_COUNT();
     TTG_LAUNCHED(op);
-    op->device_bytes += rg.vdf.bytes;
   }
   *out = prec == TTG_PREC_FP32 ? rg.v32.p : prec == TTG_PREC_BF16 ? rg.v16.p
          : prec == TTG_PREC_DF64 ? rg.vdf.p : rg.v64.p;
@@ -925,10 +919,7 @@ ttg_status launch_cheb_step(ttg_op* op, int prec, bool first, const void* src, c
 ttg_status launch_apply_df64(ttg_op* op, const double* src, double* dst, int k) {
   if (k <= 0 || k > op->max_k) return TTG_BAD_ARG;
   const size_t need = (size_t)(op->n + op->nproj) * op->ld * sizeof(float2);
-  if (op->wdf.bytes < need) {
-    TTG_TRY(op->wdf.alloc(need));
-    op->device_bytes += need;
-  }
+  if (op->wdf.bytes < need) TTG_TRY(op->wdf.alloc(need));
   void* vdf = nullptr;
   TTG_TRY(rg_values(op, TTG_PREC_DF64, &vdf));
   const int64_t rows = op->n + op->nproj;
@@ -950,10 +941,7 @@ static ttg_status proj_w_t(ttg_op* op, TS* src, int k) {
   const int nsplit = (int)((op->C.max_row_nnz + kProjChunk - 1) / kProjChunk);
   if (nsplit == 0) return TTG_OK;
   const size_t need = (size_t)op->nproj * nsplit * k * sizeof(TA);
-  if (op->wpart.bytes < need) {
-    TTG_TRY(op->wpart.alloc(need));
-    op->device_bytes += need;
-  }
+  if (op->wpart.bytes < need) TTG_TRY(op->wpart.alloc(need));
   const int threads = std::min(kProjCols, (k + 31) / 32 * 32);
   const int cg = (k + threads - 1) / threads;
   k_proj_partial<TS, TA><<<dim3(op->nproj, nsplit, cg), threads, 0, op->stream>>>(

@@ -412,10 +412,8 @@ ttg_status build_tiles(ttg_op* op, int64_t n, const int64_t* hp, const int32_t* 
                                  cudaMemcpyHostToDevice, op->stream));
     TTG_CUDA_TRY(cudaMemcpyAsync(P.tile_slot.p, tslot.data(), hp[n], cudaMemcpyHostToDevice,
                                  op->stream));
-    op->device_bytes += P.tile_base.bytes + P.tile_slot.bytes;
   }
   TTG_CUDA_TRY(cudaStreamSynchronize(op->stream));
-  op->device_bytes += T.tptr.bytes + T.tcol.bytes + T.rowmap.bytes + T.v32.bytes + T.v16.bytes;
   return TTG_OK;
 }
 

@@ -1175,7 +1175,6 @@ ttg_status build_umma_tiles(ttg_op* op, int64_t n, const int64_t* hp, const int3
   auto put = [&](DevBuf& b, const void* p, size_t bytes) -> ttg_status {
     TTG_TRY(b.alloc(std::max<size_t>(bytes, 16)));
     if (bytes) TTG_CUDA_TRY(cudaMemcpyAsync(b.p, p, bytes, cudaMemcpyHostToDevice, op->stream));
-    op->device_bytes += b.bytes;
     return TTG_OK;
   };
   U.ctas = ctas;
@@ -1208,10 +1207,8 @@ ttg_status build_umma_tiles(ttg_op* op, int64_t n, const int64_t* hp, const int3
     TTG_TRY(op->pattern.umma_row.alloc(n * sizeof(int32_t)));
     TTG_CUDA_TRY(cudaMemcpyAsync(op->pattern.umma_row.p, urow.data(), n * sizeof(int32_t),
                                  cudaMemcpyHostToDevice, op->stream));
-    op->device_bytes += op->pattern.umma_pos.bytes + op->pattern.umma_row.bytes;
   }
   TTG_CUDA_TRY(cudaStreamSynchronize(op->stream));
-  op->device_bytes += U.tptr.bytes + U.tcol.bytes + U.rowmap.bytes + U.order.bytes + U.hpl.bytes;
   return TTG_OK;
 }
 
@@ -1338,9 +1335,7 @@ ttg_status launch_cheb_umma(ttg_op* op, int prec, bool first, const void* src, c
   p.proj_blocks = op->nproj * p.nsplit * p.groups;
   auto grow = [&](DevBuf& b, size_t need, bool zero) -> ttg_status {
     if (b.bytes >= need) return TTG_OK;
-    op->device_bytes -= (int64_t)b.bytes;
     TTG_TRY(b.alloc(need));
-    op->device_bytes += (int64_t)need;
     if (zero) TTG_CUDA_TRY(cudaMemsetAsync(b.p, 0, need, op->stream));
     return TTG_OK;
   };

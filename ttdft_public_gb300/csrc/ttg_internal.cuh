@@ -326,7 +326,6 @@ struct ttg_op {
   ttg::DensityWork dw;        // density work buffers (ttg_density_device)
   int64_t launches = 0;
   int64_t shifted_orth = 0;   // shifted Cholesky-QR steps of ttg_chfsi_pass
-  int64_t device_bytes = 0;
 };
 
 struct ttg_block {
