@@ -1537,6 +1537,7 @@ __global__ void __launch_bounds__(kApThreads, 1) k_oz_apply(const OzApply a) {
 
 bool oz_apply_supported(const ttg_op* op, int k) {
   const UmmaOp& U = op->umma;
+  if (getenv("TTG_DISABLE_OZGEMM")) return false;
   if (U.n_tiles == 0 || op->tc_disabled || op->rg.n_groups == 0) return false;
   return k > 0;
 }
