@@ -11,8 +11,9 @@
 // Precision (FP32 degrees).  Every row of H and every column of the block is
 // scaled by a power of two (undone, exactly, in the epilogue) and each scaled
 // FP32 value is split into two FP16 terms v = v0 + v1, |v1| <= 2^-11 |v|, what
-// is left below 2^-22 |v| (and below 2^-31 of the row's or 2^-39 of the
-// column's largest value, where v1 runs out of exponents).  The product is
+// is left below 2^-22 |v|, or below the half of FP16's smallest step where v1
+// runs out of exponents: 2^-39 of the column's largest value, 2^-35 of the
+// row's (2^-29 for new values).  The product is
 // accumulated in FP32 from v0w0, v0w1 and v1w0; v1w1 is below 2^-22 |v w|.
 // An accumulation step of the tensor core truncates, the larger part of a
 // degree's error: three steps per 16 slots instead of the six of a three-term
@@ -23,9 +24,13 @@
 //    the degree before (k_colmax for the first one), and puts it in
 //    [2^14, 2^15).  A projector's W_a is at most L1(Cd_a) times that; its
 //    power of two is taken out of W_a and put into the entries of C^T.
-//  - H rows: the largest entry of a row is put in [2^7, 2^8) when the operator
-//    is built.  New values keep the row's scale while they stay in
-//    [2^-2, 2^15); k_umma_rescale gives the other rows a new one.
+//  - H rows: the largest entry of a row, C^T's with 2^L included, is put in
+//    [2^10, 2^11) when the operator is built.  New values keep the row's scale
+//    while they stay in [2^4, 2^15), sixteen times up and 64 down; the first
+//    potential of an SCF moves a row's largest entry by a factor of 6 at most.
+//    k_umma_rescale gives the other rows a new scale.  (C^T's entries leave H's
+//    a coarser step only where L1(Cd_a) is large, and by less than the FP32
+//    rounding of the W_a that they multiply.)
 //
 // Data movement per chunk.
 //  - H: the chunk's planes (128 x 16 values each, already in the canonical
@@ -109,6 +114,8 @@ constexpr int kBWarps = 10;
 constexpr int kThreads = 32 * (kFirstBWarp + kBWarps);
 constexpr int kMaxCtas = 152;
 constexpr int kMaxWait = 1 << 20;
+constexpr int kRowExp = 10;                   // a scaled row's largest entry: [2^10, 2^11)
+constexpr float kRowLow = 16.f;               // smallest one that keeps its row's scale
 constexpr int kAtom = 64;                     // states per 128-byte swizzle row
 constexpr int kAtomBytes = 16 * 128;          // one atom of a chunk: 16 slot rows x 128 bytes
 
@@ -921,8 +928,8 @@ __global__ void __launch_bounds__(256) k_umma_rescale(const RescaleArgs a) {
   if (row < 0) return;
   const float hmax = a.rmax[ur], largest = fmaxf(hmax, a.cmax[ur]);
   const float scaled = largest / a.rscale[ur];     // a power of two: exact or infinite
-  if (largest == 0.f || (scaled >= 0.25f && scaled < 32768.f)) return;
-  const int e = min(126, max(-126, 7 - ilogbf(largest)));
+  if (largest == 0.f || (scaled >= kRowLow && scaled < 32768.f)) return;
+  const int e = min(126, max(-126, kRowExp - ilogbf(largest)));
   const float up = scalbnf(1.f, e);
   const int64_t tile = ur >> 7;
   const int m = (int)(ur & 127);
@@ -1139,7 +1146,7 @@ ttg_status build_umma_tiles(ttg_op* op, int64_t n, const int64_t* hp, const int3
         if (nproj > 0)
           for (int64_t e = tp[r]; e < tp[r + 1]; ++e) raise_max(cmax, tvs[e]);
         const float big = std::max(hmax, cmax);
-        const int ex = big > 0.f ? std::min(126, std::max(-126, 7 - std::ilogb(big))) : 0;
+        const int ex = big > 0.f ? std::min(126, std::max(-126, kRowExp - std::ilogb(big))) : 0;
         const float up = std::ldexp(1.f, ex);
         rscale[t * UR + m] = std::ldexp(1.f, -ex);
         rcmax[t * UR + m] = cmax;
