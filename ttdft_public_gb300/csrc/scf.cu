@@ -399,29 +399,33 @@ __global__ void __launch_bounds__(256) k_lda(const double* __restrict__ rho, int
 }
 
 // partial[b] = sum over block b of f*g*wx*wy*wz (g may be null).  L lanes take
-// one x-line: the sum over x of f g wx costs two FP64 operations a point
-// (four when the weights are multiplied point by point, which bound the sum),
-// the weights wy wz one a line and lane.  360^3 points, 0.36 -> 0.23 ms.
+// one of the P pieces of an x-line: the sum over x of f g wx costs two FP64
+// operations a point (four when the weights are multiplied point by point,
+// which bound the sum), the weights wy wz one a piece and lane.  360^3 points,
+// 0.36 -> 0.23 ms.  Grids of few lines need the pieces to fill the SMs.
 __global__ void __launch_bounds__(256) k_wsum(
     const double* __restrict__ f, const double* __restrict__ g, const double* __restrict__ wx,
     const double* __restrict__ wy, const double* __restrict__ wz, int n0, int n1, int n2, int L,
-    double* __restrict__ partial) {
+    int P, double* __restrict__ partial) {
   __shared__ double red[32];
-  const int64_t lines = (int64_t)n1 * n2;
+  const int64_t items = (int64_t)n1 * n2 * P;
+  const int len = (n0 + P - 1) / P;
   const int sub = threadIdx.x % L;
   const int64_t step = (int64_t)gridDim.x * (blockDim.x / L);
   double s = 0.0;
-  for (int64_t l = (int64_t)blockIdx.x * (blockDim.x / L) + threadIdx.x / L; l < lines; l += step) {
+  for (int64_t i = (int64_t)blockIdx.x * (blockDim.x / L) + threadIdx.x / L; i < items; i += step) {
+    const int64_t l = P == 1 ? i : i / P;
+    const int x0 = P == 1 ? 0 : (int)(i - l * P) * len, x1 = min(n0, x0 + len);
     const int y = (int)(l % n1), z = (int)(l / n1);
     const double* fl = f + l * n0;
     double t = 0.0;
     if (g) {
       const double* gl = g + l * n0;
 #pragma unroll 4
-      for (int x = sub; x < n0; x += L) t = fma(fl[x] * gl[x], wx[x], t);
+      for (int x = x0 + sub; x < x1; x += L) t = fma(fl[x] * gl[x], wx[x], t);
     } else {
 #pragma unroll 4
-      for (int x = sub; x < n0; x += L) t = fma(fl[x], wx[x], t);
+      for (int x = x0 + sub; x < x1; x += L) t = fma(fl[x], wx[x], t);
     }
     s = fma(t, wy[y] * wz[z], s);
   }
@@ -458,7 +462,11 @@ void launch_wsum(cudaStream_t st, const double* f, const double* g, const double
                  const double* wy, const double* wz, const int* n, double* part, double* out) {
   int L = 32;                    // lanes a line: no more than its points
   while (L > 1 && L > n[0]) L /= 2;
-  k_wsum<<<kWsumBlocks, 256, 0, st>>>(f, g, wx, wy, wz, n[0], n[1], n[2], L, part); TTG_COUNT();
+  // lanes enough for every item of the grid at once, pieces of 128 points or more
+  const int64_t lines = std::max<int64_t>((int64_t)n[1] * n[2], 1);
+  const int P = (int)std::max<int64_t>(
+      1, std::min<int64_t>(kWsumBlocks * (256 / L) / lines, n[0] / 128));
+  k_wsum<<<kWsumBlocks, 256, 0, st>>>(f, g, wx, wy, wz, n[0], n[1], n[2], L, P, part); TTG_COUNT();
   k_sum_partials<<<1, 256, 0, st>>>(part, kWsumBlocks, out); TTG_COUNT();
 }
 
