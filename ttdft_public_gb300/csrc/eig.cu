@@ -88,6 +88,21 @@ __device__ __forceinline__ double fast_inv(double x) {
   return fma(y, fma(e, e, e), y);
 }
 
+// x / y; a reciprocal of its own where y is well inside the FP32 range (beyond
+// it 1 / y may overflow where x / y does not)
+__device__ __forceinline__ double fast_div(double x, double y) {
+  const float a = fabsf((float)y);
+  return a > 1e-30f && a < 1e30f ? x * fast_inv(y) : x / y;
+}
+
+// Largest |v| over the 128 threads of the vector stage (named barrier 1).
+__device__ __forceinline__ double vec_max(double v, double* red) {
+  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  asm volatile("bar.sync 1, %0;" ::"n"(kVecWarps * 32) : "memory");
+  return fmax(fmax(red[0], red[1]), fmax(red[2], red[3]));
+}
+
 // Stage 1.  A (n x n column-major, symmetric); outputs the diagonal d,
 // off-diagonal e (e[i] couples i and i+1), tau and the reflectors Vr (column
 // j holds v_j in rows j+1..n-1).
@@ -96,7 +111,10 @@ __device__ __forceinline__ double fast_inv(double x) {
 // whole cluster holds 16 x 226 KB), or for larger n in A itself (its column r,
 // L2 and L1 of that SM).  Per column j:
 //  - vector stage, redundantly on every CTA (four warps): the column x_j of
-//    the updated matrix -> reflector v_j, tau_j;
+//    the updated matrix -> reflector v_j, tau_j.  A column whose square is far
+//    from 1 is first scaled by a power of two, which the reflector does not see:
+//    the columns of a matrix of low rank can fall by 1e-16 each, down to where
+//    1 / |v|^2 overflows;
 //  - pass over the CTA's rows, a warp per row: the rank-2 update of column
 //    j - 1 (B -= v w^T + w v^T) and p = tau B v_j in one sweep, three FP64 FMAs
 //    an element; each row's p_r and its entry of column j + 1 go to every CTA
@@ -143,6 +161,22 @@ __global__ void __launch_bounds__(kTrThreads) k_tridiag_cluster(
       double ss = 0.0;
       for (int r = j + 1 + tid; r < n; r += kVecWarps * 32) ss = fma(v[r], v[r], ss);
       ss = vec_sum(ss, red[0]);
+      int ex = 0;                                   // the same for all threads
+      if (!(ss > 1e-200 && ss < 1e200)) {
+        double m = 0.0;
+        for (int r = j + 1 + tid; r < n; r += kVecWarps * 32) m = fmax(m, fabs(v[r]));
+        m = vec_max(m, red[1]);
+        if (m > 0.0 && m < INFINITY) {
+          ex = ilogb(m);
+          ss = 0.0;
+          for (int r = j + 1 + tid; r < n; r += kVecWarps * 32) {
+            const double x = ldexp(v[r], -ex);
+            v[r] = x;
+            ss = fma(x, x, ss);
+          }
+          ss = vec_sum(ss, red[0]);
+        }
+      }
       if (warp == 0) {
         const double x0 = v[j + 1];
         const double nrm = ss > 0.0 ? ss * fast_rsqrt(ss) : 0.0;
@@ -155,7 +189,7 @@ __global__ void __launch_bounds__(kTrThreads) k_tridiag_cluster(
           v[j + 1] = x0 - alpha;
           s_tau = t;
           if (q == 0) {
-            e[j] = h > 0.0 ? alpha : x0;
+            e[j] = ldexp(h > 0.0 ? alpha : x0, ex);
             tau[j] = t;
           }
         }
@@ -422,11 +456,11 @@ __global__ void __launch_bounds__(32) k_tridiag_vectors(
       const double sub = se[i];
       const double na = sd[i + 1] - lam, nb = (i + 2 < n ? se[i + 1] : 0.0);
       if (fabs(a) >= fabs(sub)) {
-        const double mlt = (a != 0.0 ? sub * fast_inv(a) : 0.0);
+        const double mlt = (a != 0.0 ? fast_div(sub, a) : 0.0);
         dg[i] = a; u1[i] = bb; u2[i] = c; ml[i] = mlt; sw[i] = 0;
         a = fma(-mlt, bb, na); bb = fma(-mlt, c, nb); c = 0.0;
       } else {
-        const double mlt = a * fast_inv(sub);
+        const double mlt = fast_div(a, sub);
         dg[i] = sub; u1[i] = na; u2[i] = nb; ml[i] = mlt; sw[i] = 1;
         a = fma(-mlt, na, bb); bb = fma(-mlt, nb, c); c = 0.0;
       }
