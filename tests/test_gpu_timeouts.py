@@ -84,6 +84,7 @@ def reconstruct(op, lib):
 @pytest.mark.parametrize("call", [gram, chol_qr, ritz, ritz_on_the_device, rotate, syev, update, tucker, reconstruct])
 def test_the_call_itself_reports_it(op, call, monkeypatch):
     lib = _lib.ttg()
+    monkeypatch.setenv("TTG_UPDATE_SLAB_VALUES", "100000000")        # the tensor cores for a small update
     assert call(op, lib) == 0
     monkeypatch.setenv("TTG_FAKE_TIMEOUT", "1")
     assert call(op, lib) == TIMEOUT

@@ -60,19 +60,23 @@ class Problem:
         assert np.all(np.abs(self.Ym.get() - ref) <= 2.0 ** -43 * (B @ np.abs(X) + nl))
 
 
-@pytest.fixture
-def problem():
-    p = Problem()
+@pytest.fixture(params=[11])
+def problem(request):
+    p = Problem(request.param)
     yield p
     p.op.close()
 
 
+@pytest.mark.parametrize("problem", [5, 9, 11], indirect=True)
 def test_values_in_slabs_and_by_entry(problem, monkeypatch):
-    monkeypatch.setenv("TTG_UPDATE_SLAB_VALUES", "200000")           # one y a slab
-    for seed, ranks in enumerate(((8, 6, 17), (3, 7, 40))):
-        rc, launches = problem.update(ranks, seed)
-        assert rc == 0 and launches > 11 * 3                         # scales, digits, product of each slab
-        problem.check()
+    assert problem.update((2, 3, 4), 8)[0] == 0                      # by entry: a small operator
+    problem.check()
+    for values in (200000, 100000000):                               # one y a slab (11 functions), one slab
+        monkeypatch.setenv("TTG_UPDATE_SLAB_VALUES", str(values))
+        for seed, ranks in enumerate(((8, 6, 17), (3, 7, 40))):
+            rc, launches = problem.update(ranks, seed)
+            assert rc == 0 and launches >= 12                        # scales, digits, product of three sums
+            problem.check()
     monkeypatch.setenv("TTG_DISABLE_OZGEMM", "1")
     assert problem.update((8, 6, 17), 9)[0] == 0
     problem.check()
@@ -97,6 +101,7 @@ def test_no_room_once_is_not_for_good(problem, monkeypatch):
     monkeypatch.setenv("TTG_DISABLE_OZGEMM", "1")
     by_entry = problem.update(ranks, 0)
     monkeypatch.delenv("TTG_DISABLE_OZGEMM")
+    monkeypatch.setenv("TTG_UPDATE_SLAB_VALUES", "100000000")        # the tensor cores for a small operator
     monkeypatch.setenv("TTG_ALLOC_LIMIT", "1000")
     assert problem.update(ranks, 1) == by_entry                      # nothing fits: the same kernels
     problem.check()

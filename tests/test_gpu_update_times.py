@@ -1,0 +1,64 @@
+"""Hamiltonian updates of small and flat operators are no slower than with the CUDA-core sums alone: where the
+tensor cores' launches and padded tiles cost more than they save they are not used."""
+import itertools
+import os
+import time
+
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+from ttdft_public_gb300 import _lib, api, system
+
+pytestmark = pytest.mark.gpu
+
+
+def pattern(r, reach=8):
+    n = int(np.prod(r))
+    i = np.arange(n)
+    x, y, z = i % r[0], i // r[0] % r[1], i // (r[0] * r[1])
+    rows, cols = [], []
+    for dx, dy, dz in itertools.product(range(-reach, reach + 1), repeat=3):
+        if dx * dx + dy * dy + dz * dz <= reach * reach:
+            ok = (x + dx >= 0) & (x + dx < r[0]) & (y + dy >= 0) & (y + dy < r[1]) & (z + dz >= 0) & (z + dz < r[2])
+            rows.append(i[ok])
+            cols.append(i[ok] + dx + r[0] * (dy + r[1] * dz))
+    rows, cols = np.concatenate(rows), np.concatenate(cols)
+    M = sp.csr_matrix((np.ones(rows.size), (rows, cols)), shape=(n, n))
+    M.sort_indices()
+    return system.Csr(n, n, M.indptr.astype(np.int64), M.indices.astype(np.int32), M.data)
+
+
+@pytest.mark.parametrize("r, ranks", [((5, 5, 5), (5, 6, 7)), ((40, 40, 1), (5, 6, 7)), ((100, 3, 3), (1, 1, 1)),
+                                      ((4, 4, 30), (16, 16, 16)), ((12, 12, 12), (6, 6, 6)), ((60, 60, 3), (6, 6, 6)),
+                                      ((17, 17, 17), (32, 32, 32))])
+def test_no_slower_than_the_cuda_cores(r, ranks, monkeypatch):
+    op, lib = api.Operator(api.ProjectHamiltonianSparse(pattern(r), ranks=r), 8), _lib.ttg()
+    try:
+        basis = [system.make_basis_1d(system.Fem1D(2 * m + 2, 0.0, 0.8 * m + 2), m) for m in r]
+        K = [np.ascontiguousarray(b.stiffness()) for b in basis] + [np.ascontiguousarray(b.overlap()) for b in basis]
+        assert lib.ttg_op_set_kinetic(op.h, *[_lib.ptr(k) for k in K]) == 0
+        import ctypes
+
+        import torch
+        p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+        G = torch.rand(int(np.prod(ranks)), dtype=torch.float64, device="cuda")
+        P = [torch.rand(ranks[d] * r[d] * r[d], dtype=torch.float64, device="cuda") for d in range(3)]
+        torch.cuda.synchronize()
+
+        def best():
+            times = []
+            for _ in range(12):
+                t = time.perf_counter()
+                assert lib.ttg_op_update_potential_device(op.h, _lib.ptr(np.array(ranks, np.int32)), p(G),
+                                                          *[p(m) for m in P]) == 0
+                op.sync()
+                times.append(time.perf_counter() - t)
+            return min(times)
+
+        now = best()
+        monkeypatch.setenv("TTG_DISABLE_OZGEMM", "1")
+        assert "TTG_UPDATE_SLAB_VALUES" not in os.environ
+        assert now < 1.2 * best() + 5e-6
+    finally:
+        op.close()

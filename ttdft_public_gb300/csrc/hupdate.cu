@@ -26,8 +26,9 @@
 // of 128 of them share a prefix: one ragged FP64 GEMM on the tensor cores (a few
 // GB of values at most at a time, in slabs of y), from which the entries are
 // gathered.  64 atoms: 24.6 -> 12.1 ms in all, 5.9 of
-// them the gather and the scattered writes into the formats.  The per-entry sum stays for
-// operators that the plan does not fit and where the tensor cores are off.
+// them the gather and the scattered writes into the formats.  The per-entry sum stays where it
+// is faster (entry_seconds), for operators that the plan does not fit and where
+// the tensor cores are off.
 
 #include <algorithm>
 #include <cmath>
@@ -236,6 +237,28 @@ __global__ void __launch_bounds__(256) k_pair_width(const UpdateArgs a, int* __r
   }
 }
 
+// From this many flops on T1 and T2 go to the tensor cores: their eight launches
+// cost 40 us more than the CUDA-core GEMM's two.  Update of 40 x 40 x 1
+// functions, both ways: rank 6 (3.4e7 flops) 132 against 158 us on the tensor
+// cores, rank 16 (2.4e8) 224 against 200; of 14^3, rank 32 (1.3e8) 612 against 623.
+constexpr double kTensorFlops = 1.5e8;
+
+// Seconds of the last sum on the CUDA cores and on the tensor cores (ragged
+// product of `pairs` rows, launches, scales and digits of the rows), fitted to
+// 80 updates of 125 to 13,824 functions, ranks 1 to 72, flat and long bases
+// among them.  14^3 functions, by entry against ragged: rank 1 203 and 234 us,
+// rank 6 249 and 239, rank 32 612 and 301; 60 x 60 x 3 (a million pairs), rank 6
+// 416 and 737.
+double entry_seconds(int64_t nnz, int rc) { return 2.0 * nnz * rc / 0.7e12 + 0.4e-6 * rc; }
+double ragged_seconds(int64_t pairs, int64_t nq, int rc) {
+  const double tiles = (double)pairs / 128.0 * (double)((nq + 63) / 64) * 0.6;
+  return 35e-6 + pairs * (1.5e-10 + (rc + 15) / 16 * 16 * 32 / 6e12) +
+         tiles / 152.0 * ((rc + 127) / 128 + 2) * 0.4e-6;
+}
+
+// The tests' small operators take the tensor cores where this is set.
+bool tensor_forced() { return getenv("TTG_UPDATE_SLAB_VALUES") != nullptr; }
+
 // Most values of a slab (8 bytes each); TTG_UPDATE_SLAB_VALUES sets another limit.
 int64_t slab_values() {
   const char* e = getenv("TTG_UPDATE_SLAB_VALUES");
@@ -378,13 +401,15 @@ ttg_status update_from_tables(ttg_op* op, const UpdateLayout& L) {
   // T1[b][xp][c] = sum_a PXp[xp][a] G[a + ra (b + rb c)], then
   // T2[yp][(xp, c)] = sum_b PYp[yp][b] T1[b][(xp, c)]: FP64 GEMMs on the tensor
   // cores with the long dimension, (b, c) and (xp, c), as their rows; the
-  // double-FP32 GEMM on the CUDA cores where those are off.  64-atom system,
-  // potential ranks 72: 18.2 -> 2.2 ms for both.
+  // double-FP32 GEMM on the CUDA cores where they are small or those are off.
+  // 64-atom system, potential ranks 72: 18.2 -> 2.2 ms for both.
   const int64_t xc = nxp * rc;
   const OzOperand g1{w + off_g, (int64_t)rb * rc, ra, ra, 1}, p1{w + off_x, nxp, ra, ra, 1};
   const OzOperand g2{w + off_t1, xc, rb, 1, xc}, p2{w + off_y, nyp, rb, rb, 1};
   ttg_status s = TTG_OOM;
-  if (ozgemm_supported(g1, p1) && ozgemm_supported(g2, p2)) {
+  const double flops = 2.0 * xc * rb * ra + 2.0 * nyp * xc * rb;
+  if ((flops >= kTensorFlops || tensor_forced()) && ozgemm_supported(g1, p1) &&
+      ozgemm_supported(g2, p2)) {
     s = ozgemm(op, g1, p1, w + off_t1, OzLayout{xc, rc, rb, 1}, false);
     if (s == TTG_OK) s = ozgemm(op, g2, p2, w + off_t2, OzLayout{1, xc}, false);
   }
@@ -429,7 +454,10 @@ ttg_status update_from_tables(ttg_op* op, const UpdateLayout& L) {
   if (op->nnz_h == 0) return TTG_OK;           // no entry to update
   const int nxg = (rx + 7) / 8;
   UpdatePlan& plan = P.plan;
-  const bool oz = ozgemm_supported(g1, p1);
+  int64_t nq = rz;                             // z pairs
+  for (int d = 1; d <= bw[2]; ++d) nq += 2 * std::max(0, rz - d);
+  const bool oz = (ragged_seconds(nxp * nyp, nq, rc) < entry_seconds(op->nnz_h, rc) || tensor_forced()) &&
+                  ozgemm_supported(g1, p1);
   // the plan's slabs hold for the rank it was made for and smaller ones; a rank
   // without a plan says nothing about smaller ones
   const int64_t max_rows = ozgemm_ragged_rows(rc, plan.nq);
