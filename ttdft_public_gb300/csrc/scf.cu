@@ -572,24 +572,33 @@ struct LinTerms {
 };
 
 // Four points a thread keep enough loads in flight (360^3 points, two fields:
-// 0.39 -> 0.20 ms; six: 0.73 -> 0.52 ms, where the FP64 pipe sets 0.48).
+// 0.39 -> 0.20 ms; six: 0.73 -> 0.52 ms, where the FP64 pipe sets 0.48), in equal
+// passes over the field.  Small fields take a point a thread and eight fields
+// ahead: with few threads the chain of a thread's loads is the time (device time
+// of 100,003 points, 24 fields: 9 us, 23 with four points; 1.5 million points, six
+// fields: 27 us and 25).  With many fields that holds up to larger ones (2.6
+// million, 24 fields: 122 us and 139; 5 million: 228 and 230).
+constexpr int64_t kLincombSmall = 1250000, kLincombSmallMany = 5000000;
+constexpr int kLincombMany = 12;
+
+template <int U>
 __global__ void __launch_bounds__(256) k_lincomb(const __grid_constant__ LinTerms t, int nt,
                                                  int64_t n, double* out, int take_abs) {
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 4 * step) {
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 2
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += U * step) {
+    double s[U] = {};
+#pragma unroll(8 / U)
     for (int m = 0; m < nt; ++m) {
       const double* f = t.f[m];
       const double c = t.c[m];
-      double x[4];
+      double x[U];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) x[u] = i + u * step < n ? f[i + u * step] : 0.0;
+      for (int u = 0; u < U; ++u) x[u] = i + u * step < n ? f[i + u * step] : 0.0;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) s[u] += c * x[u];
+      for (int u = 0; u < U; ++u) s[u] += c * x[u];
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < U; ++u)
       if (i + u * step < n) out[i + u * step] = take_abs ? fabs(s[u]) : s[u];
   }
 }
@@ -880,7 +889,13 @@ ttg_status ttg_grid_lincomb(int32_t nterms, const double* const* fields_dev, con
     t.f[m] = fields_dev[m];
     t.c[m] = coef[m];
   }
-  k_lincomb<<<gblocks(n), 256, 0, S.s>>>(t, nterms, n, out_dev, take_abs); TTG_COUNT();
+  if (n <= (nterms > kLincombMany ? kLincombSmallMany : kLincombSmall)) {
+    k_lincomb<1><<<gblocks(n), 256, 0, S.s>>>(t, nterms, n, out_dev, take_abs);
+  } else {                       // equal passes over the field
+    const int64_t quads = (n + 1023) / 1024, passes = (quads + 152 * 16 - 1) / (152 * 16);
+    k_lincomb<4><<<(unsigned)((quads + passes - 1) / passes), 256, 0, S.s>>>(t, nterms, n, out_dev, take_abs);
+  }
+  TTG_COUNT();
   TTG_CUDA_TRY(cudaGetLastError());
   return TTG_OK;
 }
