@@ -95,12 +95,33 @@ __device__ __forceinline__ double fast_div(double x, double y) {
   return a > 1e-30f && a < 1e30f ? x * fast_inv(y) : x / y;
 }
 
-// Largest |v| over the 128 threads of the vector stage (named barrier 1).
-__device__ __forceinline__ double vec_max(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+// Largest v over the 128 threads of the vector stage (named barrier 1).
+__device__ __forceinline__ int vec_max(int v, double* red) {
+  v = __reduce_max_sync(0xffffffffu, v);
+  int* m = reinterpret_cast<int*>(red);
+  if ((threadIdx.x & 31) == 0) m[threadIdx.x >> 5] = v;
   asm volatile("bar.sync 1, %0;" ::"n"(kVecWarps * 32) : "memory");
-  return fmax(fmax(red[0], red[1]), fmax(red[2], red[3]));
+  return max(max(m[0], m[1]), max(m[2], m[3]));
+}
+
+// The column v[j + 1 .. n) scaled by a power of two to a largest entry near 1;
+// its square, and the exponent taken out (0 for zeros and non-finite values).
+// By the 128 threads of the vector stage; a rare path, kept out of the loop.
+__device__ __noinline__ double scale_column(double* v, int j, int n, double ss, double (*red)[kVecWarps],
+                                            int& ex) {
+  int m = 0;                                        // largest biased exponent
+  for (int r = j + 1 + threadIdx.x; r < n; r += kVecWarps * 32)
+    m = max(m, (__double2hiint(v[r]) >> 20) & 0x7ff);
+  m = vec_max(m, red[1]);
+  if (m == 0 || m == 0x7ff) return ss;
+  ex = m - 1023;
+  ss = 0.0;
+  for (int r = j + 1 + threadIdx.x; r < n; r += kVecWarps * 32) {
+    const double x = ldexp(v[r], -ex);
+    v[r] = x;
+    ss = fma(x, x, ss);
+  }
+  return vec_sum(ss, red[0]);
 }
 
 // Stage 1.  A (n x n column-major, symmetric); outputs the diagonal d,
@@ -162,21 +183,8 @@ __global__ void __launch_bounds__(kTrThreads) k_tridiag_cluster(
       for (int r = j + 1 + tid; r < n; r += kVecWarps * 32) ss = fma(v[r], v[r], ss);
       ss = vec_sum(ss, red[0]);
       int ex = 0;                                   // the same for all threads
-      if (!(ss > 1e-200 && ss < 1e200)) {
-        double m = 0.0;
-        for (int r = j + 1 + tid; r < n; r += kVecWarps * 32) m = fmax(m, fabs(v[r]));
-        m = vec_max(m, red[1]);
-        if (m > 0.0 && m < INFINITY) {
-          ex = ilogb(m);
-          ss = 0.0;
-          for (int r = j + 1 + tid; r < n; r += kVecWarps * 32) {
-            const double x = ldexp(v[r], -ex);
-            v[r] = x;
-            ss = fma(x, x, ss);
-          }
-          ss = vec_sum(ss, red[0]);
-        }
-      }
+      const int be = __double2hiint(ss) >> 20;      // biased exponent: |v|^2 in 2^(+-700)
+      if (be < 323 || be > 1723) ss = scale_column(v, j, n, ss, red, ex);
       if (warp == 0) {
         const double x0 = v[j + 1];
         const double nrm = ss > 0.0 ? ss * fast_rsqrt(ss) : 0.0;
@@ -189,7 +197,8 @@ __global__ void __launch_bounds__(kTrThreads) k_tridiag_cluster(
           v[j + 1] = x0 - alpha;
           s_tau = t;
           if (q == 0) {
-            e[j] = ldexp(h > 0.0 ? alpha : x0, ex);
+            const double ej = h > 0.0 ? alpha : x0;
+            e[j] = ex ? ldexp(ej, ex) : ej;
             tau[j] = t;
           }
         }
@@ -556,8 +565,9 @@ __global__ void __launch_bounds__(32) k_tridiag_vectors(
     if (lane + 32 * v < n) U[(int64_t)b * n + lane + 32 * v] = y[v] * inv;
 }
 
-// N = (3 I - S) / 2 in place; *dev = max |S - I| (FP64 bits, zeroed before)
-__global__ void __launch_bounds__(256) k_newton_schulz(double* __restrict__ S, int r,
+// N = (3 I - S) / 2; *dev = max |S - I| (FP64 bits, zeroed before)
+__global__ void __launch_bounds__(256) k_newton_schulz(const double* __restrict__ S,
+                                                       double* __restrict__ N, int r,
                                                        unsigned long long* dev) {
   const int64_t total = (int64_t)r * r;
   double m = 0.0;
@@ -566,7 +576,7 @@ __global__ void __launch_bounds__(256) k_newton_schulz(double* __restrict__ S, i
     const double one = (i % r == i / r) ? 1.0 : 0.0, s = S[i];
     const double dv = fabs(s - one);
     m = dv <= m ? m : dv;                        // a NaN stays
-    S[i] = 1.5 * one - 0.5 * s;
+    N[i] = 1.5 * one - 0.5 * s;
   }
   unsigned long long mb = (unsigned long long)__double_as_longlong(m);
   for (int o = 16; o > 0; o >>= 1) {
@@ -759,17 +769,17 @@ ttg_status sym_topk(ttg_op* op, double* A, int n, int r, double* w, double* U, i
     }
     return dgemm(st, n, r, r, 1, Un, DOp{M, ks, js, 0}, U2, 1, n, 0, op->partial);
   };
-  // S = U^T U = I + E, replaced by (3 I - S) / 2
+  // S = U^T U = I + E; Li = (3 I - S) / 2
   TTG_TRY(gram());
   TTG_CUDA_TRY(cudaMemsetAsync(dev, 0, 8, st));
-  k_newton_schulz<<<32, 256, 0, st>>>(S, r, dev); TTG_COUNT();
+  k_newton_schulz<<<32, 256, 0, st>>>(S, Li, r, dev); TTG_COUNT();
   TTG_LAUNCHED(op);
   double far = 0.0;
   TTG_CUDA_TRY(cudaMemcpyAsync(&far, dev, 8, cudaMemcpyDeviceToHost, st));
   TTG_CUDA_TRY(cudaMemsetAsync(d_status, 0, 4, st));
   TTG_CUDA_TRY(cudaStreamSynchronize(st));
   if (far <= 1e-8) {
-    TTG_TRY(product(S, 1, r));
+    TTG_TRY(product(Li, 1, r));
     TTG_CUDA_TRY(cudaMemcpyAsync(U, U2, (size_t)n * r * sizeof(double), cudaMemcpyDeviceToDevice,
                                  st));
     op->launches += 2;
@@ -777,7 +787,7 @@ ttg_status sym_topk(ttg_op* op, double* A, int n, int r, double* w, double* U, i
   }
   // Cholesky QR2: U <- U L^-T with U^T U = L L^T
   for (int pass = 0; pass < 2; ++pass) {
-    TTG_TRY(gram());
+    if (pass > 0) TTG_TRY(gram());
     TTG_TRY(cholesky_inv(op, S, Li, r, d_status));
     int stat = 0;
     TTG_CUDA_TRY(cudaMemcpyAsync(&stat, d_status, 4, cudaMemcpyDeviceToHost, st));
