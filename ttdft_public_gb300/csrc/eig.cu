@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(256) k_newton_schulz(const double* __restrict_
        i += (int64_t)gridDim.x * blockDim.x) {
     const double one = (i % r == i / r) ? 1.0 : 0.0, s = S[i];
     const double dv = fabs(s - one);
-    m = dv <= m ? m : dv;                        // a NaN stays
+    m = dv > m || dv != dv ? dv : m;             // a NaN stays
     N[i] = 1.5 * one - 0.5 * s;
   }
   unsigned long long mb = (unsigned long long)__double_as_longlong(m);
