@@ -74,7 +74,9 @@ ttg_status check_block(const ttg_op* op, const ttg_block* b) {
 }
 
 // S = X^T Y (k x k, column-major) from FP64 blocks: on the tensor cores
-// (ozgemm.cu) where the operands allow, else the double-FP32 CUDA-core kernel.
+// (ozgemm.cu), faster at every size (a call of 1,000 x 12 54 us, 129 on the CUDA
+// cores; 9,261 x 57 61 and 141; 200,000 x 13 281 and 543), or the double-FP32
+// CUDA-core kernel where they have no room.
 ttg_status gram_fp64(ttg_op* op, const double* X, const double* Y, int k, double* S, bool sym) {
   const OzOperand A{X, k, op->n, 1, op->ld}, B{Y, k, op->n, 1, op->ld};
   if (ozgemm_supported(A, B)) {
@@ -94,9 +96,11 @@ ttg_status product_fp64(ttg_op* op, const double* X, const double* Q, double* ou
   const OzOperand A{X, op->n, k, op->ld, 1};
   const OzOperand B = transQ ? OzOperand{Q, k, k, 1, k} : OzOperand{Q, k, k, k, 1};
   const OzOperand cols{X, k, op->n, 1, op->ld};
-  // Odd widths stay on the CUDA cores, as they always were (the factor's rows
-  // once had to be 16-byte aligned): there its error is smaller (X L^-T of
-  // 9,000 x 50: 9e-15 against 3e-14), and no odd width is large.
+  // Odd widths, of any size, stay on the CUDA cores, as they always were (the
+  // factor's rows once had to be 16-byte aligned).  Their error is smaller there
+  // (X L^-T of 9,000 x 50: 9e-15 against 3e-14), so that the tensor cores would
+  // cost them precision; they pay with time (a rotation of 20,000 x 333 takes 1.5
+  // ms, of 334 columns 0.25; 512,000 x 1,199 0.40 s, of 1,200 columns 0.03).
   if (k % 2 == 0 && ozgemm_supported(A, B)) {
     const ttg_status s = ozgemm(op, A, B, out, OzLayout{op->ld, 1}, false, transQ && lower,
                                 kscale ? &cols : nullptr);

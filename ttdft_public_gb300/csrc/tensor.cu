@@ -199,7 +199,11 @@ __global__ void k_block_chunk(const double* __restrict__ X, int64_t n, int64_t l
 }
 
 // From this many flops a direction the factors' sums run on the tensor cores.
-constexpr double kFactorOzFlops = 5e7;
+// Whole evaluations with the factors there and on the FP64 pipe: 120 points, rank
+// 48, 35 terms (4.8e7 flops) 604 and 574 us; rank 60 (6e7) 682 and 665; 360
+// points, rank 60, 5 terms (7.8e7) 1,175 and 1,139; 180 points, rank 40, 35 terms
+// (9.1e7) 1,022 and 1,190.
+constexpr double kFactorOzFlops = 8e7;
 
 // Device inputs of one Hartree evaluation (all FP64, device pointers).
 struct HartreeIn {
@@ -264,7 +268,6 @@ ttg_status hartree_tc(cudaStream_t st, HartreeWork& w, const HartreeIn& in, doub
     const int nx_d = in.n[d], nq_d = in.nq[d], r_d = in.r[d];
     const int64_t rows = (int64_t)K * nx_d;
     ttg_status s = TTG_OOM;
-    // few or short sums: the two launches less are worth more
     if (2.0 * rows * nq_d * r_d >= kFactorOzFlops) {
       const OzOperand U{in.U[d], r_d, nq_d, nq_d, 1};
       if ((w.gauss.bytes >= (size_t)(rows * nq_d * 8) || w.gauss.alloc(rows * nq_d * 8) == TTG_OK) &&
