@@ -31,7 +31,8 @@ def pattern(r, reach=8):
 
 @pytest.mark.parametrize("r, ranks", [((5, 5, 5), (5, 6, 7)), ((40, 40, 1), (5, 6, 7)), ((100, 3, 3), (1, 1, 1)),
                                       ((4, 4, 30), (16, 16, 16)), ((12, 12, 12), (6, 6, 6)), ((60, 60, 3), (6, 6, 6)),
-                                      ((17, 17, 17), (32, 32, 32))])
+                                      ((17, 17, 17), (32, 32, 32)), ((3, 3, 100), (20, 3, 60)),
+                                      ((4, 4, 30), (20, 3, 60))])
 def test_no_slower_than_the_cuda_cores(r, ranks, monkeypatch):
     op, lib = api.Operator(api.ProjectHamiltonianSparse(pattern(r), ranks=r), 8), _lib.ttg()
     try:

@@ -249,7 +249,7 @@ constexpr double kTensorFlops = 1.5e8;
 // among them.  14^3 functions, by entry against ragged: rank 1 203 and 234 us,
 // rank 6 249 and 239, rank 32 612 and 301; 60 x 60 x 3 (a million pairs), rank 6
 // 416 and 737.
-double entry_seconds(int64_t nnz, int rc) { return 2.0 * nnz * rc / 0.7e12 + 0.4e-6 * rc; }
+double entry_seconds(int64_t nnz, int rc) { return 2.0 * nnz * rc / 0.7e12 + 0.2e-6 * rc; }
 double ragged_seconds(int64_t pairs, int64_t nq, int rc) {
   const double tiles = (double)pairs / 128.0 * (double)((nq + 63) / 64) * 0.6;
   return 35e-6 + pairs * (1.5e-10 + (rc + 15) / 16 * 16 * 32 / 6e12) +
