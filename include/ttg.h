@@ -135,8 +135,8 @@ ttg_status ttg_op_sync(ttg_op* op);
 ttg_status ttg_op_record(ttg_op* op, int32_t slot);
 ttg_status ttg_op_elapsed_ms(ttg_op* op, int32_t slot0, int32_t slot1, float* ms);
 
-/* Device time of the fused filter-degree kernels (one launch per degree, or
- * per 256-column block of wider blocks) and of the other stages of a ChFSI
+/* Device time of the fused filter-degree kernels (one launch per degree; wide
+ * blocks are column blocks of one launch) and of the other stages of a ChFSI
  * pass and an SCF iteration, by kind.  With timing on, each such launch (or
  * stage) is bracketed by two CUDA events on the operator's stream; the pairs
  * are read back in batches

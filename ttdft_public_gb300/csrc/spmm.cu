@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(512) k_cheb_step(
 // with k <= 16 (8) states its 2 (4) sets of lanes take every second (fourth)
 // list entry and add their sums at the end.  The group's eight warps gather
 // the same block rows within a chunk, so the gathers hit L1.
-// Measured: 8-atom operator (N = 8,000), 16 states: 3.84 -> 0.54 ms a degree;
+// Measured: 8-atom operator (N = 8,000), 16 states: 3.84 -> 0.47 ms a degree;
 // 64-atom operator, 160 states: 82 -> 33 ms.
 constexpr int kF64Chunk = 64;
 
@@ -840,7 +840,8 @@ static void launch_f64_t(ttg_op* op, const double* src, const double* xold, doub
       op->n, k, op->ld, alpha, beta, delta); TTG_COUNT();
 }
 
-// Native FP64 degree.  Widths: even up to 1,024, odd up to 512.
+// Native FP64 degree.  Widths: even up to 1,024, odd up to 512 (limits of the
+// entry points since the first kernel, not of this one).
 static ttg_status launch_f64(ttg_op* op, const void* src, const void* xold, void* dst, int k,
                              double alpha, double beta, double delta) {
   if (k > 1024 || (k % 2 != 0 && k > 512)) return TTG_BAD_ARG;
