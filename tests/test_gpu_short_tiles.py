@@ -1,6 +1,6 @@
 """Filter degrees on tiles of few chunks: the last stage of a tile then has slots without one, for the same gathering
-warps tile after tile, and the warps are on other tiles than the MMAs.  A band of +-w has 128 + 2 w columns a tile:
-9, 10, 11 and 13 chunks of 16.
+warps tile after tile, and the warps are on other tiles than the MMAs.  The rows of a tile use 60 of the 128 + 2 w
+columns around it: 9, 10, 11 and 13 chunks of 16.  And very sparse operators, whose FP32 degrees run on the row groups.
 
 Small whole numbers, whose sums every format holds, come out exact."""
 import numpy as np
@@ -16,8 +16,23 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("w", [5, 12, 20, 36])
 def test_exact_on_short_tiles(w, prec, k):
     n, rng = 152 * 128 * 2 + 77, np.random.default_rng(w + k)
-    off = np.array([-w, -w // 2, 0, 1, w])
-    M = sp.diags([rng.integers(-2, 3, n - abs(o)).astype(float) for o in off], off, format="csr")
+    first = np.arange(n) // 128 * 128 - w
+    col = first[:, None] + np.argsort(rng.random((n, 128 + 2 * w)), axis=1)[:, :60]
+    ok = ((col >= 0) & (col < n)).ravel()
+    row, val = np.repeat(np.arange(n), 60)[ok], rng.choice([-1.0, 1.0], n * 60)[ok]
+    check(sp.csr_matrix((val, (row, col.ravel()[ok])), shape=(n, n)), prec, k)
+
+
+@pytest.mark.parametrize("k", [4, 8, 36, 240])
+@pytest.mark.parametrize("band", [0, 3])
+def test_exact_on_sparse_rows(band, k):
+    n, rng = 5000, np.random.default_rng(band + k)
+    off = np.arange(-band, band + 1)
+    check(sp.diags([rng.choice([-1.0, 1.0], n - abs(o)) for o in off], off, format="csr"), "fp32", k)
+
+
+def check(M, prec, k):
+    n, rng = M.shape[0], np.random.default_rng(k)
     M.sort_indices()
     H = system.Csr(n, n, M.indptr.astype(np.int64), M.indices.astype(np.int32), M.data)
     X = rng.integers(-3, 4, (n, k)).astype(float)

@@ -1219,11 +1219,29 @@ ttg_status build_umma_tiles(ttg_op* op, int64_t n, const int64_t* hp, const int3
   return TTG_OK;
 }
 
+namespace {
+
+// Very sparse operators (short tiles, up to 48 entries a row, far from a
+// Hamiltonian's 1,500): an FP32 degree's planes of the block and padded tiles cost
+// more than the CUDA cores' row groups, unless the rows are long for the block's
+// width; the projectors' two launches come on top there.  Fitted to 390 degrees
+// of 26 operators (us, here and on the row groups): 40,000 rows of 6.5 entries, 24
+// states 28 and 13; 100,000 rows of 16, 24 states 52 and 31; 40,000 rows of 34, 24
+// states 28 and 35, 60 states 48 and 37; 20,000 rows of 18 with projectors, 24
+// states 25 and 28, 60 states 38 and 30.  None of the 390 gets slower by it.
+bool rows_win(const ttg_op* op, int k) {
+  const double row = (double)op->nnz_h / (double)op->n;
+  if (op->umma.slots > 300 * op->umma.n_tiles || row > 48.0) return false;
+  return op->nproj > 0 ? k >= std::max(48.0, 3.0 * row) : k >= std::max(8.0, 1.2 * row);
+}
+
+}  // namespace
+
 // BF16 degrees: whole 16-state steps of the MMA, as the block is gathered.
 // FP32 degrees have planes of their own, padded with zeros to such steps.
 bool umma_supported(const ttg_op* op, int prec, int k) {
   if (op->umma.n_tiles == 0 || op->tc_disabled || k > op->ld) return false;
-  if (prec == TTG_PREC_FP32) return k >= 4 && k % 4 == 0;
+  if (prec == TTG_PREC_FP32) return k >= 4 && k % 4 == 0 && !rows_win(op, k);
   return prec == TTG_PREC_BF16 && k >= 16 && k % 16 == 0;
 }
 
